@@ -819,3 +819,18 @@ def test_gemm_tc_qkv_in_pairs_equals_single_blocks():
         F().set_gemm_pairs(before)
     for a, b in zip(*results):
         assert torch.equal(torch.nan_to_num(a.float(), nan=-7.0), torch.nan_to_num(b.float(), nan=-7.0))
+
+
+# ------------------------------------------------------------------ the 32-bit kernels' own branches
+@pytest.mark.parametrize("k", [4, 31, 128, 130, 516])
+@pytest.mark.parametrize("a_dtype", [torch.float32, torch.bfloat16])
+def test_gemm_f32_chains_are_the_same_in_every_kernel(k, a_dtype):
+    """Few tokens (1 to 16), tiles of 32 and tiles of 64, rows on and off 16 bytes: one chain in order of k, bit for bit."""
+    n = 1111
+    a = rand(1200, k, seed=5).to(a_dtype).to(DEV)
+    w = rand(n, k, seed=6).float().to(DEV)
+    whole = F().linear_f32(a, w)  # 19 x 18 tiles of 64
+    want = a.double() @ w.double().T
+    assert (whole.double() - want).abs().max().item() < 4 * 2.0**-24 * k * 16  # k roundings of sums of at most 16 in size
+    for m in (1, 4, 5, 8, 9, 16, 17, 33, 65):
+        assert torch.equal(F().linear_f32(a[7:7 + m].contiguous(), w), whole[7:7 + m]), f"{m} tokens"
