@@ -324,7 +324,7 @@ def attention_exact(
     call(
         "gk_attention_exact", ptr(q), ptr(kv.k), ptr(kv.v), ptr(out), dtype_code(q.dtype), ptr(tok_pos), ptr(tok_seq),
         ptr(slots), ptr(kv.block_table), n, n_q, n_kv, d, kv.max_pages, kv.page_size, float(scale), int(window),
-        int(sink), stream_ptr(),
+        int(sink), slots.shape[0], stream_ptr(),
     )
     return out
 

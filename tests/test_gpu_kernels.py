@@ -834,3 +834,42 @@ def test_gemm_f32_chains_are_the_same_in_every_kernel(k, a_dtype):
     assert (whole.double() - want).abs().max().item() < 4 * 2.0**-24 * k * 16  # k roundings of sums of at most 16 in size
     for m in (1, 4, 5, 8, 9, 16, 17, 33, 65):
         assert torch.equal(F().linear_f32(a[7:7 + m].contiguous(), w), whole[7:7 + m]), f"{m} tokens"
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,d,window,sink", [(2, 2, 8, 0, False), (6, 2, 40, 70, True), (10, 2, 72, 0, True), (9, 1, 64, 33, False),
+                                                    (8, 1, 128, 0, False), (16, 1, 32, 0, False), (16, 1, 128, 1100, False)])
+def test_attention_exact_is_the_same_in_every_kernel(dtype, n_q, n_kv, d, window, sink):
+    """A step of many tokens (the tile kernel), the same tokens one a step and few a step (the cluster), bit for bit, with
+    values of later positions poisoned for the single steps; spans of 1,024 keys, blocks of 32 and pages of 64 are crossed."""
+    lens, past = [1300, 37, 700], [0, 0, 650]
+    kv, slots, table = scrambled_pages(3, 1300, n_kv, d, dtype, seed=12)
+    pos, seq = [], []
+    for i, (n, p) in enumerate(zip(lens, past)):
+        fill_pages(kv, table, int(slots[i]), rand(n, n_kv, d, seed=60 + i).to(dtype), rand(n, n_kv, d, seed=70 + i).to(dtype))
+        pos += list(range(p, n))
+        seq += [i] * (n - p)
+    q = rand(len(pos), n_q, d, seed=80).to(dtype).to(DEV)
+    pos, seq = torch.tensor(pos, dtype=torch.int32).to(DEV), torch.tensor(seq, dtype=torch.int32).to(DEV)
+    whole = F().attention_exact(q, kv, pos, seq, slots.to(DEV), d**-0.5, window, sink=sink)
+    assert torch.isfinite(whole).all()
+    for rows in ([0], [31], [32, 1000], [1023], [1024, 1300, 1336], [1299, 1336, 1386], list(range(1100, 1110))):
+        at = torch.tensor(rows).to(DEV)
+        got = F().attention_exact(q[at].contiguous(), kv, pos[at].contiguous(), seq[at].contiguous(), slots.to(DEV), d**-0.5, window, sink=sink)
+        assert torch.equal(got, whole[at]), f"tokens {rows}"
+
+
+def test_attention_exact_does_not_take_values_beyond_a_token():
+    """Whatever stands behind a token's own position in its last block of keys stays out of its sum, in every kernel."""
+    n_q, n_kv, d, n = 4, 2, 64, 200
+    kv, slots, table = scrambled_pages(1, 320, n_kv, d, torch.float32, seed=13)
+    v = rand(n, n_kv, d, seed=2).float()
+    v[150:] = float("inf")
+    fill_pages(kv, table, int(slots[0]), rand(n, n_kv, d, seed=1).float(), v)
+    q = rand(n, n_q, d, seed=3).float().to(DEV)
+    zeros, pos = torch.zeros(n, dtype=torch.int32).to(DEV), torch.arange(n, dtype=torch.int32).to(DEV)
+    many = F().attention_exact(q.repeat(2, 1, 1), kv, pos.repeat(2), zeros.repeat(2), slots.to(DEV), d**-0.5)
+    few = F().attention_exact(q[:150].contiguous(), kv, pos[:150].contiguous(), zeros[:150], slots.to(DEV), d**-0.5)
+    assert torch.isfinite(many[:150]).all() and torch.equal(many[:150], few) and not torch.isfinite(many[150:200]).any()
+    one = F().attention_exact(q[149:150].contiguous(), kv, pos[149:150].contiguous(), zeros[:1], slots.to(DEV), d**-0.5)
+    assert torch.equal(one[0], many[149])
