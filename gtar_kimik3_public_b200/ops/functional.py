@@ -952,10 +952,11 @@ def sample(
     if out is None:
         out = torch.empty((n,), dtype=torch.int32, device=logits.device)
     _check(out, "out", torch.int32, 1)
-    # as for argmax: several blocks share a row; eight bytes of scratch per row for the top-k thresholds (four
-    # used) and eight per row and part for the parts' results
+    # as for argmax: several blocks share a row, eight bytes of scratch per row and part for the parts' results (with
+    # top-k a cluster shares a row and needs none)
     parts = row_parts(n, vocab, logits.device)
-    scratch = torch.empty((2 * ((n + 1) // 2) + 2 * n * parts,), dtype=torch.int32, device=logits.device)
+    cut = parts > 1 and not 0 < int(top_k or 0) < vocab
+    scratch = torch.empty((2 * n * parts,), dtype=torch.int32, device=logits.device) if cut else None
     call(
         "gk_sample", ptr(logits), vocab, n, vocab, float(temperature), int(top_k or 0), int(seed) & (2**64 - 1),
         ptr(request_ids), ptr(steps), int(advance_steps), ptr(out), parts, ptr(scratch), stream_ptr(),

@@ -873,3 +873,25 @@ def test_attention_exact_does_not_take_values_beyond_a_token():
     assert torch.isfinite(many[:150]).all() and torch.equal(many[:150], few) and not torch.isfinite(many[150:200]).any()
     one = F().attention_exact(q[149:150].contiguous(), kv, pos[149:150].contiguous(), zeros[:1], slots.to(DEV), d**-0.5)
     assert torch.equal(one[0], many[149])
+
+
+@pytest.mark.parametrize("rows,vocab,top_k", [(1, 151936, 50), (3, 40001, 64), (3, 40001, 65), (2, 40001, 256), (2, 40001, 257), (130, 3001, 9),
+                                              (2, 600, 599), (1, 5, 2), (75, 9000, 128)])
+@pytest.mark.parametrize("values", ["spread", "few", "equal", "sorted", "infinite"])
+def test_sample_top_k_of_any_rows(rows, vocab, top_k, values):
+    """The bound by groups, and the counting scans where too many logits reach it (rows of few distinct or equal numbers) or k
+    is beyond half the groups; rows of odd lengths; clusters of fewer blocks where rows are many."""
+    logits = rand(rows, vocab, seed=vocab + top_k).float() * 3
+    if values == "few":
+        logits = logits.round()
+    elif values == "equal":
+        logits = torch.full((rows, vocab), 0.25)
+    elif values == "sorted":
+        logits = logits.sort(dim=1).values
+    elif values == "infinite":
+        logits[:, top_k // 2:] = -math.inf  # fewer finite numbers than are asked for
+        logits = logits[:, torch.randperm(vocab, generator=torch.Generator().manual_seed(1))].contiguous()
+    requests, steps = torch.arange(5, 5 + rows, dtype=torch.int32), torch.arange(rows, dtype=torch.int32) % 7
+    got = F().sample(logits.to(DEV), 0.9, top_k, 77, requests.to(DEV), steps.to(DEV)).cpu().tolist()
+    for i in range(min(rows, 4)):
+        assert got[i] == plain_sampling.sample(logits[i].numpy(), 0.9, top_k, 77, int(requests[i]), int(steps[i])), f"row {i}"
