@@ -13,15 +13,17 @@
 //                stands behind the router's rows (z has E + 1 entries), and the sigmoid is either the weight of one more
 //                pair (token, expert E) behind the token's chosen ones, or an output of its own.
 //   experts_up   act[pair] = silu(W_gate[e] h_t) * (W_up[e] h_t) for every pair (token, chosen expert)
-//   experts_down out_t = add_t (times a number per token, where one is given) + sum over the token's pairs, in the order they were chosen, of weight * W_down[e] act[pair]
+//   experts_down (and experts_join behind it) out_t = add_t (times a number per token, where one is given) + sum over the token's pairs, in the order they were chosen, of weight * W_down[e] act[pair]
 //                (32-bit result: it is what goes into the residual stream)
 //
-// The two expert kernels take a pair at a time, one warp per output row: the path of single-token steps, of 32-bit
-// runs and of sizes the tensor-core path does not take.  A token's result depends on the token alone.
+// The expert kernels take an expert's pairs together, so that its rows are fetched once for them: the path of few-token steps,
+// of 32-bit runs and of sizes the sorted path does not take.  A token's result depends on the token alone.
 //
 //   sort, gather_rows, combine   many-token steps: the pairs put in the order of their experts, the tokens' rows copied
 //                into that order (each expert's rows then go through one tensor-core product, made by the caller), and
 //                the weighted sum of a token's expert outputs in the order the experts were chosen
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -66,7 +68,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_scores_kernel(const T*
 #pragma unroll
         for (int j = 0; j < SCORE_EXPERTS; ++j) acc[a][j] = 0.f;
     if (width % 4 == 0) {  // four neighbouring elements a lane and turn
-#pragma unroll 2
+#pragma unroll (SCORE_EXPERTS == 2 ? 4 : 2)
         for (int i = lane * 4; i < width; i += 128) {
             float xv[SCORE_TOKENS][4], wv[SCORE_EXPERTS][4];
 #pragma unroll
@@ -290,12 +292,15 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_choose_kernel(
     }
 }
 
-// A lane's share of NR dot products of one vector in shared memory with NR rows in memory, summed in index order; the
-// rows' loads are independent, so all of them are on their way together.  The caller finishes each with warp_sum.
-template <typename TW, int NR>
-__device__ __forceinline__ void dot_parts(const float* __restrict__ x, const TW* const (&rows)[NR], int n, int lane, float (&acc)[NR]) {
+// A lane's share of the dot products of NR rows in memory with NT vectors in shared memory (`stride` apart), each summed in
+// index order; the rows' loads are independent, so all of them are on their way together, and a piece of a vector is read once
+// for all rows.  The caller finishes each with warp_sum.
+template <typename TW, int NR, int NT>
+__device__ __forceinline__ void dot_many(const float* __restrict__ x, int stride, const TW* const (&rows)[NR], int n, int lane, float (&acc)[NT][NR]) {
 #pragma unroll
-    for (int j = 0; j < NR; ++j) acc[j] = 0.f;
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int j = 0; j < NR; ++j) acc[t][j] = 0.f;
     constexpr int VEC = 16 / sizeof(TW);
     if (n % VEC == 0) {
 #pragma unroll 2
@@ -303,6 +308,7 @@ __device__ __forceinline__ void dot_parts(const float* __restrict__ x, const TW*
             uint4 raw[NR];
 #pragma unroll
             for (int j = 0; j < NR; ++j) raw[j] = *reinterpret_cast<const uint4*>(rows[j] + i);
+            float w[NR][VEC];
 #pragma unroll
             for (int j = 0; j < NR; ++j) {
                 if constexpr (sizeof(TW) == 2) {
@@ -310,140 +316,445 @@ __device__ __forceinline__ void dot_parts(const float* __restrict__ x, const TW*
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         const float2 f = __bfloat1622float2(p[c]);
-                        acc[j] = fmaf(x[i + 2 * c], f.x, acc[j]);
-                        acc[j] = fmaf(x[i + 2 * c + 1], f.y, acc[j]);
+                        w[j][2 * c] = f.x, w[j][2 * c + 1] = f.y;
                     }
                 } else {
                     const float* f = reinterpret_cast<const float*>(&raw[j]);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[j] = fmaf(x[i + c], f[c], acc[j]);
+                    for (int c = 0; c < VEC; ++c) w[j][c] = f[c];
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+#pragma unroll
+                for (int c = 0; c < VEC; c += 4) {
+                    const float4 xv = *reinterpret_cast<const float4*>(x + t * stride + i + c);
+#pragma unroll
+                    for (int j = 0; j < NR; ++j) {
+                        acc[t][j] = fmaf(xv.x, w[j][c], acc[t][j]);
+                        acc[t][j] = fmaf(xv.y, w[j][c + 1], acc[t][j]);
+                        acc[t][j] = fmaf(xv.z, w[j][c + 2], acc[t][j]);
+                        acc[t][j] = fmaf(xv.w, w[j][c + 3], acc[t][j]);
+                    }
                 }
             }
         }
     } else {
         for (int i = lane; i < n; i += 32)
-#pragma unroll
-            for (int j = 0; j < NR; ++j) acc[j] = fmaf(x[i], to_float(rows[j][i]), acc[j]);
-    }
-}
-
-// The same for NR vectors in shared memory, x_stride apart, each with a row of its own.
-template <typename TW, int NR>
-__device__ __forceinline__ void dot_pairs(const float* __restrict__ x, int x_stride, const TW* const (&rows)[NR], int n, int lane, float (&acc)[NR]) {
-#pragma unroll
-    for (int j = 0; j < NR; ++j) acc[j] = 0.f;
-    constexpr int VEC = 16 / sizeof(TW);
-    if (n % VEC == 0) {
-#pragma unroll 2
-        for (int i = lane * VEC; i < n; i += 32 * VEC) {
-            uint4 raw[NR];
-#pragma unroll
-            for (int j = 0; j < NR; ++j) raw[j] = *reinterpret_cast<const uint4*>(rows[j] + i);
 #pragma unroll
             for (int j = 0; j < NR; ++j) {
-                const float* xj = x + j * x_stride + i;
-                if constexpr (sizeof(TW) == 2) {
-                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
+                const float w = to_float(rows[j][i]);
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float2 f = __bfloat1622float2(p[c]);
-                        acc[j] = fmaf(xj[2 * c], f.x, acc[j]);
-                        acc[j] = fmaf(xj[2 * c + 1], f.y, acc[j]);
-                    }
-                } else {
-                    const float* f = reinterpret_cast<const float*>(&raw[j]);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[j] = fmaf(xj[c], f[c], acc[j]);
-                }
+                for (int t = 0; t < NT; ++t) acc[t][j] = fmaf(x[t * stride + i], w, acc[t][j]);
             }
-        }
-    } else {
-        for (int i = lane; i < n; i += 32)
-#pragma unroll
-            for (int j = 0; j < NR; ++j) acc[j] = fmaf(x[j * x_stride + i], to_float(rows[j][i]), acc[j]);
     }
 }
 
-template <int N>
-struct Count {
-    static constexpr int value = N;
-};
+constexpr int UP_WARPS = 8, LIST = 1024, MAX_NT = 4;
 
-constexpr int UP_WARPS = 8;
+// The pairs of one expert among the LIST pairs from `first` on, in their order.  A block asks for the expert `blockIdx.x`
+// (by_expert) or for that of pair `blockIdx.x`; in the second form only the block of the expert's first pair goes on.
+// Returns how many there are (0: nothing to do), the same in all threads.
+template <int WARPS>
+__device__ __forceinline__ int list_pairs(const int* __restrict__ ids, int n_pairs, int first, bool by_expert, int& expert, int* list, int* scratch) {
+    expert = by_expert ? (int)blockIdx.x : ids[blockIdx.x];
+    const int last = min(first + LIST, n_pairs), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int count = 0;
+    for (int i0 = first; i0 < last; i0 += WARPS * 32) {
+        const int i = i0 + threadIdx.x;
+        const bool mine = i < last && ids[i] == expert;
+        const unsigned int found = __ballot_sync(0xffffffffu, mine);
+        if (lane == 0) scratch[warp] = __popc(found);
+        __syncthreads();
+        int before = count;
+        for (int w = 0; w < WARPS; ++w) {
+            if (w < warp) before += scratch[w];
+            count += scratch[w];
+        }
+        if (mine) list[before + __popc(found & ((1u << lane) - 1))] = i;
+        __syncthreads();
+    }
+    if (!by_expert && count > 0 && list[0] != (int)blockIdx.x) count = 0;
+    return count;
+}
 
-// grid (pairs, chunks of ff): w_gate_up [E, 2, ff, width] (gate rows then up rows of an expert)
-template <typename T, typename TW>
-__global__ void __launch_bounds__(UP_WARPS * 32) experts_up_kernel(
-    const T* __restrict__ h, const TW* __restrict__ w_gate_up, const int* __restrict__ ids, T* __restrict__ act, int width,
-    int ff, int top, int rows_per_block) {
-    extern __shared__ __align__(16) float xs[];  // width
-    pdl_launch_dependents();
-    pdl_wait();
-    const int pair = blockIdx.x, t = pair / top;
-    const int e = ids[pair];
-    for (int i = threadIdx.x; i < width; i += UP_WARPS * 32) xs[i] = to_float(h[(size_t)t * width + i]);
-    __syncthreads();
+// act[pair] = silu(gate) * up for NT pairs of one expert (their tokens' rows in `xs`), rows f0 .. f_end - 1
+template <typename T, typename TW, int NT>
+__device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int count, const TW* wg, const TW* wu, T* __restrict__ act, int width, int ff, int f0, int f_end) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const TW* wg = w_gate_up + (size_t)e * 2 * ff * width;
-    const TW* wu = wg + (size_t)ff * width;
-    const int f0 = blockIdx.y * rows_per_block;
-    const int f_end = min(ff, f0 + rows_per_block);
     int f = f0 + warp;
     for (; f + UP_WARPS < f_end; f += 2 * UP_WARPS) {  // two rows of gate and of up at once: four rows' loads in flight
         const TW* const rows[4] = {wg + (size_t)f * width, wu + (size_t)f * width, wg + (size_t)(f + UP_WARPS) * width,
                                    wu + (size_t)(f + UP_WARPS) * width};
-        float part[4];
-        dot_parts<TW, 4>(xs, rows, width, lane, part);
+        float part[NT][4];
+        dot_many<TW, 4, NT>(xs, width, rows, width, lane, part);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) part[j] = warp_sum(part[j]);
-        if (lane == 0) {
-            act[(size_t)pair * ff + f] = from_float<T>(part[0] / (1.f + expf(-part[0])) * part[1]);
-            act[(size_t)pair * ff + f + UP_WARPS] = from_float<T>(part[2] / (1.f + expf(-part[2])) * part[3]);
+        for (int t = 0; t < NT; ++t) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) part[t][j] = warp_sum(part[t][j]);
+            if (lane == 0 && t < count) {
+                T* to = act + (size_t)pairs[t] * ff + f;
+                to[0] = from_float<T>(part[t][0] / (1.f + expf(-part[t][0])) * part[t][1]);
+                to[UP_WARPS] = from_float<T>(part[t][2] / (1.f + expf(-part[t][2])) * part[t][3]);
+            }
         }
     }
     for (; f < f_end; f += UP_WARPS) {
         const TW* const rows[2] = {wg + (size_t)f * width, wu + (size_t)f * width};
-        float part[2];
-        dot_parts<TW, 2>(xs, rows, width, lane, part);
-        const float gate = warp_sum(part[0]), up = warp_sum(part[1]);
-        if (lane == 0) act[(size_t)pair * ff + f] = from_float<T>(gate / (1.f + expf(-gate)) * up);
+        float part[NT][2];
+        dot_many<TW, 2, NT>(xs, width, rows, width, lane, part);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const float gate = warp_sum(part[t][0]), up = warp_sum(part[t][1]);
+            if (lane == 0 && t < count) act[(size_t)pairs[t] * ff + f] = from_float<T>(gate / (1.f + expf(-gate)) * up);
+        }
     }
 }
 
-// grid (tokens, chunks of width): w_down [E, width, ff]
+// grid (experts or pairs, chunks of ff, lists of pairs): w_gate_up [E, 2, ff, width] (gate rows then up rows of an expert).
+// An expert's rows are fetched once for `at_once` of the tokens that chose it (more tokens take the rows again, out of L2).
 template <typename T, typename TW>
-__global__ void __launch_bounds__(UP_WARPS * 32) experts_down_kernel(
-    const T* __restrict__ act, const TW* __restrict__ w_down, const int* __restrict__ ids, const float* __restrict__ weights,
-    const T* __restrict__ add, const float* __restrict__ add_weight, float* __restrict__ out, int width, int ff, int top,
-    int rows_per_block) {
-    extern __shared__ __align__(16) float as[];  // top * ff
+__global__ void __launch_bounds__(UP_WARPS * 32) experts_up_kernel(
+    const T* __restrict__ h, const TW* __restrict__ w_gate_up, const int* __restrict__ ids, T* __restrict__ act, int n_pairs, int width,
+    int ff, int top, int rows_per_block, int by_expert, int at_once) {
+    extern __shared__ __align__(16) unsigned char expert_smem[];
+    float* xs = reinterpret_cast<float*>(expert_smem);  // [at_once][width]
+    __shared__ int list[LIST], scratch[UP_WARPS];
     pdl_launch_dependents();
     pdl_wait();
-    const int t = blockIdx.x;
-    for (int i = threadIdx.x; i < top * ff; i += UP_WARPS * 32) as[i] = to_float(act[(size_t)t * top * ff + i]);
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c0 = blockIdx.y * rows_per_block;
-    for (int c = c0 + warp; c < min(width, c0 + rows_per_block); c += UP_WARPS) {
-        float acc = add != nullptr ? to_float(add[(size_t)t * width + c]) : 0.f;
-        if (add_weight != nullptr) acc *= add_weight[t];
-        int kk = 0;
-        auto add_pairs = [&](auto count) {  // their rows in flight together; the sum still takes them in the order they were chosen
-            constexpr int NR = decltype(count)::value;
-            const TW* rows[NR];
-            float part[NR];
-#pragma unroll
-            for (int j = 0; j < NR; ++j) rows[j] = w_down + ((size_t)ids[(size_t)t * top + kk + j] * width + c) * ff;
-            dot_pairs<TW, NR>(as + (size_t)kk * ff, ff, rows, ff, lane, part);
-#pragma unroll
-            for (int j = 0; j < NR; ++j) acc = fmaf(weights[(size_t)t * top + kk + j], warp_sum(part[j]), acc);
-            kk += NR;
-        };
-        while (kk + 4 <= top) add_pairs(Count<4>{});
-        if (kk + 2 <= top) add_pairs(Count<2>{});
-        if (kk < top) add_pairs(Count<1>{});
-        if (lane == 0) out[(size_t)t * width + c] = acc;
+    int e;
+    const int n = list_pairs<UP_WARPS>(ids, n_pairs, blockIdx.z * LIST, by_expert != 0, e, list, scratch);
+    const TW* wg = w_gate_up + (size_t)e * 2 * ff * width;
+    const TW* wu = wg + (size_t)ff * width;
+    const int f0 = blockIdx.y * rows_per_block, f_end = min(ff, f0 + rows_per_block);
+    for (int at = 0; at < n; at += at_once) {
+        const int count = min(at_once, n - at);
+        __syncthreads();
+        for (int k = 0; k < count; ++k) {
+            const T* x = h + (size_t)(list[at + k] / top) * width;
+            for (int i = threadIdx.x; i < width; i += UP_WARPS * 32) xs[k * width + i] = to_float(x[i]);
+        }
+        __syncthreads();
+        if (count == 1) up_rows<T, TW, 1>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
+        else if (count == 2) up_rows<T, TW, 2>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
+        else up_rows<T, TW, MAX_NT>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
     }
+}
+
+template <typename TW, int NT>
+__device__ __forceinline__ void down_rows(const float* as, const int* pairs, int count, const TW* w, float* __restrict__ parts, int width, int ff, int c0, int c_end) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int c = c0 + 4 * warp; c < c_end; c += 4 * UP_WARPS) {
+        if (c + 4 <= c_end) {  // four rows' loads in flight
+            const TW* const rows[4] = {w + (size_t)c * ff, w + (size_t)(c + 1) * ff, w + (size_t)(c + 2) * ff, w + (size_t)(c + 3) * ff};
+            float part[NT][4];
+            dot_many<TW, 4, NT>(as, ff, rows, ff, lane, part);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                float mine = 0.f;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float sum = warp_sum(part[t][j]);
+                    if (lane == j) mine = sum;
+                }
+                if (lane < 4 && t < count) parts[(size_t)pairs[t] * width + c + lane] = mine;
+            }
+        } else {  // what is left of a chunk that is no multiple of four
+            for (int cc = c; cc < c_end; ++cc) {
+                const TW* const rows[1] = {w + (size_t)cc * ff};
+                float part[NT][1];
+                dot_many<TW, 1, NT>(as, ff, rows, ff, lane, part);
+#pragma unroll
+                for (int t = 0; t < NT; ++t) {
+                    const float sum = warp_sum(part[t][0]);
+                    if (lane == 0 && t < count) parts[(size_t)pairs[t] * width + cc] = sum;
+                }
+            }
+        }
+    }
+}
+
+// grid as experts_up: w_down [E, width, ff], parts [pairs, width] = the pairs' unweighted outputs, which experts_join adds up.
+template <typename T, typename TW>
+__global__ void __launch_bounds__(UP_WARPS * 32) experts_down_kernel(
+    const T* __restrict__ act, const TW* __restrict__ w_down, const int* __restrict__ ids, float* __restrict__ parts, int n_pairs, int width,
+    int ff, int rows_per_block, int by_expert, int at_once) {
+    extern __shared__ __align__(16) unsigned char expert_smem[];
+    float* as = reinterpret_cast<float*>(expert_smem);  // [at_once][ff]
+    __shared__ int list[LIST], scratch[UP_WARPS];
+    pdl_launch_dependents();
+    pdl_wait();
+    int e;
+    const int n = list_pairs<UP_WARPS>(ids, n_pairs, blockIdx.z * LIST, by_expert != 0, e, list, scratch);
+    const TW* w = w_down + (size_t)e * width * ff;
+    const int c0 = blockIdx.y * rows_per_block, c_end = min(width, c0 + rows_per_block);
+    for (int at = 0; at < n; at += at_once) {
+        const int count = min(at_once, n - at);
+        __syncthreads();
+        for (int k = 0; k < count; ++k) {
+            const T* x = act + (size_t)list[at + k] * ff;
+            for (int i = threadIdx.x; i < ff; i += UP_WARPS * 32) as[k * ff + i] = to_float(x[i]);
+        }
+        __syncthreads();
+        if (count == 1) down_rows<TW, 1>(as, list + at, count, w, parts, width, ff, c0, c_end);
+        else if (count == 2) down_rows<TW, 2>(as, list + at, count, w, parts, width, ff, c0, c_end);
+        else down_rows<TW, MAX_NT>(as, list + at, count, w, parts, width, ff, c0, c_end);
+    }
+}
+
+// ---- the same products on the tensor cores, for bfloat16 rows and weights of sizes in whole tiles (mma.sync m16n8k16, 32-bit sums)
+//
+// A block has sixteen rows of an expert's matrix at a time (of gate and of up together), each of its four warps a quarter of
+// the reduction, and the tokens that chose the expert are the product's columns, eight or sixteen of them.  The order in which
+// a product walks k is free as long as both operands take the same one, so a lane reads eight neighbouring entries of its row
+// at once (16 bytes) and they serve as its fragments of two products; the tokens' rows lie in shared memory and are read the
+// same way.  What remains is the stream of the weights, every expert's rows once whatever number of tokens chose it.  Blocks stay
+// and take equal runs of (expert, sixteen rows) units: the experts that were chosen are listed by every block for itself, and a
+// warp asks for its first rows of the next unit before it adds up this one's.  (One block a pair and chunk of rows, most of
+// which found that another had their expert, spent their time in the chain ids - list - weights - tokens: 60 us where the
+// weights take 21.)  (Tensor-memory products would want 128 rows a tile and the weights through shared memory, for a
+// step that does next to no arithmetic.)
+// Measured (us; up, down and join; 6 of 64 experts of 2,048 x 1,024), before (every pair streamed its expert's rows by itself, a
+// row a warp on the FP32 pipes) and now: 2 tokens 51 / 45, 4: 88 / 53, 8: 159 / 73 (16 experts: 2.8 TB/s), 16: 298 / 99, 42:
+// 739 / 166; 4 of 32 experts of 1,024 x 768: one token 10 / 12, 3: 19 / 15, 8: 39 / 24, 63: 260 / 46.
+constexpr int MMA_WARPS = 4, MMA_STEPS = 2, MMA_TOKENS = 16, MMA_LIST = 512;
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// bytes from one token's row in shared memory to the next: 64 beyond a multiple of 128, so that the eight lanes that read
+// together (two rows, four pieces) fall into different banks
+__host__ __device__ constexpr int mma_stride(int k) { return (k * 2 + 127) / 128 * 128 + 64; }
+
+// MMA_STEPS pieces of 32 entries of a lane's two rows (`k` entries a row, eight rows apart) of each matrix
+template <int NM>
+struct MmaBatch {
+    uint4 lo[MMA_STEPS][NM], hi[MMA_STEPS][NM];
+    __device__ __forceinline__ void load(const __nv_bfloat16* const (&row0)[NM], int k, int i, int end) {
+#pragma unroll
+        for (int u = 0; u < MMA_STEPS; ++u)
+            if (i + u < end) {
+#pragma unroll
+                for (int m = 0; m < NM; ++m) {
+                    const __nv_bfloat16* at = row0[m] + (i + u) * 32;
+                    lo[u][m] = *reinterpret_cast<const uint4*>(at);
+                    hi[u][m] = *reinterpret_cast<const uint4*>(at + (size_t)8 * k);
+                }
+            }
+    }
+    template <int NB>
+    __device__ __forceinline__ void multiply(const unsigned char* x_at, int stride, int i, int end, float (&sums)[NM][NB][4]) const {
+#pragma unroll
+        for (int u = 0; u < MMA_STEPS; ++u)
+            if (i + u < end) {
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    const uint4 x = *reinterpret_cast<const uint4*>(x_at + b * 8 * stride + (i + u) * 64);
+#pragma unroll
+                    for (int m = 0; m < NM; ++m) {
+                        mma_bf16(sums[m][b], lo[u][m].x, hi[u][m].x, lo[u][m].y, hi[u][m].y, x.x, x.y);
+                        mma_bf16(sums[m][b], lo[u][m].z, hi[u][m].z, lo[u][m].w, hi[u][m].w, x.z, x.w);
+                    }
+                }
+            }
+    }
+};
+
+// rows of `source` (`divide` pairs share one) for pairs[0 .. count - 1] into shared memory; what stands in the rows behind them
+// is multiplied into columns that nobody reads
+__device__ __forceinline__ void mma_stage(unsigned char* xs, int stride, const __nv_bfloat16* __restrict__ source, const int* pairs, int count, int divide, int k) {
+    const int pieces = k / 8;
+    for (int i = threadIdx.x; i < count * pieces; i += MMA_WARPS * 32) {
+        const int t = i / pieces, c = i - t * pieces;
+        *reinterpret_cast<uint4*>(xs + t * stride + c * 16) = *reinterpret_cast<const uint4*>(source + (size_t)(pairs[t] / divide) * k + c * 8);
+    }
+}
+
+// Sixteen rows of NM matrices times the staged tokens, this warp's quarter: part[(m NB + b) 4 + e][lane].  `first`: the batch that
+// this warp has already asked for.
+template <int NM, int NB>
+__device__ __forceinline__ void mma_tile(MmaBatch<NM>& first, const __nv_bfloat16* const (&row0)[NM], int k, int begin, int end, const unsigned char* xs, int stride,
+                                         float (*part)[32]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const unsigned char* x_at = xs + g * stride + q * 16;
+    float sums[NM][NB][4];
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sums[m][b][e] = 0.f;
+    for (int i = begin; i < end; i += 2 * MMA_STEPS) {
+        MmaBatch<NM> second;
+        second.load(row0, k, i + MMA_STEPS, end);
+        first.template multiply<NB>(x_at, stride, i, end, sums);
+        first.load(row0, k, i + 2 * MMA_STEPS, end);
+        second.template multiply<NB>(x_at, stride, i + MMA_STEPS, end, sums);
+    }
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[(m * NB + b) * 4 + e][lane] = sums[m][b][e];
+}
+
+// the sum of one entry over the warps
+template <int N>
+__device__ __forceinline__ float mma_sum(const float (*part)[N][32], int entry, int lane) {
+    return ((part[0][entry][lane] + part[1][entry][lane]) + part[2][entry][lane]) + part[3][entry][lane];
+}
+
+// A run of up to `at_once` pairs of one expert: places `start` .. of the pairs in the order of their experts.
+struct MmaRun {
+    int expert, start, count;
+};
+
+// The pairs ids[first .. last - 1] (at most MMA_LIST) in the order of their experts, an expert's in their own order, and their runs:
+// all blocks come to the same list, so that each may take some of a run's rows.  `counts`: 2 n_experts + MMA_LIST ints of shared
+// memory.  Returns the number of runs.
+__device__ __forceinline__ int mma_list(const int* __restrict__ ids, int first, int last, int n_experts, int at_once, int* counts, int* list, MmaRun* runs, int* n_runs) {
+    constexpr int THREADS = MMA_WARPS * 32;
+    if (last - first <= 32) {  // a few tokens: one warp, a lane a pair, the experts in the order of their first pairs
+        if (threadIdx.x < 32) {
+            const int lane = threadIdx.x, i = first + lane, e = i < last ? ids[i] : -1 - lane;
+            const unsigned int same = __match_any_sync(0xffffffffu, e);
+            const int rank = __popc(same & ((1u << lane) - 1)), leader = __ffs(same) - 1;
+            const int mine = i < last && rank == 0 ? __popc(same) : 0, mine_runs = (mine + at_once - 1) / at_once;
+            int upto = mine, upto_runs = mine_runs;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, upto, o), b = __shfl_up_sync(0xffffffffu, upto_runs, o);
+                if (lane >= o) upto += a, upto_runs += b;
+            }
+            const int start = __shfl_sync(0xffffffffu, upto - mine, leader);
+            if (i < last) list[start + rank] = i;
+            for (int r = 0; r < mine_runs; ++r) runs[upto_runs - mine_runs + r] = MmaRun{e, start + r * at_once, min(at_once, mine - r * at_once)};
+            if (lane == 31) *n_runs = upto_runs;
+        }
+        __syncthreads();
+        return *n_runs;
+    }
+    int *starts = counts + n_experts, *expert_of = starts + n_experts;
+    for (int e = threadIdx.x; e < n_experts; e += THREADS) counts[e] = 0;
+    __syncthreads();
+    for (int i = first + threadIdx.x; i < last; i += THREADS) {
+        expert_of[i - first] = ids[i];
+        atomicAdd(&counts[ids[i]], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int pairs = 0, all = 0;  // of the experts before
+        for (int e0 = 0; e0 < n_experts; e0 += 32) {
+            const int e = e0 + lane, mine = e < n_experts ? counts[e] : 0, mine_runs = (mine + at_once - 1) / at_once;
+            int upto = mine, upto_runs = mine_runs;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, upto, o), b = __shfl_up_sync(0xffffffffu, upto_runs, o);
+                if (lane >= o) upto += a, upto_runs += b;
+            }
+            const int start = pairs + upto - mine;
+            if (e < n_experts) starts[e] = start;
+            for (int r = 0; r < mine_runs; ++r) runs[all + upto_runs - mine_runs + r] = MmaRun{e, start + r * at_once, min(at_once, mine - r * at_once)};
+            pairs += __shfl_sync(0xffffffffu, upto, 31);
+            all += __shfl_sync(0xffffffffu, upto_runs, 31);
+        }
+        if (lane == 0) *n_runs = all;
+        __syncwarp();
+        for (int i0 = first; i0 < last; i0 += 32) {
+            const int i = i0 + lane;
+            const unsigned int there = __ballot_sync(0xffffffffu, i < last);
+            if (i < last) {
+                const int e = expert_of[i - first];
+                const unsigned int same = __match_any_sync(there, e);
+                const int before = __popc(same & ((1u << lane) - 1)), at = starts[e];
+                list[at + before] = i;
+                __syncwarp(there);
+                if (before == 0) starts[e] = at + __popc(same);
+            }
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    return *n_runs;
+}
+
+// UP: gate and up rows, act[pair] = silu(gate) * up; else rows of w_down, parts[pair].  k entries a row, n_rows rows a matrix.
+template <bool UP>
+__global__ void __launch_bounds__(MMA_WARPS * 32, UP ? 3 : 4) experts_mma_kernel(
+    const __nv_bfloat16* __restrict__ source, const __nv_bfloat16* __restrict__ weights, const int* __restrict__ ids, __nv_bfloat16* __restrict__ act,
+    float* __restrict__ parts, int n_pairs, int k, int n_rows, int divide, int n_experts, int at_once) {
+    constexpr int NM = UP ? 2 : 1, ENTRIES = NM * MMA_TOKENS / 8 * 4;
+    extern __shared__ __align__(16) unsigned char expert_smem[];  // the tokens' rows [at_once][stride]; before that, counts
+    __shared__ int list[MMA_LIST], n_runs;
+    __shared__ MmaRun runs[MMA_LIST];
+    __shared__ float part[MMA_WARPS][ENTRIES][32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int first_pair = blockIdx.z * MMA_LIST, last_pair = min(first_pair + MMA_LIST, n_pairs);
+    const int tiles = n_rows / 16;
+    const long long units = (long long)mma_list(ids, first_pair, last_pair, n_experts, at_once, (int*)expert_smem, list, runs, &n_runs) * tiles;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int stride = mma_stride(k), pieces = k / 32, share = (pieces + MMA_WARPS - 1) / MMA_WARPS;
+    const int begin = min(warp * share, pieces), end = min(begin + share, pieces);
+    int unit = (int)(units * blockIdx.x / gridDim.x);
+    const int unit_end = (int)(units * (blockIdx.x + 1) / gridDim.x);
+    const __nv_bfloat16* rows[NM];
+    const auto point = [&](int u) {
+        const __nv_bfloat16* at = weights + (size_t)runs[u / tiles].expert * NM * n_rows * k + (size_t)((u % tiles) * 16 + g) * k + q * 8;
+#pragma unroll
+        for (int m = 0; m < NM; ++m) rows[m] = at + (size_t)m * n_rows * k;
+    };
+    MmaBatch<NM> first;
+    if (unit < unit_end) {
+        point(unit);
+        first.load(rows, k, begin, end);
+    }
+    for (int staged = -1; unit < unit_end; ++unit) {
+        const int at = unit / tiles, tile = unit % tiles, count = runs[at].count, NB = count <= 8 ? 1 : 2;
+        const int* pairs = list + runs[at].start;
+        if (at != staged) {  // all warps are through with the rows of before: they stand behind the barrier after their sums
+            mma_stage(expert_smem, stride, source, pairs, count, divide, k);
+            staged = at;
+        }
+        __syncthreads();
+        if (NB == 1) mma_tile<NM, 1>(first, rows, k, begin, end, expert_smem, stride, part[warp]);
+        else mma_tile<NM, 2>(first, rows, k, begin, end, expert_smem, stride, part[warp]);
+        if (unit + 1 < unit_end) {
+            point(unit + 1);
+            first.load(rows, k, begin, end);
+        }
+        __syncthreads();
+        // entry (b, i) of lane (g, q): token 8 b + 2 q + i % 2, row g + 8 (i / 2)
+        for (int entry = warp; entry < NB * 4; entry += MMA_WARPS) {
+            const int t = (entry >> 2) * 8 + q * 2 + (entry & 1), row = tile * 16 + g + ((entry >> 1) & 1) * 8;
+            if (t >= count) continue;
+            const float sum = mma_sum<ENTRIES>(part, entry, lane);
+            if constexpr (UP) act[(size_t)pairs[t] * n_rows + row] = __float2bfloat16_rn(sum / (1.f + expf(-sum)) * mma_sum<ENTRIES>(part, NB * 4 + entry, lane));
+            else parts[(size_t)pairs[t] * n_rows + row] = sum;
+        }
+        // the next unit's first barrier stands before `part` is written again
+    }
+}
+
+// out_t = add_t (times add_weight_t) + the token's parts times their weights, in the order they were chosen
+template <typename T>
+__global__ void experts_join_kernel(const float* __restrict__ parts, const float* __restrict__ weights, const T* __restrict__ add,
+                                    const float* __restrict__ add_weight, float* __restrict__ out, int width, int top) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+    if (c >= width) return;
+    float acc = add != nullptr ? to_float(add[t * width + c]) : 0.f;
+    if (add_weight != nullptr) acc *= add_weight[t];
+    const float* p = parts + t * top * width + c;
+#pragma unroll 4
+    for (int kk = 0; kk < top; ++kk) acc = fmaf(weights[t * top + kk], p[(size_t)kk * width], acc);
+    out[t * width + c] = acc;
 }
 
 // ---- pairs in the order of their experts, for products that take all rows of an expert at once
@@ -591,49 +902,130 @@ GK_EXPORT int gk_route_groups(const void* h, int dtype, const float* w_router, c
     return GK_OK;
 }
 
-GK_EXPORT int gk_experts_up(const void* h, int dtype, const void* w_gate_up, int w_dtype, const int* ids, void* act, int n_tokens,
-                            int width, int ff, int top, void* stream) {
-    GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts_up: bad dtype");
-    GK_REQUIRE(width > 0 && ff > 0 && top > 0, "experts_up: bad sizes");
-    if (n_tokens == 0) return GK_OK;
-    const size_t smem = (size_t)width * sizeof(float);
-    GK_REQUIRE(smem <= 200 * 1024, "experts_up: rows of %d are longer than the kernel stages", width);
-    // few pairs: cut the expert's rows over more blocks, so that a single token still finds every SM a share
-    const long long pairs = (long long)n_tokens * top;
+namespace {
+
+// How the pairs of a step are dealt to blocks: by pair where those are fewer than the experts (blocks of an expert's later pairs
+// leave at once), else by expert; an expert's rows are cut into chunks so that every SM finds some blocks' worth of work even if
+// half of the pairs share their experts.
+struct ExpertGrid {
+    dim3 grid;
+    int rows, by_expert, at_once;
+    size_t smem;
+};
+
+ExpertGrid expert_grid(long long pairs, int n_experts, int n_rows, int row_length, int least_rows) {
+    ExpertGrid g;
+    g.by_expert = pairs > n_experts || pairs > LIST;
+    const long long items = g.by_expert ? n_experts : pairs;
     int chunks = 1;
-    while (pairs * chunks < 592 && ff / (chunks * 2) >= UP_WARPS) chunks *= 2;
-    const int rows = (ff + chunks - 1) / chunks;
-    GK_REQUIRE(pairs < 2147483647LL, "experts_up: too many pairs");
-    cudaStream_t s = (cudaStream_t)stream;
+    while (items * chunks < 1184 && n_rows / (chunks * 2) >= least_rows) chunks *= 2;
+    g.rows = (n_rows + chunks - 1) / chunks;
+    g.grid = dim3((unsigned)items, (n_rows + g.rows - 1) / g.rows, (unsigned)((pairs + LIST - 1) / LIST));
+    g.at_once = MAX_NT;
+    while (g.at_once > 1 && (size_t)g.at_once * row_length * sizeof(float) > 64 * 1024) g.at_once /= 2;
+    g.smem = (size_t)g.at_once * row_length * sizeof(float);
+    return g;
+}
+
+// Whole tiles: rows of k entries in pieces of 32, sixteen rows a tile; eight tokens' rows fit in shared memory, and so do
+// the experts' counts.
+bool mma_suits(int k, int n_rows, int n_experts) {
+    return k % 32 == 0 && n_rows % 16 == 0 && 8 * (size_t)mma_stride(k) <= 160 * 1024 && n_experts <= 4096;
+}
+
+constexpr size_t MMA_STATIC_SMEM = MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + MMA_WARPS * 2 * (MMA_TOKENS / 8 * 4) * 32 * sizeof(float) + 64;
+
+template <bool UP>
+void launch_mma(const void* source, const void* weights, const int* ids, void* act, float* parts, long long pairs, int n_tokens, int k, int n_rows, int divide,
+                int n_experts, cudaStream_t s) {
+    static const int sms = [] {
+        int device = 0, n = 0;
+        cudaGetDevice(&device);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+        return n > 0 ? n : 148;
+    }();
+    const int at_once = n_tokens > 8 && MMA_TOKENS * (size_t)mma_stride(k) <= 48 * 1024 ? MMA_TOKENS : 8;
+    const size_t rows = (size_t)at_once * mma_stride(k), counts = (2 * (size_t)n_experts + MMA_LIST) * 4, smem = rows > counts ? rows : counts;
+    // as many blocks as stay on the device at once: by their registers (the bound above) and by shared memory
+    const long long blocks = std::max(1LL, std::min(UP ? 3LL : 4LL, (long long)(227 * 1024 / (smem + MMA_STATIC_SMEM + 1024))));
+    const long long most = std::min(pairs, (long long)MMA_LIST) * (n_rows / 16), places = blocks * sms;
+    if (smem > 16 * 1024) cudaFuncSetAttribute(experts_mma_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    gk_launch(experts_mma_kernel<UP>, dim3((unsigned)std::min(most, places), 1, (unsigned)((pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32), smem, s,
+              (const __nv_bfloat16*)source, (const __nv_bfloat16*)weights, ids, (__nv_bfloat16*)act, parts, (int)pairs, k, n_rows, divide, n_experts, at_once);
+}
+
+int experts_up(const void* h, int dtype, const void* w_gate_up, int w_dtype, const int* ids, void* act, int n_tokens,
+                            int width, int ff, int top, int n_experts, cudaStream_t s) {
+    GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts_up: bad dtype");
+    GK_REQUIRE(width > 0 && ff > 0 && top > 0 && n_experts > 0, "experts_up: bad sizes");
+    GK_REQUIRE((size_t)width * sizeof(float) <= 200 * 1024, "experts_up: rows of %d are longer than the kernel stages", width);
+    const long long pairs = (long long)n_tokens * top;
+    GK_REQUIRE(pairs <= 65535LL * MMA_LIST, "experts_up: too many pairs");
+    if (dtype == GK_BF16 && w_dtype == GK_BF16 && mma_suits(width, ff, n_experts) && (((uintptr_t)h | (uintptr_t)w_gate_up) & 15) == 0) {
+        launch_mma<true>(h, w_gate_up, ids, act, nullptr, pairs, n_tokens, width, ff, top, n_experts, s);
+        GK_CHECK_LAUNCH("experts_up");
+        return GK_OK;
+    }
+    const ExpertGrid g = expert_grid(pairs, n_experts, ff, width, 2 * UP_WARPS);
     GK_DISPATCH_DTYPE(dtype, T, {
         GK_DISPATCH_DTYPE(w_dtype, TW, {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(experts_up_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            gk_launch(experts_up_kernel<T, TW>, dim3((unsigned)pairs, (ff + rows - 1) / rows), dim3(UP_WARPS * 32), smem, s, (const T*)h,
-                      (const TW*)w_gate_up, ids, (T*)act, width, ff, top, rows);
+            if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_up_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+            gk_launch(experts_up_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)h, (const TW*)w_gate_up, ids, (T*)act,
+                      (int)pairs, width, ff, top, g.rows, g.by_expert, g.at_once);
         })
     })
     GK_CHECK_LAUNCH("experts_up");
     return GK_OK;
 }
 
-GK_EXPORT int gk_experts_down(const void* act, int dtype, const void* w_down, int w_dtype, const int* ids, const float* weights,
-                              const void* add, const float* add_weight, float* out, int n_tokens, int width, int ff, int top, void* stream) {
+// parts: 32-bit scratch [n_tokens * top, width]
+int experts_down(const void* act, int dtype, const void* w_down, int w_dtype, const int* ids, const float* weights,
+                              const void* add, const float* add_weight, float* parts, float* out, int n_tokens, int width, int ff, int top,
+                              int n_experts, cudaStream_t s) {
     GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts_down: bad dtype");
-    GK_REQUIRE(width > 0 && ff > 0 && top > 0 && (add != nullptr || add_weight == nullptr), "experts_down: bad sizes");
-    if (n_tokens == 0) return GK_OK;
-    const size_t smem = (size_t)top * ff * sizeof(float);
-    GK_REQUIRE(smem <= 200 * 1024, "experts_down: %d experts of %d are more than the kernel stages", top, ff);
-    int chunks = 1;
-    while ((long long)n_tokens * chunks < 592 && width / (chunks * 2) >= UP_WARPS) chunks *= 2;
-    const int rows = (width + chunks - 1) / chunks;
-    cudaStream_t s = (cudaStream_t)stream;
-    GK_DISPATCH_DTYPE(dtype, T, {
-        GK_DISPATCH_DTYPE(w_dtype, TW, {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(experts_down_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            gk_launch(experts_down_kernel<T, TW>, dim3(n_tokens, (width + rows - 1) / rows), dim3(UP_WARPS * 32), smem, s, (const T*)act,
-                      (const TW*)w_down, ids, weights, (const T*)add, add_weight, out, width, ff, top, rows);
+    GK_REQUIRE(width > 0 && ff > 0 && top > 0 && n_experts > 0 && (add != nullptr || add_weight == nullptr), "experts_down: bad sizes");
+    GK_REQUIRE((size_t)top * ff * sizeof(float) <= 200 * 1024, "experts_down: %d experts of %d are more than the kernel stages", top, ff);
+    const long long pairs = (long long)n_tokens * top;
+    GK_REQUIRE(pairs <= 65535LL * MMA_LIST, "experts_down: too many pairs");
+    if (dtype == GK_BF16 && w_dtype == GK_BF16 && mma_suits(ff, width, n_experts) && (((uintptr_t)act | (uintptr_t)w_down) & 15) == 0) {
+        launch_mma<false>(act, w_down, ids, nullptr, parts, pairs, n_tokens, ff, width, 1, n_experts, s);
+    } else {
+        const ExpertGrid g = expert_grid(pairs, n_experts, width, ff, 4 * UP_WARPS);
+        GK_DISPATCH_DTYPE(dtype, T, {
+            GK_DISPATCH_DTYPE(w_dtype, TW, {
+                if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_down_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+                gk_launch(experts_down_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)act, (const TW*)w_down, ids, parts,
+                          (int)pairs, width, ff, g.rows, g.by_expert, g.at_once);
+            })
         })
-    })
+    }
     GK_CHECK_LAUNCH("experts_down");
+    GK_DISPATCH_DTYPE(dtype, T, {
+        gk_launch(experts_join_kernel<T>, dim3(n_tokens, (width + 255) / 256), dim3(256), 0, s, (const float*)parts, weights, (const T*)add,
+                  add_weight, out, width, top);
+    })
+    GK_CHECK_LAUNCH("experts_join");
+    return GK_OK;
+}
+
+}  // namespace
+
+// The whole routed feed-forward behind the router.  `work`: 32-bit scratch of `at_once` rows of top * (width + ff) numbers; more
+// tokens than that go in several turns.
+GK_EXPORT int gk_experts(const void* h, int dtype, const void* w_gate_up, const void* w_down, int w_dtype, const int* ids, const float* weights,
+                         const void* add, const float* add_weight, float* work, float* out, int n_tokens, int at_once, int width, int ff, int top,
+                         int n_experts, void* stream) {
+    GK_REQUIRE(GK_VALID_DTYPE(dtype) && at_once > 0 && width > 0 && ff > 0 && top > 0, "experts: bad sizes");
+    const size_t size = dtype == GK_F32 ? 4 : 2;
+    for (int at = 0; at < n_tokens; at += at_once) {
+        const int n = std::min(at_once, n_tokens - at);
+        const size_t row = (size_t)at * width;
+        void* act = work + (size_t)at_once * top * width;
+        int status = experts_up((const char*)h + row * size, dtype, w_gate_up, w_dtype, ids + (size_t)at * top, act, n, width, ff, top, n_experts, (cudaStream_t)stream);
+        if (status == GK_OK)
+            status = experts_down(act, dtype, w_down, w_dtype, ids + (size_t)at * top, weights + (size_t)at * top, add ? (const char*)add + row * size : nullptr,
+                                  add_weight ? add_weight + at : nullptr, work, out + row, n, width, ff, top, n_experts, (cudaStream_t)stream);
+        if (status != GK_OK) return status;
+    }
     return GK_OK;
 }

@@ -1544,10 +1544,13 @@ def route_groups(h: torch.Tensor, w_router: torch.Tensor, correction: torch.Tens
     return (ids, weights) if share is None else (ids, weights, share)
 
 
+EXPERT_PAIRS_AT_ONCE = 8192
+
+
 def experts_pairwise(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, ids: torch.Tensor, weights: torch.Tensor,
                      add: torch.Tensor | None = None, add_weight: torch.Tensor | None = None) -> torch.Tensor:
-    """``add + sum_k weights[t, k] * down_e(silu(gate_e h_t) * up_e h_t)`` with ``e = ids[t, k]``, a (token, expert) pair
-    at a time (``add`` times ``add_weight [T]`` where given).  ``w_gate_up [E, 2, ff, width]``, ``w_down [E, width, ff]``.  Returns
+    """``add + sum_k weights[t, k] * down_e(silu(gate_e h_t) * up_e h_t)`` with ``e = ids[t, k]``, the pairs of an expert
+    together (``add`` times ``add_weight [T]`` where given).  ``w_gate_up [E, 2, ff, width]``, ``w_down [E, width, ff]``.  Returns
     32-bit ``[T, width]``."""
     require_device(h.device)
     _check(h, "h", dims=2)
@@ -1562,12 +1565,12 @@ def experts_pairwise(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Ten
         raise KernelError("experts: weight shapes do not fit")
     if add is not None:
         _check(add, "add", h.dtype, 2)
-    act = torch.empty((T * top, ff), dtype=h.dtype, device=h.device)
     out = torch.empty((T, width), dtype=torch.float32, device=h.device)
-    call("gk_experts_up", ptr(h), dtype_code(h.dtype), ptr(w_gate_up), dtype_code(w_gate_up.dtype), ptr(ids), ptr(act), T, width, ff,
-         top, stream_ptr())
-    call("gk_experts_down", ptr(act), dtype_code(h.dtype), ptr(w_down), dtype_code(w_down.dtype), ptr(ids), ptr(weights), ptr(add),
-         ptr(add_weight), ptr(out), T, width, ff, top, stream_ptr())
+    # scratch for every pair's inner values and output; long prompts of 32-bit runs go some thousand pairs at a time
+    at_once = max(1, min(T, EXPERT_PAIRS_AT_ONCE // top))
+    work = torch.empty((at_once * top, width + ff), dtype=torch.float32, device=h.device)
+    call("gk_experts", ptr(h), dtype_code(h.dtype), ptr(w_gate_up), ptr(w_down), dtype_code(w_gate_up.dtype), ptr(ids), ptr(weights), ptr(add),
+         ptr(add_weight), ptr(work), ptr(out), T, at_once, width, ff, top, E, stream_ptr())
     return out
 
 

@@ -562,3 +562,31 @@ def test_a_loop_around_blocks_that_leave_the_adds_to_the_model():
                 want = plan.head.forward(plan.final_norm.forward(h, None, torch.float32, rows=ctx.want_rows))
         assert done[start] == times and len(plan.run_list) == n + (times - 1) * (stop - start)
         assert (_wide(got) - _wide(want)).abs().max().item() < 2e-5 * (1.0 + want.abs().max().item())
+
+
+@pytest.mark.parametrize("tokens,width,ff,experts,top", [(1, 64, 32, 4, 2), (3, 96, 48, 5, 1), (9, 2048, 32, 3, 3), (33, 128, 160, 2, 2), (40, 1024, 768, 32, 4),
+                                                         (700, 64, 32, 5, 2), (5, 40, 24, 4, 2), (21, 70, 30, 3, 2), (2, 8192, 16, 2, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_take_each_expert_once_for_all_its_tokens(tokens, width, ff, experts, top, dtype):
+    """Experts with one token, with more tokens than a product's columns (8, 16) and with lists of more than 512 and 1,024 pairs;
+    sizes in whole tiles and beside them.  A token's result is that of a call of its own."""
+    gen = torch.Generator().manual_seed(tokens * width + ff)
+    draw = lambda *shape: torch.randn(shape, generator=gen)
+    h = draw(tokens, width).to(dtype)
+    gate_up, down = (draw(experts, 2, ff, width) * width**-0.5).to(dtype), (draw(experts, width, ff) * ff**-0.5).to(dtype)
+    ids = torch.stack([torch.randperm(experts, generator=gen)[:top] for _ in range(tokens)]).to(torch.int32)
+    weights, add = torch.rand(tokens, top, generator=gen), draw(tokens, width).to(dtype)
+    dev = [t.cuda() for t in (h, gate_up, down, ids, weights, add)]
+    got = F().experts_pairwise(*dev[:5], dev[5])
+    want = add.double()
+    for t in range(tokens) if tokens < 100 else (0, 255, 256, 511, 512, 699):
+        for e, w in zip(ids[t].tolist(), weights[t].double()):
+            z = gate_up[e].double() @ h[t].double()
+            act = (torch.nn.functional.silu(z[0]) * z[1]).to(dtype).double()
+            want[t] += w * (down[e].double() @ act)
+        # the inner values round to bfloat16 on either side of a tie: 2^-9 of them, through a sum of ff products
+        tol = 2e-5 if dtype == torch.float32 else 2.0**-9 * 6 * top
+        assert (got[t].double().cpu() - want[t]).abs().max() < tol, f"token {t}"
+    for t in (0, tokens // 2, tokens - 1):
+        one = F().experts_pairwise(dev[0][t:t + 1], dev[1], dev[2], dev[3][t:t + 1].contiguous(), dev[4][t:t + 1].contiguous(), dev[5][t:t + 1])
+        assert torch.equal(one[0], got[t])
