@@ -32,6 +32,10 @@ namespace {
 constexpr int ROUTE_WARPS = 4;
 
 
+// Loads of several elements want their address on as many bytes: a row length that is a multiple of them says so only where the
+// matrix starts on them (a view into a larger buffer may start anywhere).
+__device__ __forceinline__ bool starts_on(const void* p, int bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; }
+
 // four neighbouring numbers of a row (which start on four elements), zeros where `in` is false
 template <typename T>
 __device__ __forceinline__ void load_four(const T* p, bool in, float (&v)[4]) {
@@ -67,7 +71,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_scores_kernel(const T*
     for (int a = 0; a < SCORE_TOKENS; ++a)
 #pragma unroll
         for (int j = 0; j < SCORE_EXPERTS; ++j) acc[a][j] = 0.f;
-    if (width % 4 == 0) {  // four neighbouring elements a lane and turn
+    if (width % 4 == 0 && starts_on(h, 4 * sizeof(T)) && starts_on(w_router, 16)) {  // four neighbouring elements a lane and turn
 #pragma unroll (SCORE_EXPERTS == 2 ? 4 : 2)
         for (int i = lane * 4; i < width; i += 128) {
             float xv[SCORE_TOKENS][4], wv[SCORE_EXPERTS][4];
@@ -292,17 +296,20 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_choose_kernel(
     }
 }
 
+template <typename TW>
+__device__ __forceinline__ bool wide_rows(const TW* matrix, int n) { return n % (16 / (int)sizeof(TW)) == 0 && starts_on(matrix, 16); }
+
 // A lane's share of the dot products of NR rows in memory with NT vectors in shared memory (`stride` apart), each summed in
 // index order; the rows' loads are independent, so all of them are on their way together, and a piece of a vector is read once
-// for all rows.  The caller finishes each with warp_sum.
+// for all rows.  `wide` (wide_rows): 16-byte loads.  The caller finishes each with warp_sum.
 template <typename TW, int NR, int NT>
-__device__ __forceinline__ void dot_many(const float* __restrict__ x, int stride, const TW* const (&rows)[NR], int n, int lane, float (&acc)[NT][NR]) {
+__device__ __forceinline__ void dot_many(const float* __restrict__ x, int stride, const TW* const (&rows)[NR], int n, bool wide, int lane, float (&acc)[NT][NR]) {
 #pragma unroll
     for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int j = 0; j < NR; ++j) acc[t][j] = 0.f;
     constexpr int VEC = 16 / sizeof(TW);
-    if (n % VEC == 0) {
+    if (wide) {
 #pragma unroll 2
         for (int i = lane * VEC; i < n; i += 32 * VEC) {
             uint4 raw[NR];
@@ -380,14 +387,14 @@ __device__ __forceinline__ int list_pairs(const int* __restrict__ ids, int n_pai
 
 // act[pair] = silu(gate) * up for NT pairs of one expert (their tokens' rows in `xs`), rows f0 .. f_end - 1
 template <typename T, typename TW, int NT>
-__device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int count, const TW* wg, const TW* wu, T* __restrict__ act, int width, int ff, int f0, int f_end) {
+__device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int count, const TW* wg, const TW* wu, T* __restrict__ act, int width, int ff, bool wide, int f0, int f_end) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int f = f0 + warp;
     for (; f + UP_WARPS < f_end; f += 2 * UP_WARPS) {  // two rows of gate and of up at once: four rows' loads in flight
         const TW* const rows[4] = {wg + (size_t)f * width, wu + (size_t)f * width, wg + (size_t)(f + UP_WARPS) * width,
                                    wu + (size_t)(f + UP_WARPS) * width};
         float part[NT][4];
-        dot_many<TW, 4, NT>(xs, width, rows, width, lane, part);
+        dot_many<TW, 4, NT>(xs, width, rows, width, wide, lane, part);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
 #pragma unroll
@@ -402,7 +409,7 @@ __device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int c
     for (; f < f_end; f += UP_WARPS) {
         const TW* const rows[2] = {wg + (size_t)f * width, wu + (size_t)f * width};
         float part[NT][2];
-        dot_many<TW, 2, NT>(xs, width, rows, width, lane, part);
+        dot_many<TW, 2, NT>(xs, width, rows, width, wide, lane, part);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const float gate = warp_sum(part[t][0]), up = warp_sum(part[t][1]);
@@ -427,6 +434,7 @@ __global__ void __launch_bounds__(UP_WARPS * 32) experts_up_kernel(
     const TW* wg = w_gate_up + (size_t)e * 2 * ff * width;
     const TW* wu = wg + (size_t)ff * width;
     const int f0 = blockIdx.y * rows_per_block, f_end = min(ff, f0 + rows_per_block);
+    const bool wide = wide_rows(w_gate_up, width);
     for (int at = 0; at < n; at += at_once) {
         const int count = min(at_once, n - at);
         __syncthreads();
@@ -435,20 +443,20 @@ __global__ void __launch_bounds__(UP_WARPS * 32) experts_up_kernel(
             for (int i = threadIdx.x; i < width; i += UP_WARPS * 32) xs[k * width + i] = to_float(x[i]);
         }
         __syncthreads();
-        if (count == 1) up_rows<T, TW, 1>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
-        else if (count == 2) up_rows<T, TW, 2>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
-        else up_rows<T, TW, MAX_NT>(xs, list + at, count, wg, wu, act, width, ff, f0, f_end);
+        if (count == 1) up_rows<T, TW, 1>(xs, list + at, count, wg, wu, act, width, ff, wide, f0, f_end);
+        else if (count == 2) up_rows<T, TW, 2>(xs, list + at, count, wg, wu, act, width, ff, wide, f0, f_end);
+        else up_rows<T, TW, MAX_NT>(xs, list + at, count, wg, wu, act, width, ff, wide, f0, f_end);
     }
 }
 
 template <typename TW, int NT>
-__device__ __forceinline__ void down_rows(const float* as, const int* pairs, int count, const TW* w, float* __restrict__ parts, int width, int ff, int c0, int c_end) {
+__device__ __forceinline__ void down_rows(const float* as, const int* pairs, int count, const TW* w, float* __restrict__ parts, int width, int ff, bool wide, int c0, int c_end) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int c = c0 + 4 * warp; c < c_end; c += 4 * UP_WARPS) {
         if (c + 4 <= c_end) {  // four rows' loads in flight
             const TW* const rows[4] = {w + (size_t)c * ff, w + (size_t)(c + 1) * ff, w + (size_t)(c + 2) * ff, w + (size_t)(c + 3) * ff};
             float part[NT][4];
-            dot_many<TW, 4, NT>(as, ff, rows, ff, lane, part);
+            dot_many<TW, 4, NT>(as, ff, rows, ff, wide, lane, part);
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 float mine = 0.f;
@@ -463,7 +471,7 @@ __device__ __forceinline__ void down_rows(const float* as, const int* pairs, int
             for (int cc = c; cc < c_end; ++cc) {
                 const TW* const rows[1] = {w + (size_t)cc * ff};
                 float part[NT][1];
-                dot_many<TW, 1, NT>(as, ff, rows, ff, lane, part);
+                dot_many<TW, 1, NT>(as, ff, rows, ff, wide, lane, part);
 #pragma unroll
                 for (int t = 0; t < NT; ++t) {
                     const float sum = warp_sum(part[t][0]);
@@ -488,6 +496,7 @@ __global__ void __launch_bounds__(UP_WARPS * 32) experts_down_kernel(
     const int n = list_pairs<UP_WARPS>(ids, n_pairs, blockIdx.z * LIST, by_expert != 0, e, list, scratch);
     const TW* w = w_down + (size_t)e * width * ff;
     const int c0 = blockIdx.y * rows_per_block, c_end = min(width, c0 + rows_per_block);
+    const bool wide = wide_rows(w_down, ff);
     for (int at = 0; at < n; at += at_once) {
         const int count = min(at_once, n - at);
         __syncthreads();
@@ -496,9 +505,9 @@ __global__ void __launch_bounds__(UP_WARPS * 32) experts_down_kernel(
             for (int i = threadIdx.x; i < ff; i += UP_WARPS * 32) as[k * ff + i] = to_float(x[i]);
         }
         __syncthreads();
-        if (count == 1) down_rows<TW, 1>(as, list + at, count, w, parts, width, ff, c0, c_end);
-        else if (count == 2) down_rows<TW, 2>(as, list + at, count, w, parts, width, ff, c0, c_end);
-        else down_rows<TW, MAX_NT>(as, list + at, count, w, parts, width, ff, c0, c_end);
+        if (count == 1) down_rows<TW, 1>(as, list + at, count, w, parts, width, ff, wide, c0, c_end);
+        else if (count == 2) down_rows<TW, 2>(as, list + at, count, w, parts, width, ff, wide, c0, c_end);
+        else down_rows<TW, MAX_NT>(as, list + at, count, w, parts, width, ff, wide, c0, c_end);
     }
 }
 
@@ -799,7 +808,7 @@ __global__ void gather_rows_kernel(const T* __restrict__ x, const int* __restric
     const size_t place = blockIdx.x;
     const T* src = x + (size_t)(pair_at[place] / top) * width;
     T* dst = out + place * width;
-    if ((width * sizeof(T)) % 16 == 0) {
+    if ((width * sizeof(T)) % 16 == 0 && starts_on(x, 16) && starts_on(out, 16)) {
         const int n16 = width * (int)sizeof(T) / 16;
         for (int i = threadIdx.x; i < n16; i += blockDim.x) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
     } else {

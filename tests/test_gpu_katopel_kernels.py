@@ -590,3 +590,31 @@ def test_experts_take_each_expert_once_for_all_its_tokens(tokens, width, ff, exp
     for t in (0, tokens // 2, tokens - 1):
         one = F().experts_pairwise(dev[0][t:t + 1], dev[1], dev[2], dev[3][t:t + 1].contiguous(), dev[4][t:t + 1].contiguous(), dev[5][t:t + 1])
         assert torch.equal(one[0], got[t])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("width,ff", [(64, 32), (40, 24)])
+def test_routed_experts_on_matrices_that_start_anywhere(width, ff, dtype):
+    """Views that start one element into their buffer, with row lengths that would allow 16-byte loads: router scores, the experts'
+    products and the rows copied into the experts' order take them element by element."""
+    tokens, experts, top = 5, 4, 2
+    gen = torch.Generator().manual_seed(width)
+
+    def beside(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+        flat[1:] = t.reshape(-1).cuda()
+        return flat[1:].view(t.shape)
+
+    h = torch.randn(tokens, width, generator=gen).to(dtype)
+    router, correction = torch.randn(experts, width, generator=gen), torch.zeros(experts)
+    gate_up = (torch.randn(experts, 2, ff, width, generator=gen) * width**-0.5).to(dtype)
+    down = (torch.randn(experts, width, ff, generator=gen) * ff**-0.5).to(dtype)
+    straight = F().route_groups(h.cuda(), router.cuda(), correction.cuda(), top, 1, 1, 1.0)
+    ids, weights = F().route_groups(beside(h), beside(router), correction.cuda(), top, 1, 1, 1.0)
+    assert torch.equal(ids, straight[0]) and (weights - straight[1]).abs().max() < 1e-5
+    want = F().experts_pairwise(h.cuda(), gate_up.cuda(), down.cuda(), ids, weights)
+    got = F().experts_pairwise(beside(h), beside(gate_up), beside(down), ids, weights)
+    # inner values that round to bfloat16 on either side of a tie: 2^-9 of them, through a sum of ff products
+    assert (got - want).abs().max() < (2e-5 if dtype == torch.float32 else 2.0**-9 * 6 * top)
+    _, _, pair_at = F().experts_sort(ids, experts)
+    assert torch.equal(F().gather_rows(beside(h), pair_at, top), F().gather_rows(h.cuda(), pair_at, top))
