@@ -618,3 +618,12 @@ def test_routed_experts_on_matrices_that_start_anywhere(width, ff, dtype):
     assert (got - want).abs().max() < (2e-5 if dtype == torch.float32 else 2.0**-9 * 6 * top)
     _, _, pair_at = F().experts_sort(ids, experts)
     assert torch.equal(F().gather_rows(beside(h), pair_at, top), F().gather_rows(h.cuda(), pair_at, top))
+
+
+def test_experts_without_a_choice_are_refused():
+    """No expert a token is an error of the library like every other bad size."""
+    from gtar_kimik3_public_b200.ops.library import KernelError
+
+    h, gate_up, down = torch.randn(2, 16).cuda(), torch.randn(3, 2, 8, 16).cuda(), torch.randn(3, 16, 8).cuda()
+    with pytest.raises(KernelError):
+        F().experts_pairwise(h, gate_up, down, torch.empty(2, 0, dtype=torch.int32, device="cuda"), torch.empty(2, 0, device="cuda"))
