@@ -16,14 +16,16 @@
 //   experts_down (and experts_join behind it) out_t = add_t (times a number per token, where one is given) + sum over the token's pairs, in the order they were chosen, of weight * W_down[e] act[pair]
 //                (32-bit result: it is what goes into the residual stream)
 //
-// The expert kernels take an expert's pairs together, so that its rows are fetched once for them: the path of few-token steps,
-// of 32-bit runs and of sizes the sorted path does not take.  A token's result depends on the token alone.
+// This is the path of few-token steps, of 32-bit runs and of sizes the sorted path does not take.  Its kernels come in two forms with
+// the same sums: an expert's pairs together, so that its rows are fetched once for several of them, and, where the pairs' experts
+// are nearly all different or small, a pair and a token by itself (`experts` below).  A token's result depends on the token alone.
 //
 //   sort, gather_rows, combine   many-token steps: the pairs put in the order of their experts, the tokens' rows copied
 //                into that order (each expert's rows then go through one tensor-core product, made by the caller), and
 //                the weighted sum of a token's expert outputs in the order the experts were chosen
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -386,7 +388,7 @@ __device__ __forceinline__ int list_pairs(const int* __restrict__ ids, int n_pai
 }
 
 // act[pair] = silu(gate) * up for NT pairs of one expert (their tokens' rows in `xs`), rows f0 .. f_end - 1
-template <typename T, typename TW, int NT>
+template <typename T, typename TW, int NT, bool LISTED = true>
 __device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int count, const TW* wg, const TW* wu, T* __restrict__ act, int width, int ff, bool wide, int f0, int f_end) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int f = f0 + warp;
@@ -394,7 +396,7 @@ __device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int c
         const TW* const rows[4] = {wg + (size_t)f * width, wu + (size_t)f * width, wg + (size_t)(f + UP_WARPS) * width,
                                    wu + (size_t)(f + UP_WARPS) * width};
         float part[NT][4];
-        dot_many<TW, 4, NT>(xs, width, rows, width, wide, lane, part);
+        dot_many<TW, 4, NT>(xs, width, rows, width, LISTED ? wide : wide_rows(rows[0], width), lane, part);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
 #pragma unroll
@@ -409,7 +411,7 @@ __device__ __forceinline__ void up_rows(const float* xs, const int* pairs, int c
     for (; f < f_end; f += UP_WARPS) {
         const TW* const rows[2] = {wg + (size_t)f * width, wu + (size_t)f * width};
         float part[NT][2];
-        dot_many<TW, 2, NT>(xs, width, rows, width, wide, lane, part);
+        dot_many<TW, 2, NT>(xs, width, rows, width, LISTED ? wide : wide_rows(rows[0], width), lane, part);
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
             const float gate = warp_sum(part[t][0]), up = warp_sum(part[t][1]);
@@ -511,21 +513,119 @@ __global__ void __launch_bounds__(UP_WARPS * 32) experts_down_kernel(
     }
 }
 
+// ---- a pair, a token at a time: every pair streams its expert's rows by itself.  The sums are those of the kernels above.  Measured
+// (us, lists / here): 64 tokens, 2 of 6 experts of 70 x 30: 55 / 5.9; 256 tokens, 2 of 8 of 256 x 128, 32-bit: 111 / 33.
+
+// grid (pairs, chunks of ff)
+template <typename T, typename TW>
+__global__ void __launch_bounds__(UP_WARPS * 32, 4) pair_up_kernel(const T* __restrict__ h, const TW* __restrict__ w_gate_up, const int* __restrict__ ids,
+                                                                T* __restrict__ act, int width, int ff, int top, int rows_per_block) {
+    extern __shared__ __align__(16) unsigned char expert_smem[];
+    float* xs = reinterpret_cast<float*>(expert_smem);  // [width]
+    pdl_launch_dependents();
+    pdl_wait();
+    const int pair = blockIdx.x;
+    const TW* wg = w_gate_up + (size_t)ids[pair] * 2 * ff * width;
+    const T* x = h + (size_t)(pair / top) * width;
+    for (int i = threadIdx.x; i < width; i += UP_WARPS * 32) xs[i] = to_float(x[i]);
+    __syncthreads();
+    const int f0 = blockIdx.y * rows_per_block;
+    up_rows<T, TW, 1, false>(xs, &pair, 1, wg, wg + (size_t)ff * width, act, width, ff, false, f0, min(ff, f0 + rows_per_block));
+}
+
+// The dot products of NR vectors in shared memory, `stride` apart, with a row of their own each (dot_many's order).
+template <typename TW, int NR>
+__device__ __forceinline__ void dot_pairs(const float* __restrict__ x, int stride, const TW* const (&rows)[NR], int n, int lane, float (&acc)[NR]) {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) acc[j] = 0.f;
+    constexpr int VEC = 16 / sizeof(TW);
+    if (n % VEC == 0 && starts_on(rows[0], 16)) {  // the other rows are whole rows away
+#pragma unroll 2
+        for (int i = lane * VEC; i < n; i += 32 * VEC) {
+            uint4 raw[NR];
+#pragma unroll
+            for (int j = 0; j < NR; ++j) raw[j] = *reinterpret_cast<const uint4*>(rows[j] + i);
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                const float* xj = x + j * stride + i;
+                if constexpr (sizeof(TW) == 2) {
+                    const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&raw[j]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float2 f = __bfloat1622float2(p[c]);
+                        acc[j] = fmaf(xj[2 * c], f.x, acc[j]);
+                        acc[j] = fmaf(xj[2 * c + 1], f.y, acc[j]);
+                    }
+                } else {
+                    const float* f = reinterpret_cast<const float*>(&raw[j]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[j] = fmaf(xj[c], f[c], acc[j]);
+                }
+            }
+        }
+    } else {
+        for (int i = lane; i < n; i += 32)
+#pragma unroll
+            for (int j = 0; j < NR; ++j) acc[j] = fmaf(x[j * stride + i], to_float(rows[j][i]), acc[j]);
+    }
+}
+
+template <int N>
+struct Count {
+    static constexpr int value = N;
+};
+
+// grid (tokens, chunks of width): the down product of a token's pairs and their sum
+template <typename T, typename TW>
+__global__ void __launch_bounds__(UP_WARPS * 32) token_down_kernel(const T* __restrict__ act, const TW* __restrict__ w_down, const int* __restrict__ ids,
+                                                                   const float* __restrict__ weights, const T* __restrict__ add,
+                                                                   const float* __restrict__ add_weight, float* __restrict__ out, int width, int ff,
+                                                                   int top, int rows_per_block) {
+    extern __shared__ __align__(16) unsigned char expert_smem[];
+    float* as = reinterpret_cast<float*>(expert_smem);  // [top][ff]
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    for (int i = threadIdx.x; i < top * ff; i += UP_WARPS * 32) as[i] = to_float(act[t * top * ff + i]);
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.y * rows_per_block;
+    for (int c = c0 + warp; c < min(width, c0 + rows_per_block); c += UP_WARPS) {
+        float acc = add != nullptr ? to_float(add[t * width + c]) : 0.f;
+        if (add_weight != nullptr) acc *= add_weight[t];
+        int kk = 0;
+        const auto add_pairs = [&](auto count) {  // their rows in flight together; the sum still takes them in the order they were chosen
+            constexpr int NR = decltype(count)::value;
+            const TW* rows[NR];
+            float part[NR];
+#pragma unroll
+            for (int j = 0; j < NR; ++j) rows[j] = w_down + ((size_t)ids[t * top + kk + j] * width + c) * ff;
+            dot_pairs<TW, NR>(as + (size_t)kk * ff, ff, rows, ff, lane, part);
+#pragma unroll
+            for (int j = 0; j < NR; ++j) acc = fmaf(weights[t * top + kk + j], warp_sum(part[j]), acc);
+            kk += NR;
+        };
+        while (kk + 4 <= top) add_pairs(Count<4>{});
+        if (kk + 2 <= top) add_pairs(Count<2>{});
+        if (kk < top) add_pairs(Count<1>{});
+        if (lane == 0) out[t * width + c] = acc;
+    }
+}
+
 // ---- the same products on the tensor cores, for bfloat16 rows and weights of sizes in whole tiles (mma.sync m16n8k16, 32-bit sums)
 //
 // A block has sixteen rows of an expert's matrix at a time (of gate and of up together), each of its four warps a quarter of
 // the reduction, and the tokens that chose the expert are the product's columns, eight or sixteen of them.  The order in which
 // a product walks k is free as long as both operands take the same one, so a lane reads eight neighbouring entries of its row
 // at once (16 bytes) and they serve as its fragments of two products; the tokens' rows lie in shared memory and are read the
-// same way.  What remains is the stream of the weights, every expert's rows once whatever number of tokens chose it.  Blocks stay
+// same way.  What remains is the stream of the weights, an expert's rows once for sixteen of its tokens (for eight where rows are longer
+// than some 1,500 entries: two blocks an SM would not hold sixteen) and for every list of 512 pairs.  Blocks stay
 // and take equal runs of (expert, sixteen rows) units: the experts that were chosen are listed by every block for itself, and a
 // warp asks for its first rows of the next unit before it adds up this one's.  (One block a pair and chunk of rows, most of
 // which found that another had their expert, spent their time in the chain ids - list - weights - tokens: 60 us where the
 // weights take 21.)  (Tensor-memory products would want 128 rows a tile and the weights through shared memory, for a
 // step that does next to no arithmetic.)
-// Measured (us; up, down and join; 6 of 64 experts of 2,048 x 1,024), before (every pair streamed its expert's rows by itself, a
-// row a warp on the FP32 pipes) and now: 2 tokens 51 / 45, 4: 88 / 53, 8: 159 / 73 (16 experts: 2.8 TB/s), 16: 298 / 99, 42:
-// 739 / 166; 4 of 32 experts of 1,024 x 768: one token 10 / 12, 3: 19 / 15, 8: 39 / 24, 63: 260 / 46.
+// Measured (us; up, down and join; 6 of 64 experts of 2,048 x 1,024), every pair by itself on the FP32 pipes and here: 4 tokens 93 / 88,
+// 8: 170 / 121 (experts drawn at random), 16: 319 / 173, 42: 763 / 248; 4 of 32 experts of 1,024 x 768: 8 tokens 43 / 38, 63: 265 / 66.
 constexpr int MMA_WARPS = 4, MMA_STEPS = 2, MMA_TOKENS = 16, MMA_LIST = 512;
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -749,6 +849,107 @@ __global__ void __launch_bounds__(MMA_WARPS * 32, UP ? 3 : 4) experts_mma_kernel
     }
 }
 
+// ---- the same for so few pairs that their experts are nearly all different: no list, no third kernel, and a pair's row is the
+// product's column (all eight of them).  A column's sums are those of the kernel above, so a token's result does not depend on
+// which of the two its step takes.  Bound by two launches and the chain ids - rows - sums in each of them; a block asks for all of
+// its rows (64 KB of gate and up at 1,024) at once.
+// Measured (us), every pair by itself on the FP32 pipes / lists / here: 4 of 32 experts of 1,024 x 768: one token 9.4 / 11.7 / 8.4, 3:
+// 18.5 / 19.4 / 13.4; 6 of 64 of 2,048 x 1,024, one token: 26.6 / 21.4 / 19.1; 2 of 8 of 256 x 128: one token 4.3 / 8.8 / 4.5, 64: 12.7 /
+// 13.5 / 10.2.
+
+// This warp's quarter of sixteen rows of NM matrices (row0: this lane's row of each) times one vector: the sums of column 0 come to
+// rest in lanes 0, 4, ... 28, rows lane / 4 and lane / 4 + 8.
+template <int NM>
+__device__ __forceinline__ void mma_column(const __nv_bfloat16* const (&row0)[NM], const __nv_bfloat16* __restrict__ x, int k, int begin, int end, float (&sums)[NM][4]) {
+    constexpr int STEPS = 4;
+    const __nv_bfloat16* x_at = x + (threadIdx.x & 3) * 8;
+#pragma unroll
+    for (int m = 0; m < NM; ++m)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sums[m][e] = 0.f;
+    for (int i = begin; i < end; i += STEPS) {
+        uint4 lo[STEPS][NM], hi[STEPS][NM], xv[STEPS];
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u)
+            if (i + u < end) {
+#pragma unroll
+                for (int m = 0; m < NM; ++m) {
+                    const __nv_bfloat16* at = row0[m] + (i + u) * 32;
+                    lo[u][m] = *reinterpret_cast<const uint4*>(at);
+                    hi[u][m] = *reinterpret_cast<const uint4*>(at + (size_t)8 * k);
+                }
+                xv[u] = *reinterpret_cast<const uint4*>(x_at + (i + u) * 32);
+            }
+#pragma unroll
+        for (int u = 0; u < STEPS; ++u)
+            if (i + u < end) {
+#pragma unroll
+                for (int m = 0; m < NM; ++m) {
+                    mma_bf16(sums[m], lo[u][m].x, hi[u][m].x, lo[u][m].y, hi[u][m].y, xv[u].x, xv[u].y);
+                    mma_bf16(sums[m], lo[u][m].z, hi[u][m].z, lo[u][m].w, hi[u][m].w, xv[u].z, xv[u].w);
+                }
+            }
+    }
+}
+
+// grid (pairs, tiles of sixteen rows)
+__global__ void __launch_bounds__(MMA_WARPS * 32) pair_up_mma_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ weights,
+                                                                     const int* __restrict__ ids, __nv_bfloat16* __restrict__ act, int k, int n_rows, int top) {
+    __shared__ float part[MMA_WARPS][2][16];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int pair = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const int pieces = k / 32, share = (pieces + MMA_WARPS - 1) / MMA_WARPS, begin = min(warp * share, pieces), end = min(begin + share, pieces);
+    const __nv_bfloat16* gate = weights + (size_t)ids[pair] * 2 * n_rows * k + (size_t)(blockIdx.y * 16 + g) * k + q * 8;
+    const __nv_bfloat16* const rows[2] = {gate, gate + (size_t)n_rows * k};
+    float sums[2][4];
+    mma_column<2>(rows, h + (size_t)(pair / top) * k, k, begin, end, sums);
+    if (q == 0) {
+#pragma unroll
+        for (int m = 0; m < 2; ++m) part[warp][m][g] = sums[m][0], part[warp][m][g + 8] = sums[m][2];
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        const int r = threadIdx.x;
+        const float z = ((part[0][0][r] + part[1][0][r]) + part[2][0][r]) + part[3][0][r], up = ((part[0][1][r] + part[1][1][r]) + part[2][1][r]) + part[3][1][r];
+        act[(size_t)pair * n_rows + blockIdx.y * 16 + r] = __float2bfloat16_rn(z / (1.f + expf(-z)) * up);
+    }
+}
+
+// grid (tokens, tiles of sixteen columns of the result): four warps a pair, up to TOKEN_PAIRS pairs of the token at a time
+constexpr int TOKEN_PAIRS = 4;
+__global__ void __launch_bounds__(TOKEN_PAIRS * MMA_WARPS * 32) token_down_mma_kernel(
+    const __nv_bfloat16* __restrict__ act, const __nv_bfloat16* __restrict__ weights, const int* __restrict__ ids, const float* __restrict__ pair_weights,
+    const __nv_bfloat16* __restrict__ add, const float* __restrict__ add_weight, float* __restrict__ out, int k, int n_rows, int top) {
+    __shared__ float part[2][TOKEN_PAIRS][MMA_WARPS][16];
+    pdl_launch_dependents();
+    pdl_wait();
+    const size_t t = blockIdx.x;
+    const int lane = threadIdx.x & 31, group = threadIdx.x / (MMA_WARPS * 32), groups = blockDim.x / (MMA_WARPS * 32), warp = (threadIdx.x >> 5) % MMA_WARPS;
+    const int g = lane >> 2, q = lane & 3, column = blockIdx.y * 16 + threadIdx.x;
+    const int pieces = k / 32, share = (pieces + MMA_WARPS - 1) / MMA_WARPS, begin = min(warp * share, pieces), end = min(begin + share, pieces);
+    float acc = 0.f;
+    if (threadIdx.x < 16 && add != nullptr) acc = to_float(add[t * n_rows + column]);
+    if (threadIdx.x < 16 && add_weight != nullptr) acc *= add_weight[t];
+    for (int kk0 = 0, turn = 0; kk0 < top; kk0 += groups, turn ^= 1) {
+        const int kk = kk0 + group;
+        if (kk < top) {
+            const __nv_bfloat16* const rows[1] = {weights + (size_t)ids[t * top + kk] * n_rows * k + (size_t)(blockIdx.y * 16 + g) * k + q * 8};
+            float sums[1][4];
+            mma_column<1>(rows, act + (t * top + kk) * k, k, begin, end, sums);
+            if (q == 0) part[turn][group][warp][g] = sums[0][0], part[turn][group][warp][g + 8] = sums[0][2];
+        }
+        __syncthreads();  // two sets of parts in turn: one barrier a turn
+        if (threadIdx.x < 16)
+            for (int j = 0; j < groups && kk0 + j < top; ++j) {
+                const float (*p)[16] = part[turn][j];
+                const int r = threadIdx.x;
+                acc = fmaf(pair_weights[t * top + kk0 + j], ((p[0][r] + p[1][r]) + p[2][r]) + p[3][r], acc);
+            }
+    }
+    if (threadIdx.x < 16) out[t * n_rows + column] = acc;
+}
+
 // out_t = add_t (times add_weight_t) + the token's parts times their weights, in the order they were chosen
 template <typename T>
 __global__ void experts_join_kernel(const float* __restrict__ parts, const float* __restrict__ weights, const T* __restrict__ add,
@@ -913,6 +1114,15 @@ GK_EXPORT int gk_route_groups(const void* h, int dtype, const float* w_router, c
 
 namespace {
 
+int sm_count() {
+    static const int sms = [] {
+        int device = 0, n = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n = 148;
+        return n;
+    }();
+    return sms;
+}
+
 // How the pairs of a step are dealt to blocks: by pair where those are fewer than the experts (blocks of an expert's later pairs
 // leave at once), else by expert; an expert's rows are cut into chunks so that every SM finds some blocks' worth of work even if
 // half of the pairs share their experts.
@@ -920,7 +1130,9 @@ struct ExpertGrid {
     dim3 grid;
     int rows, by_expert, at_once;
     size_t smem;
+    long long blocks() const { return (long long)grid.x * grid.y; }
 };
+constexpr int UP_ROWS = 2 * UP_WARPS, DOWN_ROWS = 4 * UP_WARPS;  // the least of a chunk: every warp has its rows in flight
 
 ExpertGrid expert_grid(long long pairs, int n_experts, int n_rows, int row_length, int least_rows) {
     ExpertGrid g;
@@ -947,93 +1159,146 @@ constexpr size_t MMA_STATIC_SMEM = MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + M
 template <bool UP>
 void launch_mma(const void* source, const void* weights, const int* ids, void* act, float* parts, long long pairs, int n_tokens, int k, int n_rows, int divide,
                 int n_experts, cudaStream_t s) {
-    static const int sms = [] {
-        int device = 0, n = 0;
-        cudaGetDevice(&device);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
-        return n > 0 ? n : 148;
-    }();
     const int at_once = n_tokens > 8 && MMA_TOKENS * (size_t)mma_stride(k) <= 48 * 1024 ? MMA_TOKENS : 8;
     const size_t rows = (size_t)at_once * mma_stride(k), counts = (2 * (size_t)n_experts + MMA_LIST) * 4, smem = rows > counts ? rows : counts;
     // as many blocks as stay on the device at once: by their registers (the bound above) and by shared memory
     const long long blocks = std::max(1LL, std::min(UP ? 3LL : 4LL, (long long)(227 * 1024 / (smem + MMA_STATIC_SMEM + 1024))));
-    const long long most = std::min(pairs, (long long)MMA_LIST) * (n_rows / 16), places = blocks * sms;
+    const long long most = std::min(pairs, (long long)MMA_LIST) * (n_rows / 16), places = blocks * sm_count();
     if (smem > 16 * 1024) cudaFuncSetAttribute(experts_mma_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     gk_launch(experts_mma_kernel<UP>, dim3((unsigned)std::min(most, places), 1, (unsigned)((pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32), smem, s,
               (const __nv_bfloat16*)source, (const __nv_bfloat16*)weights, ids, (__nv_bfloat16*)act, parts, (int)pairs, k, n_rows, divide, n_experts, at_once);
 }
 
-int experts_up(const void* h, int dtype, const void* w_gate_up, int w_dtype, const int* ids, void* act, int n_tokens,
-                            int width, int ff, int top, int n_experts, cudaStream_t s) {
-    GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts_up: bad dtype");
-    GK_REQUIRE(width > 0 && ff > 0 && top > 0 && n_experts > 0, "experts_up: bad sizes");
-    GK_REQUIRE((size_t)width * sizeof(float) <= 200 * 1024, "experts_up: rows of %d are longer than the kernel stages", width);
-    const long long pairs = (long long)n_tokens * top;
-    GK_REQUIRE(pairs <= 65535LL * MMA_LIST, "experts_up: too many pairs");
-    if (dtype == GK_BF16 && w_dtype == GK_BF16 && mma_suits(width, ff, n_experts) && (((uintptr_t)h | (uintptr_t)w_gate_up) & 15) == 0) {
-        launch_mma<true>(h, w_gate_up, ids, act, nullptr, pairs, n_tokens, width, ff, top, n_experts, s);
-        GK_CHECK_LAUNCH("experts_up");
-        return GK_OK;
-    }
-    const ExpertGrid g = expert_grid(pairs, n_experts, ff, width, 2 * UP_WARPS);
-    GK_DISPATCH_DTYPE(dtype, T, {
-        GK_DISPATCH_DTYPE(w_dtype, TW, {
-            if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_up_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-            gk_launch(experts_up_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)h, (const TW*)w_gate_up, ids, (T*)act,
-                      (int)pairs, width, ff, top, g.rows, g.by_expert, g.at_once);
-        })
-    })
-    GK_CHECK_LAUNCH("experts_up");
-    return GK_OK;
+// Megabytes of weights that the pairs of a step fetch and that they would not if every expert came once (a token's experts are all
+// different, two tokens' are chosen independently).
+double repeated_megabytes(int n_tokens, int top, int n_experts, double expert_bytes) {
+    const double different = n_experts * (1.0 - std::pow(1.0 - std::min(1.0, (double)top / n_experts), (double)n_tokens));
+    return ((double)n_tokens * top - different) * expert_bytes * 1e-6;
 }
 
-// parts: 32-bit scratch [n_tokens * top, width]
-int experts_down(const void* act, int dtype, const void* w_down, int w_dtype, const int* ids, const float* weights,
-                              const void* add, const float* add_weight, float* parts, float* out, int n_tokens, int width, int ff, int top,
-                              int n_experts, cudaStream_t s) {
-    GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts_down: bad dtype");
-    GK_REQUIRE(width > 0 && ff > 0 && top > 0 && n_experts > 0 && (add != nullptr || add_weight == nullptr), "experts_down: bad sizes");
-    GK_REQUIRE((size_t)top * ff * sizeof(float) <= 200 * 1024, "experts_down: %d experts of %d are more than the kernel stages", top, ff);
-    const long long pairs = (long long)n_tokens * top;
-    GK_REQUIRE(pairs <= 65535LL * MMA_LIST, "experts_down: too many pairs");
-    if (dtype == GK_BF16 && w_dtype == GK_BF16 && mma_suits(ff, width, n_experts) && (((uintptr_t)act | (uintptr_t)w_down) & 15) == 0) {
-        launch_mma<false>(act, w_down, ids, nullptr, parts, pairs, n_tokens, ff, width, 1, n_experts, s);
-    } else {
-        const ExpertGrid g = expert_grid(pairs, n_experts, width, ff, 4 * UP_WARPS);
-        GK_DISPATCH_DTYPE(dtype, T, {
-            GK_DISPATCH_DTYPE(w_dtype, TW, {
-                if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_down_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-                gk_launch(experts_down_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)act, (const TW*)w_down, ids, parts,
-                          (int)pairs, width, ff, g.rows, g.by_expert, g.at_once);
-            })
-        })
+struct ExpertStep {
+    const void *h, *w_gate_up, *w_down;
+    int dtype, w_dtype;
+    const int* ids;
+    const float* weights;
+    const void* add;
+    const float* add_weight;
+    float* parts;  // 32-bit scratch [n_tokens * top, width]
+    void* act;     // [n_tokens * top, ff] in the run's type
+    float* out;
+    int n_tokens, width, ff, top, n_experts;
+};
+
+template <typename T>
+void launch_join(const ExpertStep& p, cudaStream_t s) {
+    gk_launch(experts_join_kernel<T>, dim3(p.n_tokens, (p.width + 255) / 256), dim3(256), 0, s, (const float*)p.parts, p.weights, (const T*)p.add,
+              p.add_weight, p.out, p.width, p.top);
+}
+
+// up: inner values of all pairs; down: their products and the sums.  Each on the tensor cores where its sizes are whole tiles, and
+// each either a pair by itself or an expert's pairs together.
+void up_mma(const ExpertStep& p, bool few, cudaStream_t s) {
+    const long long pairs = (long long)p.n_tokens * p.top;
+    if (few)
+        gk_launch(pair_up_mma_kernel, dim3((unsigned)pairs, p.ff / 16), dim3(MMA_WARPS * 32), 0, s, (const __nv_bfloat16*)p.h, (const __nv_bfloat16*)p.w_gate_up,
+                  p.ids, (__nv_bfloat16*)p.act, p.width, p.ff, p.top);
+    else
+        launch_mma<true>(p.h, p.w_gate_up, p.ids, p.act, nullptr, pairs, p.n_tokens, p.width, p.ff, p.top, p.n_experts, s);
+}
+
+void down_mma(const ExpertStep& p, bool few, cudaStream_t s) {
+    if (few) {
+        const int turns = (p.top + TOKEN_PAIRS - 1) / TOKEN_PAIRS, groups = (p.top + turns - 1) / turns;
+        gk_launch(token_down_mma_kernel, dim3(p.n_tokens, p.width / 16), dim3(groups * MMA_WARPS * 32), 0, s, (const __nv_bfloat16*)p.act,
+                  (const __nv_bfloat16*)p.w_down, p.ids, p.weights, (const __nv_bfloat16*)p.add, p.add_weight, p.out, p.ff, p.width, p.top);
+        return;
     }
-    GK_CHECK_LAUNCH("experts_down");
-    GK_DISPATCH_DTYPE(dtype, T, {
-        gk_launch(experts_join_kernel<T>, dim3(n_tokens, (width + 255) / 256), dim3(256), 0, s, (const float*)parts, weights, (const T*)add,
-                  add_weight, out, width, top);
-    })
-    GK_CHECK_LAUNCH("experts_join");
+    launch_mma<false>(p.act, p.w_down, p.ids, nullptr, p.parts, (long long)p.n_tokens * p.top, p.n_tokens, p.ff, p.width, 1, p.n_experts, s);
+    launch_join<__nv_bfloat16>(p, s);
+}
+
+template <typename T, typename TW>
+void up_fp32(const ExpertStep& p, bool few, cudaStream_t s) {
+    const long long pairs = (long long)p.n_tokens * p.top;
+    if (few) {  // cut the experts' rows over more blocks, so that a single token still finds every SM a share
+        int chunks = 1;
+        while (pairs * chunks < 592 && p.ff / (chunks * 2) >= UP_WARPS) chunks *= 2;
+        const int rows = (p.ff + chunks - 1) / chunks;
+        const size_t smem = (size_t)p.width * sizeof(float);
+        if (smem > 48 * 1024) cudaFuncSetAttribute(pair_up_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        gk_launch(pair_up_kernel<T, TW>, dim3((unsigned)pairs, (p.ff + rows - 1) / rows), dim3(UP_WARPS * 32), smem, s, (const T*)p.h, (const TW*)p.w_gate_up, p.ids,
+                  (T*)p.act, p.width, p.ff, p.top, rows);
+        return;
+    }
+    const ExpertGrid g = expert_grid(pairs, p.n_experts, p.ff, p.width, UP_ROWS);
+    if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_up_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    gk_launch(experts_up_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)p.h, (const TW*)p.w_gate_up, p.ids, (T*)p.act, (int)pairs, p.width,
+              p.ff, p.top, g.rows, g.by_expert, g.at_once);
+}
+
+template <typename T, typename TW>
+void down_fp32(const ExpertStep& p, bool few, cudaStream_t s) {
+    if (few) {
+        int chunks = 1;
+        while ((long long)p.n_tokens * chunks < 592 && p.width / (chunks * 2) >= UP_WARPS) chunks *= 2;
+        const int rows = (p.width + chunks - 1) / chunks;
+        const size_t smem = (size_t)p.top * p.ff * sizeof(float);
+        if (smem > 48 * 1024) cudaFuncSetAttribute(token_down_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        gk_launch(token_down_kernel<T, TW>, dim3(p.n_tokens, (p.width + rows - 1) / rows), dim3(UP_WARPS * 32), smem, s, (const T*)p.act, (const TW*)p.w_down, p.ids,
+                  p.weights, (const T*)p.add, p.add_weight, p.out, p.width, p.ff, p.top, rows);
+        return;
+    }
+    const long long pairs = (long long)p.n_tokens * p.top;
+    const ExpertGrid g = expert_grid(pairs, p.n_experts, p.width, p.ff, DOWN_ROWS);
+    if (g.smem > 40 * 1024) cudaFuncSetAttribute(experts_down_kernel<T, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    gk_launch(experts_down_kernel<T, TW>, g.grid, dim3(UP_WARPS * 32), g.smem, s, (const T*)p.act, (const TW*)p.w_down, p.ids, p.parts, (int)pairs, p.width,
+              p.ff, g.rows, g.by_expert, g.at_once);
+    launch_join<T>(p, s);
+}
+
+int experts(const ExpertStep& p, cudaStream_t s) {
+    const bool bf16 = p.dtype == GK_BF16 && p.w_dtype == GK_BF16;
+    const bool mma_up = bf16 && mma_suits(p.width, p.ff, p.n_experts) && (((uintptr_t)p.h | (uintptr_t)p.w_gate_up) & 15) == 0;
+    const bool mma_down = bf16 && mma_suits(p.ff, p.width, p.n_experts) && (((uintptr_t)p.act | (uintptr_t)p.w_down) & 15) == 0;
+    const long long pairs = (long long)p.n_tokens * p.top;
+    const double third = (double)p.ff * p.width * (p.w_dtype == GK_F32 ? 4 : 2), repeated = repeated_megabytes(p.n_tokens, p.top, p.n_experts, 3 * third);
+    // A pair by itself where hardly any expert has two, or where the pairs' rows are little in all.  The lists cost some 4 us, as
+    // much as fetching 8 MB again.  Measured (us, by itself / lists; tensor cores): 3 tokens, 5 of 33 experts of 1,024 x 768 (10 MB
+    // again): 16.7 / 18.9, 4 tokens (19 MB): 20.4 / 19.6; 3 tokens, 6 of 64 of 2,048 x 1,024 (21 MB): 75.7 / 71.9.  On the FP32 pipes a
+    // list serves four tokens at a time and wins later, and not where its blocks are few: 4 tokens, 6 of 64 of 2,048 x 1,024 in 32
+    // bits (80 MB): 126.7 / 116; 3 tokens (40 MB): 88.6 / 100; 1,024 tokens, 2 of 8 of 256 x 128: 106 / 217.
+    const bool few_mma = (repeated <= 8 || (double)pairs * 3e-6 * third <= 32) && p.width / 16 <= 65535 && p.ff / 16 <= 65535;
+    const bool few_up = repeated <= 64 || expert_grid(pairs, p.n_experts, p.ff, p.width, UP_ROWS).blocks() < 2LL * sm_count();
+    const bool few_down = repeated <= 64 || expert_grid(pairs, p.n_experts, p.width, p.ff, DOWN_ROWS).blocks() < 2LL * sm_count();
+    if (mma_up) up_mma(p, few_mma, s);
+    else GK_DISPATCH_DTYPE(p.dtype, T, { GK_DISPATCH_DTYPE(p.w_dtype, TW, { up_fp32<T, TW>(p, few_up, s); }) })
+    if (mma_down) down_mma(p, few_mma, s);
+    else GK_DISPATCH_DTYPE(p.dtype, T, { GK_DISPATCH_DTYPE(p.w_dtype, TW, { down_fp32<T, TW>(p, few_down, s); }) })
+    GK_CHECK_LAUNCH("experts");
     return GK_OK;
 }
 
 }  // namespace
 
-// The whole routed feed-forward behind the router.  `work`: 32-bit scratch of `at_once` rows of top * (width + ff) numbers; more
+// The whole routed feed-forward behind the router.  `work`: scratch of `at_once` times top * (4 width + ff * the type's size) bytes; more
 // tokens than that go in several turns.
 GK_EXPORT int gk_experts(const void* h, int dtype, const void* w_gate_up, const void* w_down, int w_dtype, const int* ids, const float* weights,
                          const void* add, const float* add_weight, float* work, float* out, int n_tokens, int at_once, int width, int ff, int top,
                          int n_experts, void* stream) {
-    GK_REQUIRE(GK_VALID_DTYPE(dtype) && at_once > 0 && width > 0 && ff > 0 && top > 0, "experts: bad sizes");
+    GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts: bad dtype");
+    GK_REQUIRE(at_once > 0 && width > 0 && ff > 0 && top > 0 && n_experts > 0 && (add != nullptr || add_weight == nullptr), "experts: bad sizes");
+    if (n_tokens == 0) return GK_OK;
+    // a token's inner values stand in shared memory in the down product of few pairs
+    GK_REQUIRE((size_t)width * sizeof(float) <= 200 * 1024, "experts: rows of %d are longer than the kernels stage", width);
+    GK_REQUIRE((size_t)top * ff * sizeof(float) <= 200 * 1024, "experts: %d experts of %d are more than the kernels stage", top, ff);
+    GK_REQUIRE((long long)std::min(at_once, n_tokens) * top <= 65535LL * MMA_LIST, "experts: too many pairs at once");
     const size_t size = dtype == GK_F32 ? 4 : 2;
     for (int at = 0; at < n_tokens; at += at_once) {
-        const int n = std::min(at_once, n_tokens - at);
         const size_t row = (size_t)at * width;
-        void* act = work + (size_t)at_once * top * width;
-        int status = experts_up((const char*)h + row * size, dtype, w_gate_up, w_dtype, ids + (size_t)at * top, act, n, width, ff, top, n_experts, (cudaStream_t)stream);
-        if (status == GK_OK)
-            status = experts_down(act, dtype, w_down, w_dtype, ids + (size_t)at * top, weights + (size_t)at * top, add ? (const char*)add + row * size : nullptr,
-                                  add_weight ? add_weight + at : nullptr, work, out + row, n, width, ff, top, n_experts, (cudaStream_t)stream);
+        const ExpertStep p{(const char*)h + row * size, w_gate_up, w_down, dtype, w_dtype, ids + (size_t)at * top, weights + (size_t)at * top,
+                           add ? (const char*)add + row * size : nullptr, add_weight ? add_weight + at : nullptr, work, work + (size_t)at_once * top * width,
+                           out + row, std::min(at_once, n_tokens - at), width, ff, top, n_experts};
+        const int status = experts(p, (cudaStream_t)stream);
         if (status != GK_OK) return status;
     }
     return GK_OK;

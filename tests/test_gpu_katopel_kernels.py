@@ -627,3 +627,69 @@ def test_experts_without_a_choice_are_refused():
     h, gate_up, down = torch.randn(2, 16).cuda(), torch.randn(3, 2, 8, 16).cuda(), torch.randn(3, 16, 8).cuda()
     with pytest.raises(KernelError):
         F().experts_pairwise(h, gate_up, down, torch.empty(2, 0, dtype=torch.int32, device="cuda"), torch.empty(2, 0, device="cuda"))
+
+
+def _random_experts(tokens, width, ff, experts, top, dtype, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed + tokens * width + ff)
+    draw = lambda *shape: torch.randn(shape, generator=gen, device="cuda")
+    ids = torch.rand(tokens, experts, generator=gen, device="cuda").argsort(dim=1)[:, :top].to(torch.int32).contiguous()
+    return ((draw(tokens, width)).to(dtype), (draw(experts, 2, ff, width) * width**-0.5).to(dtype), (draw(experts, width, ff) * ff**-0.5).to(dtype), ids,
+            torch.rand(tokens, top, generator=gen, device="cuda"), draw(tokens, width).to(dtype), torch.rand(tokens, generator=gen, device="cuda"))
+
+
+# steps of few pairs (a pair, a token a block) and of many (an expert's pairs together): whole tiles and sizes beside them, one and
+# several turns of a token's pairs, lists of more than 512 and 1,024 pairs, sixteen tokens at once and eight
+@pytest.mark.parametrize("tokens,width,ff,experts,top", [(300, 1024, 768, 32, 4), (64, 2048, 512, 16, 4), (40, 1030, 770, 32, 4), (24, 2048, 528, 16, 9), (24, 2064, 512, 16, 3)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_of_a_few_tokens_have_the_sums_of_a_step_of_many(tokens, width, ff, experts, top, dtype):
+    h, gate_up, down, ids, weights, add, share = _random_experts(tokens, width, ff, experts, top, dtype)
+    got = F().experts_pairwise(h, gate_up, down, ids, weights, add, share)
+    for t in (0, tokens // 2, tokens - 1):
+        want = add[t].double() * share[t].double()
+        for e, w in zip(ids[t].tolist(), weights[t].double()):
+            z = gate_up[e].double() @ h[t].double()
+            want += w * (down[e].double() @ (torch.nn.functional.silu(z[0]) * z[1]).to(dtype).double())
+        # the inner values round to bfloat16 on either side of a tie: 2^-9 of them, through a sum of ff products
+        assert (got[t].double() - want).abs().max() < (2e-5 if dtype == torch.float32 else 2.0**-9 * 6 * top)
+        for n in (1, 2):
+            rows = slice(t, t + n) if t + n <= tokens else slice(t - n + 1, t + 1)
+            few = F().experts_pairwise(h[rows], gate_up, down, ids[rows].contiguous(), weights[rows].contiguous(), add[rows], share[rows].contiguous())
+            assert torch.equal(few, got[rows])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_experts_in_several_turns(dtype, monkeypatch):
+    """More pairs than go at a time: the same numbers, with another branch's output and its weights, at a token count that is no
+    multiple of a turn's."""
+    inputs = _random_experts(23, 96, 64, 5, 2, dtype)
+    whole = F().experts_pairwise(*inputs)
+    monkeypatch.setattr(F(), "EXPERT_PAIRS_AT_ONCE", 14)  # seven tokens
+    assert torch.equal(F().experts_pairwise(*inputs), whole)
+    assert torch.equal(F().experts_pairwise(*inputs[:5]), F().experts_pairwise(*inputs[:5]))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens,width,ff,experts,top", [(64, 70, 30, 6, 2), (128, 256, 128, 8, 2)])
+def test_experts_of_small_layers_are_not_slowed_by_their_lists(tokens, width, ff, experts, top, dtype):
+    """A step of small experts stays within a few times the step of one token: measured 1.1 to 1.2 (70 x 30) and 3.4 to 4.1 times (256 x 128);
+    an expert's pairs together: 5.4 to 6.6 and 1.8 to 8.4, of a step of one token that takes twice as long."""
+    inputs = _random_experts(tokens, width, ff, experts, top, dtype)[:5]
+    one = [t[:1].contiguous() if i in (0, 3, 4) else t for i, t in enumerate(inputs)]
+
+    def device_time(args):
+        F().experts_pairwise(*args)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            for _ in range(10):
+                F().experts_pairwise(*args)
+        times = []
+        for _ in range(6):
+            begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            begin.record()
+            graph.replay()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times[1:])
+
+    assert device_time(inputs) < 5 * device_time(one)
