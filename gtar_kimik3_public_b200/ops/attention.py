@@ -66,7 +66,7 @@ def paged_attention(q: torch.Tensor, kv: F.PagedKV, ctx, scale: float, window: i
         return F.attention_decode(q, kv, ctx.kv_len, ctx.slots, scale, window, splits, sink=sink)
     if fast:
         return F.attention_prefill(q, kv, ctx.cu_q, ctx.kv_len, ctx.slots, ctx.max_q_len, scale, window, sink=sink)
-    return F.attention_exact(q, kv, ctx.tok_pos, ctx.tok_seq, ctx.slots, scale, window, sink=sink)
+    return F.attention_exact(q, kv, ctx.tok_pos, ctx.tok_seq, ctx.slots, scale, window, sink=sink, longest_run=ctx.max_q_len)
 
 
 # "0" sends bfloat16 latent attention through the exact kernel too (for measurements and for telling the kernels apart)

@@ -306,9 +306,11 @@ def attention_exact(
     window: int = 0,
     out: torch.Tensor | None = None,
     sink: bool = False,
+    longest_run: int = 0,
 ) -> torch.Tensor:
-    """Causal grouped-query attention of ``q [n_tokens, n_q, d]`` over the pages (exact kernel).  ``sink``: the
-    softmax's denominator has one more term, a key of score 0 without a value."""
+    """Causal grouped-query attention of ``q [n_tokens, n_q, d]`` over the pages (exact kernels).  ``sink``: the
+    softmax's denominator has one more term, a key of score 0 without a value.  ``longest_run``: the most tokens that one
+    sequence brings, where the caller knows; it bears on speed alone."""
     require_device(q.device)
     _check(q, "q", dims=3)
     n, n_q, d = q.shape
@@ -324,7 +326,7 @@ def attention_exact(
     call(
         "gk_attention_exact", ptr(q), ptr(kv.k), ptr(kv.v), ptr(out), dtype_code(q.dtype), ptr(tok_pos), ptr(tok_seq),
         ptr(slots), ptr(kv.block_table), n, n_q, n_kv, d, kv.max_pages, kv.page_size, float(scale), int(window),
-        int(sink), slots.shape[0], stream_ptr(),
+        int(sink), slots.shape[0], int(longest_run), stream_ptr(),
     )
     return out
 

@@ -840,8 +840,8 @@ def test_gemm_f32_chains_are_the_same_in_every_kernel(k, a_dtype):
 @pytest.mark.parametrize("n_q,n_kv,d,window,sink", [(2, 2, 8, 0, False), (6, 2, 40, 70, True), (10, 2, 72, 0, True), (9, 1, 64, 33, False),
                                                     (8, 1, 128, 0, False), (16, 1, 32, 0, False), (16, 1, 128, 1100, False)])
 def test_attention_exact_is_the_same_in_every_kernel(dtype, n_q, n_kv, d, window, sink):
-    """A step of many tokens (the tile kernel), the same tokens one a step and few a step (the cluster), bit for bit, with
-    values of later positions poisoned for the single steps; spans of 1,024 keys, blocks of 32 and pages of 64 are crossed."""
+    """A step of many tokens (tiles), the same tokens one a step and few a step (clusters), bit for bit; spans of 1,024 keys, blocks of
+    32 and pages of 64 are crossed, and what lies behind a sequence's last token is poisoned."""
     lens, past = [1300, 37, 700], [0, 0, 650]
     kv, slots, table = scrambled_pages(3, 1300, n_kv, d, dtype, seed=12)
     pos, seq = [], []
@@ -895,3 +895,77 @@ def test_sample_top_k_of_any_rows(rows, vocab, top_k, values):
     got = F().sample(logits.to(DEV), 0.9, top_k, 77, requests.to(DEV), steps.to(DEV)).cpu().tolist()
     for i in range(min(rows, 4)):
         assert got[i] == plain_sampling.sample(logits[i].numpy(), 0.9, top_k, 77, int(requests[i]), int(steps[i])), f"row {i}"
+
+
+# runs of a step, (tokens, past): long ones that fill tiles, short ones and single tokens between them, more than 1,024 tokens in all
+MIXED_RUNS = [(1, 90), (600, 0), (3, 40), (1, 1100), (20, 5), (2, 63), (1, 0), (33, 30), (7, 64), (1, 31), (1, 32), (420, 100), (5, 200), (5, 0)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,d,window,sink", [(4, 4, 96, 0, False), (8, 4, 64, 70, False), (18, 6, 32, 0, True), (16, 1, 128, 0, False), (10, 2, 40, 300, True)])
+def test_attention_exact_of_mixed_steps_is_that_of_single_tokens(dtype, n_q, n_kv, d, window, sink):
+    """Tiles and single warps side by side in one step, tokens in packed order and in any order, against every token by itself with
+    whatever stands behind it poisoned, bit for bit."""
+    kv, slots, table = scrambled_pages(len(MIXED_RUNS), 1102, n_kv, d, dtype, seed=21)
+    pos, seq = [], []
+    for i, (n, past) in enumerate(MIXED_RUNS):
+        fill_pages(kv, table, int(slots[i]), rand(past + n, n_kv, d, seed=160 + i).to(dtype), rand(past + n, n_kv, d, seed=190 + i).to(dtype))
+        pos += list(range(past, past + n))
+        seq += [i] * n
+    q = rand(len(pos), n_q, d, seed=220).to(dtype).to(DEV)
+    tok_pos, tok_seq = torch.tensor(pos, dtype=torch.int32).to(DEV), torch.tensor(seq, dtype=torch.int32).to(DEV)
+    run = lambda at, **more: F().attention_exact(q[at].contiguous(), kv, tok_pos[at].contiguous(), tok_seq[at].contiguous(), slots.to(DEV), d**-0.5, window, sink=sink, **more)
+    everything = torch.arange(len(pos), device=DEV)
+    whole = run(everything)
+    assert torch.isfinite(whole).all()
+    assert torch.equal(run(everything, longest_run=600), whole)
+    assert torch.equal(run(everything, longest_run=1), whole)  # not true, and bears on speed alone: warps for all
+    order = torch.randperm(len(pos), generator=torch.Generator().manual_seed(4)).to(DEV)
+    assert torch.equal(run(order), whole[order])
+    for i, (n, past) in enumerate(MIXED_RUNS):
+        first = seq.index(i)
+        for t in sorted({n - 1, n // 2, 0}, reverse=True):  # the last first: what is poisoned stays so
+            for at in range(past + t + 1, past + n):
+                page = int(table[slots[i], at // 64])
+                kv.k[page, :, at % 64] = float("nan")
+                kv.v[page, :, at % 64] = float("nan")
+            one = torch.tensor([first + t]).to(DEV)
+            assert torch.equal(run(one), whole[one]), f"token {t} of run {i}"
+
+
+def device_time(step, repeats=5):
+    """Microseconds of the fastest of some replays of `step`, captured ten times in a row."""
+    step()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        for _ in range(10):
+            step()
+    times = []
+    for _ in range(repeats + 1):
+        begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        begin.record()
+        graph.replay()
+        end.record()
+        torch.cuda.synchronize()
+        times.append(begin.elapsed_time(end) * 100)
+    return min(times[1:])
+
+
+@pytest.mark.parametrize("runs,parts", [
+    ([(1, 1000)] * 64 + [(512, 0)], ([(1, 1000)] * 64, [(512, 0)])),  # measured 2.1 times the larger part; a tile that walks its 32 runs: 30
+    ([(3, 1000)] * 64, ([(1, 1000)] * 64,) * 3),  # measured 0.5 of the parts' sum; tiles that walk ten runs each: 7
+    ([(1, 10)] * 64, ([(1, 10)],) * 4),  # measured 0.4; a cluster a token and kv head: 3.7
+])
+def test_attention_exact_of_many_sequences_does_not_walk_them_one_after_another(runs, parts):
+    """A step takes at most twice as long as the steps that it could be cut into, one after another."""
+    n_q, n_kv, d = 16, 8, 128
+
+    def step(some):
+        kv, slots, table = scrambled_pages(len(some), 1064, n_kv, d, torch.float32, seed=5)
+        kv.k.normal_(), kv.v.normal_()
+        pos = torch.tensor([p + t for n, p in some for t in range(n)], dtype=torch.int32).to(DEV)
+        seq = torch.tensor([i for i, (n, _) in enumerate(some) for _ in range(n)], dtype=torch.int32).to(DEV)
+        q, at = torch.randn(len(pos), n_q, d, device=DEV), slots.to(DEV)
+        return device_time(lambda: F().attention_exact(q, kv, pos, seq, at, d**-0.5))
+
+    assert step(runs) < 2 * sum(step(part) for part in parts)

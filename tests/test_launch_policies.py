@@ -138,3 +138,27 @@ def test_latent_attention_splits():
                 splits = latent_splits(n_seqs, heads, kv_len, window, sms)
                 span = min(kv_len, window) if window else kv_len
                 assert 1 <= splits <= min(LATENT_TILED_MAX_SPLITS, span // 64 + 1)
+
+
+SINGLE, TILES, WARPS = 1, 2, 4
+
+
+def test_exact_attention_routes_at_measured_points():
+    """Few tokens go to clusters, many single tokens and short runs to warps, and tiles never stand alone where a step has several
+    sequences (a tile leaves the tokens of short runs to the warps)."""
+    from gtar_kimik3_public_b200.ops.library import library
+
+    route = lambda tokens, seqs, longest=0, n_q=16, n_kv=8, d=128, dtype=0: library().gk_attention_exact_route(tokens, seqs, longest, n_q, n_kv, d, dtype, 148)
+    assert route(1, 1) == route(3, 3) == route(16, 16) == SINGLE
+    assert route(32, 32) == route(64, 64) == route(512, 512) == WARPS
+    assert route(64 + 512, 65) == route(805, 3) == TILES | WARPS and route(64 + 512, 65, 512) == TILES | WARPS
+    assert route(2048, 1) == TILES  # one sequence fills its tiles
+    assert route(640, 16, 40) == WARPS and route(640, 16) == TILES | WARPS  # the longest run would not fill two tiles
+    for dtype in (0, 1):
+        for n_q, n_kv, d in ((16, 8, 128), (16, 1, 128), (4, 4, 96), (6, 2, 32), (9, 1, 64), (2, 2, 8)):
+            for seqs in (1, 2, 7, 64, 500):
+                for longest in (1, 2, 8, 40, 700):
+                    tokens = seqs + longest - 1
+                    got = route(tokens, seqs, longest, n_q, n_kv, d, dtype)
+                    assert got in (SINGLE, WARPS, TILES, TILES | WARPS), (n_q, n_kv, d, seqs, longest, got)
+                    assert got != TILES or seqs == 1, (n_q, n_kv, d, seqs, longest)
