@@ -10,6 +10,8 @@
 //
 // Ties go to the lowest index in both kernels.
 
+#include <cstddef>
+
 #include "common.cuh"
 
 namespace {
@@ -36,6 +38,8 @@ __device__ __forceinline__ unsigned int float_key(float f) {
     unsigned int u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
+
+__device__ __forceinline__ float key_float(unsigned int key) { return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key); }
 
 struct Best {
     float value;
@@ -106,6 +110,53 @@ __device__ __forceinline__ void scan_slice(const float* __restrict__ row, int be
     for (int i = vec_begin + 4 * n_vec + threadIdx.x; i < end; i += blockDim.x) visit(row[i], i);
 }
 
+// The same for the elements whose key reaches `least`, of which there are few: what is done with one stands in the code once and
+// fetches it again, instead of sixteen times behind the loads.
+template <typename Visit>
+__device__ __forceinline__ void scan_reaching(const float* __restrict__ row, int begin, int end, unsigned int least, Visit visit) {
+    const int lead = min((int)((16 - ((uintptr_t)(row + begin) & 15)) & 15) / 4, max(end - begin, 0));
+    const int vec_begin = begin + lead, n_vec = max(end - vec_begin, 0) / 4, rest = vec_begin + 4 * n_vec;
+    const float4* vec = reinterpret_cast<const float4*>(row + vec_begin);
+    const float least_value = key_float(least);
+    const auto maybe = [&](float x) { return !(x < least_value); };  // true for all that reach it, for a zero of the other sign and for NaN
+    constexpr int IN_FLIGHT = 4;
+    // the last turn of all threads is for the elements beside the whole pieces: at most three in front and three behind
+    for (int v0 = threadIdx.x;; v0 += blockDim.x * IN_FLIGHT) {
+        unsigned int hits = 0;
+        int first = vec_begin + 4 * v0, step = 4 * (int)blockDim.x;
+        const bool last = v0 >= n_vec;
+        if (!last) {
+            float4 got[IN_FLIGHT];
+#pragma unroll
+            for (int u = 0; u < IN_FLIGHT; ++u) {
+                const int v = v0 + u * (int)blockDim.x;
+                if (v < n_vec) got[u] = vec[v];
+            }
+#pragma unroll
+            for (int u = 0; u < IN_FLIGHT; ++u) {
+                if (maybe(got[u].x)) hits |= 1u << (4 * u);
+                if (maybe(got[u].y)) hits |= 2u << (4 * u);
+                if (maybe(got[u].z)) hits |= 4u << (4 * u);
+                if (maybe(got[u].w)) hits |= 8u << (4 * u);
+            }
+            if (v0 + (IN_FLIGHT - 1) * (int)blockDim.x >= n_vec)  // what was not loaded
+#pragma unroll
+                for (int u = 1; u < IN_FLIGHT; ++u)
+                    if (v0 + u * (int)blockDim.x >= n_vec) hits &= ~(15u << (4 * u));
+        } else {
+            if ((int)threadIdx.x < lead) hits |= 1u;
+            if ((int)threadIdx.x < end - rest) hits |= 1u << 4;
+            first = begin + (int)threadIdx.x, step = rest - begin;
+        }
+        for (; hits != 0; hits &= hits - 1) {
+            const int bit = __ffs(hits) - 1, i = first + (bit >> 2) * step + (bit & 3);
+            const float x = row[i];
+            if (float_key(x) >= least) visit(x, i);
+        }
+        if (last) break;
+    }
+}
+
 // Grid (parts, rows): block (p, r) scans its slice of row r and leaves its best (value, index) in
 // `partial[r * parts + p]`; with one part it writes the answer itself.
 __global__ void argmax_kernel(const float* __restrict__ logits, long long row_stride, int vocab,
@@ -148,15 +199,18 @@ __global__ void best_merge_kernel(const Best* __restrict__ partial, int parts, i
 
 // ---- top-k: the choice among the logits that reach the row's k-th largest, in one kernel.
 //
-// A cluster of up to SELECT_BLOCKS blocks shares a row.  Short way (top_k up to half the groups): the lanes of a warp, or
-// eight of them where k is larger, form a group; of all groups' largest logits the k-th largest is a bound that at least k
-// logits reach, and hardly more do (of random rows about 63 with 128 groups and k = 50).  A second scan, which finds the row in L2, hands those on to the cluster's first block, which
-// finds the k-th largest among them by counting and draws.  So a row is scanned twice and noise is formed for the candidates
-// alone.  Long way, where more logits reach the bound than the list holds (a row of equal numbers) or k is larger: a radix
-// select over the order-preserving keys, eight bits a scan, with the blocks' histograms added up through distributed shared
-// memory, and a last scan that draws.
-// Bound by the two scans and the cluster's barriers between them.  Measured (64 rows of 151,936, k = 50): see gk_sample.
-constexpr int SELECT_BLOCKS = 8, SELECT_THREADS = 512, MAX_GROUPS = SELECT_THREADS / 8, CANDIDATES = 2048;
+// A cluster of up to SELECT_BLOCKS blocks shares a row (top_k up to half of MAX_KEYS).  The lanes of a warp, or a
+// half, a quarter ... of them where k is larger, form a group, at least two groups for each of the k; of all groups' largest logits
+// the k-th largest is a bound that at least k logits reach, and hardly more do (of random rows about 63 with 128 groups and k =
+// 50).  A second scan, which finds the row in L2, hands those on to the cluster's first block, which finds the k-th largest among
+// them and draws.  So a row is scanned twice and noise is formed for the candidates alone.  Where more logits reach the bound than
+// the list holds, they stop asking for a place; if fewer than k of them are above it (rows of equal numbers, rows masked down to
+// fewer than k), the bound is the k-th largest and a third scan draws.  Else (rows in order), as for larger k: a radix select over the
+// order-preserving keys, eight bits a scan, with the blocks' histograms added up through distributed shared memory, and a last scan
+// that draws.
+// Bound by the scans and the cluster's barriers between them.  A block has 40 registers a thread (three blocks an SM, a few of
+// them spilled): with four blocks an SM and 32 registers 64 rows of 151,936 took 22.0 us instead of 17.4.
+constexpr int SELECT_BLOCKS = 8, SELECT_THREADS = 512, MAX_KEYS = 512, CANDIDATES = 2048;
 
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -177,10 +231,16 @@ struct Draw {
     float temperature;
     unsigned long long seed, request, step;
     __device__ __forceinline__ Best of(float x, int i) const {
+        if (x == -INFINITY) return Best{x, i};  // whatever the noise
         const float u = uniform_open(seed, request, step, (unsigned long long)i);
         const float g = -logf(-logf(u));
         return Best{x / temperature + g, i};
     }
+};
+
+struct CandidateList {
+    int2 entries[CANDIDATES];  // a logit's bits and its index
+    unsigned int count;
 };
 
 struct SelectShared {
@@ -188,8 +248,9 @@ struct SelectShared {
 };
 
 // The key of the row's k-th largest logit, by the long way.  Two histograms in turn, so that a block may clear the next one
-// while others still read this one.  Lanes that meet in a bin add to it once.
-__device__ __noinline__ unsigned int radix_threshold(const float* __restrict__ row, int begin, int end, int top_k, int n_ranks, SelectShared& sh) {
+// while others still read this one.  Lanes that meet in a bin add to it once.  `least`: a key that is not above the k-th largest.
+__device__ __noinline__ unsigned int radix_threshold(const float* __restrict__ row, int begin, int end, int top_k, int n_ranks, unsigned int least,
+                                                     SelectShared& sh) {
     const int lane = threadIdx.x & 31;
     unsigned int prefix = 0, mask = 0;
     if (threadIdx.x == 0) sh.sel_remaining = (unsigned)top_k;
@@ -200,7 +261,7 @@ __device__ __noinline__ unsigned int radix_threshold(const float* __restrict__ r
         unsigned int* mine = sh.hist[pass & 1];
         scan_slice(row, begin, end, [&](float x, int) {
             const unsigned int key = float_key(x);
-            if ((key & mask) == prefix) {
+            if ((key & mask) == prefix && key >= least) {
                 const unsigned int bin = (key >> shift) & 255u;
                 const unsigned int same = __match_any_sync(__activemask(), bin);
                 if (lane == __ffs(same) - 1) atomicAdd(&mine[bin], (unsigned)__popc(same));
@@ -251,27 +312,91 @@ __device__ __noinline__ unsigned int radix_threshold(const float* __restrict__ r
     return prefix;
 }
 
-// keys[0 .. n - 1] in shared memory: `*found` becomes the k-th largest (n >= k).  A thread a key counts those in front of it
-// (larger, or equal with a lower index); whoever stands on the k-th place says so.
-__device__ __forceinline__ void kth_largest(const unsigned int* keys, int n, int k, unsigned int* found) {
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const unsigned int mine = keys[i];
-        int front = 0;
+// The least of keys[first .. first + count - 1] (up to MAX_KEYS of them) in front of which fewer than k of keys[0 .. n - 1] stand
+// (larger ones): over all n keys that is the k-th largest.  As many threads a key as there are take a run of the n each, a warp
+// the same run, four keys a load.  `in_front` holds zeros and `*least` all ones before and `in_front` zeros afterwards; a barrier
+// stands between that and the call.  (One thread for each of 512 keys, which goes through all of them, took 29 of 43 us for 64 rows of
+// 32,000 with k = 65.)
+__device__ __noinline__ unsigned int least_of_first(const unsigned int* keys, int n, int k, int first, int count, unsigned int* in_front, unsigned int* least) {
+    if (n <= 128) {  // first = 0, count = n: a thread a key, and whoever stands on the k-th place says so
+        if ((int)threadIdx.x < n) {
+            const unsigned int mine = keys[threadIdx.x];
+            int front = 0;
 #pragma unroll 8
-        for (int j = 0; j < n; ++j) front += keys[j] > mine || (keys[j] == mine && j < i);
-        if (front == k - 1) *found = mine;
+            for (int j = 0; j < n; ++j) front += keys[j] > mine || (keys[j] == mine && j < (int)threadIdx.x);
+            if (front == k - 1) *least = mine;
+        }
+        __syncthreads();
+        return *least;
     }
+    const int padded = (count + 31) & ~31, runs = SELECT_THREADS / padded, run = (int)threadIdx.x / padded, at = (int)threadIdx.x - run * padded;
+    const int length = ((n + runs - 1) / runs + 3) & ~3, end = min(n, (run + 1) * length);
+    if (run < runs) {
+        const unsigned int mine = at < count ? keys[first + at] : 0u;
+        unsigned int larger = 0;
+        int j = run * length;
+#pragma unroll 4
+        for (; j + 4 <= end; j += 4) {
+            const uint4 four = *reinterpret_cast<const uint4*>(keys + j);
+            larger += (four.x > mine) + (four.y > mine) + (four.z > mine) + (four.w > mine);
+        }
+        for (; j < end; ++j) larger += keys[j] > mine;
+        if (at < count) atomicAdd(&in_front[at], larger);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < padded) {
+        const unsigned int mine = (int)threadIdx.x < count && in_front[threadIdx.x] < (unsigned int)k ? keys[first + threadIdx.x] : 0xffffffffu;
+        const unsigned int of_warp = __reduce_min_sync(0xffffffffu, mine);
+        if ((threadIdx.x & 31) == 0) atomicMin(least, of_warp);
+        in_front[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    return *least;
 }
 
-__global__ void __launch_bounds__(SELECT_THREADS, 4) sample_top_k_kernel(
+// The k-th largest of keys[0 .. n - 1] (n >= k), the same in all threads: the largest number that k keys reach, four bits a turn,
+// each of sixteen warps counting for one value of the four.  For lists where counting all pairs takes longer.
+__device__ __noinline__ unsigned int kth_of_many(const unsigned int* keys, int n, int k, unsigned int (*enough)[16]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int reached = 0;
+    int turn = 0;
+    for (int shift = 28; shift >= 0; shift -= 4, turn ^= 1) {
+        const unsigned int wanted = reached | ((unsigned int)warp << shift);
+        unsigned int count = 0;
+        for (int i = lane; i < n; i += 32) count += keys[i] >= wanted;
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == 0) enough[turn][warp] = count >= (unsigned int)k;
+        __syncthreads();  // two sets of answers in turn: one barrier a turn
+        const unsigned int those = __ballot_sync(0xffffffffu, enough[turn][lane & 15] != 0) & 0xffffu;
+        reached |= (31u - __clz(those)) << shift;
+    }
+    return reached;
+}
+
+// The thresholds of all rows, for sample_kernel.
+__global__ void __launch_bounds__(1024, 1) top_k_threshold_kernel(const float* __restrict__ logits, long long row_stride, int vocab, int top_k,
+                                                                  unsigned int* __restrict__ threshold) {
+    __shared__ SelectShared sh;
+    pdl_launch_dependents();
+    pdl_wait();
+    uint32_t n_ranks;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(n_ranks));
+    const int r = blockIdx.x / (int)n_ranks, rank = blockIdx.x % (int)n_ranks;  // the cluster's blocks are consecutive
+    const int per = (vocab + (int)n_ranks - 1) / (int)n_ranks;
+    const int begin = min(rank * per, vocab), end = min(begin + per, vocab);
+    const unsigned int found = radix_threshold(logits + (size_t)r * row_stride, begin, end, top_k, (int)n_ranks, 0u, sh);
+    if (threadIdx.x == 0 && rank == 0) threshold[r] = found;
+    cluster_barrier();  // nobody leaves while its histogram may still be read
+}
+
+__global__ void __launch_bounds__(SELECT_THREADS, 3) sample_top_k_kernel(
     const float* __restrict__ logits, long long row_stride, int vocab, int top_k, float temperature, unsigned long long seed,
     const int* __restrict__ request_ids, int* __restrict__ steps, int advance_steps, int* __restrict__ out) {
     __shared__ SelectShared sh;
     __shared__ Best scratch[32], block_result;
     __shared__ __align__(16) unsigned int keys[CANDIDATES];  // first the groups' largest keys, then the candidates' keys
-    __shared__ unsigned int own_keys[MAX_GROUPS], bound;
-    __shared__ float values[CANDIDATES];
-    __shared__ int indices[CANDIDATES], n_candidates;
+    __shared__ unsigned int own_keys[MAX_KEYS], enough[2][16], in_front[MAX_KEYS], bounds[2], n_above;
+    __shared__ CandidateList list;
     pdl_launch_dependents();
     pdl_wait();
     uint32_t n_ranks_raw;
@@ -280,12 +405,17 @@ __global__ void __launch_bounds__(SELECT_THREADS, 4) sample_top_k_kernel(
     const float* row = logits + (size_t)r * row_stride;
     const int per = (vocab + n_ranks - 1) / n_ranks;
     const int begin = min(rank * per, vocab), end = min(begin + per, vocab);
-    const Draw draw{temperature, seed, (unsigned long long)(unsigned int)request_ids[r], (unsigned long long)(unsigned int)steps[r]};
+    const auto key_of_row = [&] { return Draw{temperature, seed, (unsigned long long)(unsigned int)request_ids[r], (unsigned long long)(unsigned int)steps[r]}; };
     Best mine{-INFINITY, 0x7fffffff};
-    bool settled = false;  // the same in all blocks of the cluster
-    const int lanes = 2 * top_k <= n_ranks * (SELECT_THREADS / 32) ? 32 : 8, groups = SELECT_THREADS / lanes;  // of a group; in a block
-    if (2 * top_k <= n_ranks * groups) {
-        if (threadIdx.x == 0) n_candidates = 0;
+    bool settled = false, known = false;  // the same in all blocks of the cluster
+    unsigned int threshold = 0;           // the k-th largest key, where it is known
+    int lanes = 32;                       // of a group
+    while (lanes > 1 && 2 * top_k > n_ranks * (SELECT_THREADS / lanes) && n_ranks * (SELECT_THREADS / lanes) < MAX_KEYS) lanes /= 2;
+    const int groups = SELECT_THREADS / lanes;  // in a block
+    unsigned int least = 0;  // no smaller key can be the k-th largest
+    if (2 * top_k <= n_ranks * groups) {  // so it is for every top_k that comes here, up to half of MAX_KEYS
+        if (threadIdx.x == 0) list.count = 0, n_above = 0, bounds[0] = bounds[1] = 0xffffffffu;
+        in_front[threadIdx.x] = 0;
         unsigned int largest = 0;  // below every key but that of the NaN of all ones
         scan_slice(row, begin, end, [&](float x, int) { largest = max(largest, float_key(x)); });
         for (int o = 1; o < lanes; o <<= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
@@ -293,36 +423,57 @@ __global__ void __launch_bounds__(SELECT_THREADS, 4) sample_top_k_kernel(
         cluster_barrier();
         for (int i = threadIdx.x; i < n_ranks * groups; i += SELECT_THREADS) keys[i] = remote_read(&own_keys[i % groups], i / groups);
         __syncthreads();
-        kth_largest(keys, n_ranks * groups, top_k, &bound);
-        __syncthreads();
-        const unsigned int reach = bound;
-        const uint32_t counter = remote_address(&n_candidates, 0), to_value = remote_address(values, 0), to_index = remote_address(indices, 0);
-        scan_slice(row, begin, end, [&](float x, int i) {
-            if (float_key(x) < reach) return;
+        const int n_keys = n_ranks * groups;
+        unsigned int reach;
+        if (n_keys <= 256) {
+            reach = least_of_first(keys, n_keys, top_k, 0, n_keys, in_front, &bounds[0]);
+        } else {  // every block looks among its own groups' keys
+            least_of_first(keys, n_keys, top_k, rank * groups, groups, in_front, &bounds[0]);
+            cluster_barrier();
+            reach = 0xffffffffu;
+            for (int b = 0; b < n_ranks; ++b) reach = min(reach, remote_read(&bounds[0], b));
+        }
+        const uint32_t first_list = remote_address(&list, 0);
+        bool full = false;
+        unsigned int above = 0;
+        scan_reaching(row, begin, end, reach, [&](float x, int i) {
+            above += float_key(x) > reach;
+            if (full) return;
+            // one request for all lanes that stand here together
+            const unsigned int here = __activemask(), leader = __ffs(here) - 1, lane = threadIdx.x & 31;
             unsigned int at;
-            asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], 1;" : "=r"(at) : "r"(counter) : "memory");
+            if (lane == leader) asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at) : "r"(first_list + (uint32_t)offsetof(CandidateList, count)), "r"(__popc(here)) : "memory");
+            at = __shfl_sync(here, at, leader) + __popc(here & ((1u << lane) - 1));
             if (at < CANDIDATES) {
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to_value + 4 * at), "f"(x) : "memory");
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to_index + 4 * at), "r"(i) : "memory");
+                asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(first_list + 8 * at), "r"(__float_as_uint(x)), "r"(i) : "memory");
+            } else {
+                full = true;
             }
         });
+        for (int o = 1; o < 32; o <<= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(&n_above, above);
         cluster_barrier();
-        const int n = (int)remote_read(&n_candidates, 0);
+        const int n = (int)remote_read(&list.count, 0);
         settled = n <= CANDIDATES;
         if (settled && rank == 0) {
-            for (int i = threadIdx.x; i < n; i += SELECT_THREADS) keys[i] = float_key(values[i]);
+            for (int i = threadIdx.x; i < n; i += SELECT_THREADS) keys[i] = float_key(__int_as_float(list.entries[i].x));
             __syncthreads();
-            kth_largest(keys, n, top_k, &bound);
-            __syncthreads();
+            const unsigned int kth = n <= MAX_KEYS ? least_of_first(keys, n, top_k, 0, n, in_front, &bounds[1]) : kth_of_many(keys, n, top_k, enough);
+            const Draw draw = key_of_row();
             for (int i = threadIdx.x; i < n; i += SELECT_THREADS)
-                if (keys[i] >= bound) mine = better(mine, draw.of(values[i], indices[i]));
+                if (keys[i] >= kth) mine = better(mine, draw.of(__int_as_float(list.entries[i].x), list.entries[i].y));
+        }
+        if (!settled) {  // fewer than k logits above the bound, which at least k reach: it is the k-th largest itself
+            unsigned int all = 0;
+            for (int b = 0; b < n_ranks; ++b) all += remote_read(&n_above, b);
+            known = all < (unsigned int)top_k;
+            threshold = least = reach;
         }
     }
     if (!settled) {
-        const unsigned int threshold = radix_threshold(row, begin, end, top_k, n_ranks, sh);
-        scan_slice(row, begin, end, [&](float x, int i) {
-            if (float_key(x) >= threshold) mine = better(mine, draw.of(x, i));
-        });
+        if (!known) threshold = radix_threshold(row, begin, end, top_k, n_ranks, least, sh);
+        const Draw draw = key_of_row();
+        scan_reaching(row, begin, end, threshold, [&](float x, int i) { mine = better(mine, draw.of(x, i)); });
     }
     if (!settled || rank == 0) {
         const Best b = block_best(mine, scratch);
@@ -339,9 +490,10 @@ __global__ void __launch_bounds__(SELECT_THREADS, 4) sample_top_k_kernel(
     cluster_barrier();  // nobody leaves while its result may still be read
 }
 
-// Grid (parts, rows): the best of  logit / T + Gumbel noise  over the block's slice of the row.
+// Grid (parts, rows): the best of  logit / T + Gumbel noise  over the block's slice of the row, among the logits whose key reaches
+// the row's threshold (`threshold` null: all).
 __global__ void sample_kernel(const float* __restrict__ logits, long long row_stride, int vocab, float temperature,
-                              unsigned long long seed,
+                              const unsigned int* __restrict__ threshold, unsigned long long seed,
                               const int* __restrict__ request_ids, int* __restrict__ steps, int advance_steps,
                               int* __restrict__ out, Best* __restrict__ partial) {
     __shared__ Best scratch[32];
@@ -353,7 +505,10 @@ __global__ void sample_kernel(const float* __restrict__ logits, long long row_st
     const int begin = part * per, end = min(begin + per, vocab);
     const Draw draw{temperature, seed, (unsigned long long)(unsigned int)request_ids[r], (unsigned long long)(unsigned int)steps[r]};
     Best mine{-INFINITY, 0x7fffffff};
-    scan_slice(row, begin, end, [&](float x, int i) { mine = better(mine, draw.of(x, i)); });
+    const unsigned int least = threshold != nullptr ? threshold[r] : 0u;
+    scan_slice(row, begin, end, [&](float x, int i) {
+        if (float_key(x) >= least) mine = better(mine, draw.of(x, i));
+    });
     Best b = block_best(mine, scratch);
     if (threadIdx.x == 0) {
         if (parts == 1) {
@@ -385,7 +540,8 @@ GK_EXPORT int gk_argmax(const float* logits, long long row_stride, int n_rows, i
     return GK_OK;
 }
 
-// `scratch`: 8 bytes * n_rows * parts for the parts' results (temperature alone, rows cut into parts).
+// `scratch`: 4 bytes * n_rows for thresholds (rounded up to 8), then 8 bytes * n_rows * parts for the parts' results; not read with
+// a top_k of up to half of MAX_KEYS.
 GK_EXPORT int gk_sample(const float* logits, long long row_stride, int n_rows, int vocab, float temperature, int top_k,
                         unsigned long long seed, const int* request_ids, int* steps, int advance_steps, int* out,
                         int parts, void* scratch, void* stream) {
@@ -393,28 +549,38 @@ GK_EXPORT int gk_sample(const float* logits, long long row_stride, int n_rows, i
     GK_REQUIRE(temperature > 0.f, "sample: temperature must be positive (0 means greedy: call argmax)");
     GK_REQUIRE(top_k >= 0, "sample: top_k must be >= 0 (0 = off)");
     GK_REQUIRE(parts >= 1 && parts <= 1024 && n_rows <= 65535, "sample: bad split %d of %d rows", parts, n_rows);
-    const bool select = top_k > 0 && top_k < vocab;
-    GK_REQUIRE(parts == 1 || select || scratch, "sample: scratch is needed when a row is split");
+    const bool select = top_k > 0 && top_k < vocab, short_way = select && top_k <= MAX_KEYS / 2;
+    GK_REQUIRE((parts == 1 && !select) || short_way || scratch, "sample: scratch is needed for a large top_k and when a row is split");
     if (n_rows == 0) return GK_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    if (select) {
-        // As many blocks a row as leaves all of them on the GPU at once (four of 512 threads fit an SM).  Measured (64 rows
-        // of 151,936, k = 50), before with four counting scans, a scan that draws and a join in three kernels: 71.7 us, now 28.6.
-        static const int n_sms = [] {
-            int device = 0, n = 0;
-            if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n = 148;
-            return n;
-        }();
-        int blocks = SELECT_BLOCKS;
-        while (blocks > 1 && (long long)n_rows * blocks > 4LL * n_sms) blocks /= 2;
+    static const int n_sms = [] {
+        int device = 0, n = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n = 148;
+        return n;
+    }();
+    int blocks = SELECT_BLOCKS;
+    if (short_way) {
+        // As many blocks a row as leaves all of them on the GPU at once (three of 512 threads fit an SM).  Measured (us; the threshold by
+        // four counting scans, a scan that draws and a join in three kernels / here): 64 rows of 151,936, k = 50: 65.4 / 17.4, k = 200:
+        // 66.8 / 24.6; 64 rows of 32,000, k = 200: 30.0 / 17.0; one row of 151,936, k = 50: 24.6 / 10.7.  Rows of equal numbers: 64: 101 /
+        // 86, one: 29.8 / 36 (its eight blocks form all the noise, which the three kernels spread); rows masked down to 25: 64: 116 / 59,
+        // one: 32.4 / 28.  Larger k: the three kernels; in one kernel a row of 151,936 took 32 instead of 24.6 us with k = 257.
+        while (blocks > 1 && (long long)n_rows * blocks > 3LL * n_sms) blocks /= 2;
         gk_launch_cluster(sample_top_k_kernel, dim3(n_rows * blocks), dim3(SELECT_THREADS), 0, s, dim3(blocks, 1, 1), logits, row_stride,
                           vocab, top_k, temperature, seed, request_ids, steps, advance_steps, out);
         GK_CHECK_LAUNCH("sample_top_k");
         return GK_OK;
     }
-    Best* partial = (Best*)scratch;
-    gk_launch(sample_kernel, dim3(parts, n_rows), dim3(256), 0, s, logits, row_stride, vocab, temperature, seed, request_ids, steps,
-              advance_steps, out, partial);
+    unsigned int* threshold = select ? (unsigned int*)scratch : nullptr;
+    Best* partial = (Best*)((char*)scratch + 8 * (((size_t)n_rows + 1) / 2));  // 8-byte aligned, after the thresholds
+    if (select) {
+        while (blocks > 1 && (long long)n_rows * blocks > 2LL * n_sms) blocks /= 2;  // two of 1,024 threads fit an SM
+        gk_launch_cluster(top_k_threshold_kernel, dim3(n_rows * blocks), dim3(1024), 0, s, dim3(blocks, 1, 1), logits, row_stride, vocab, top_k,
+                          threshold);
+        GK_CHECK_LAUNCH("top_k_threshold");
+    }
+    gk_launch(sample_kernel, dim3(parts, n_rows), dim3(256), 0, s, logits, row_stride, vocab, temperature, (const unsigned int*)threshold, seed,
+              request_ids, steps, advance_steps, out, partial);
     GK_CHECK_LAUNCH("sample");
     if (parts > 1) {
         gk_launch(best_merge_kernel, dim3(n_rows), dim3(32), 0, s, (const Best*)partial, parts, out, advance_steps ? steps : (int*)nullptr);

@@ -930,6 +930,9 @@ def argmax(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tenso
     return out
 
 
+TOP_K_IN_ONE_KERNEL = 256  # half of the groups of csrc/sampling.cu
+
+
 def sample(
     logits: torch.Tensor,
     temperature: float,
@@ -954,11 +957,12 @@ def sample(
     if out is None:
         out = torch.empty((n,), dtype=torch.int32, device=logits.device)
     _check(out, "out", torch.int32, 1)
-    # as for argmax: several blocks share a row, eight bytes of scratch per row and part for the parts' results (with
-    # top-k a cluster shares a row and needs none)
+    # as for argmax: several blocks share a row; eight bytes of scratch per row for a threshold (four used) and eight per
+    # row and part for the parts' results (a cluster that shares a row, for a top-k of up to 256, needs none)
     parts = row_parts(n, vocab, logits.device)
-    cut = parts > 1 and not 0 < int(top_k or 0) < vocab
-    scratch = torch.empty((2 * n * parts,), dtype=torch.int32, device=logits.device) if cut else None
+    select = 0 < int(top_k or 0) < vocab
+    whole = int(top_k or 0) <= TOP_K_IN_ONE_KERNEL if select else parts == 1
+    scratch = None if whole else torch.empty((2 * ((n + 1) // 2) + 2 * n * parts,), dtype=torch.int32, device=logits.device)
     call(
         "gk_sample", ptr(logits), vocab, n, vocab, float(temperature), int(top_k or 0), int(seed) & (2**64 - 1),
         ptr(request_ids), ptr(steps), int(advance_steps), ptr(out), parts, ptr(scratch), stream_ptr(),

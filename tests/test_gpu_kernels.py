@@ -969,3 +969,40 @@ def test_attention_exact_of_many_sequences_does_not_walk_them_one_after_another(
         return device_time(lambda: F().attention_exact(q, kv, pos, seq, at, d**-0.5))
 
     assert step(runs) < 2 * sum(step(part) for part in parts)
+
+
+@pytest.mark.parametrize("rows,vocab,top_k", [(3, 40001, 100), (2, 151936, 200), (200, 9001, 33), (300, 2500, 256), (2, 3000, 256), (1, 2049, 130)])
+@pytest.mark.parametrize("values", ["spread", "few", "one above", "tied", "sorted", "nearly masked"])
+def test_sample_top_k_where_many_reach_the_bound(rows, vocab, top_k, values):
+    """More logits at the bound than the list holds, with fewer and with more than k of them above it; as many at the k-th place as
+    beside it; every number of lanes a group; clusters of one, two and four blocks."""
+    gen = torch.Generator().manual_seed(vocab + top_k)
+    logits = torch.randn(rows, vocab, generator=gen) * 3
+    if values == "few":
+        logits = (logits / 6).round()
+    elif values == "one above":
+        logits = torch.full((rows, vocab), -1.5)
+        logits[:, vocab // 3] = 2.0
+    elif values == "tied":
+        logits = torch.where(torch.rand(rows, vocab, generator=gen) < 0.6, torch.tensor(1.0), logits.clamp(max=0.5))
+        logits[:, ::977] = 2.5
+    elif values == "sorted":
+        logits = logits.sort(dim=1, descending=True).values
+    elif values == "nearly masked":
+        logits = torch.where(torch.rand(rows, vocab, generator=gen) < (top_k - 0.5) / vocab, logits, torch.tensor(-math.inf))
+    requests, steps = torch.arange(3, 3 + rows, dtype=torch.int32), torch.arange(rows, dtype=torch.int32) % 5
+    got = F().sample(logits.to(DEV), 0.7, top_k, 78, requests.to(DEV), steps.to(DEV)).cpu().tolist()
+    for i in sorted({0, rows // 2, rows - 1}):
+        assert got[i] == plain_sampling.sample(logits[i].numpy(), 0.7, top_k, 78, int(requests[i]), int(steps[i])), f"row {i}"
+
+
+@pytest.mark.parametrize("rows,top_k", [(8, 50), (8, 200), (64, 200)])
+def test_sample_top_k_of_equal_and_masked_rows_costs_no_more_scans(rows, top_k):
+    """Rows in which most logits reach the bound against rows in which few do.  Measured: equal numbers 2.7 to 3.7 times, masked down to
+    k / 2 numbers 2.0 to 2.6 times; one request a logit and the scans of a larger k behind it: 5.1 and 5.6 (8 rows, k = 50)."""
+    spread = torch.randn(rows, 151936, generator=torch.Generator().manual_seed(1)).to(DEV)
+    equal, masked = torch.full_like(spread, 0.25), spread.clone()
+    masked[:, top_k // 2:] = -math.inf
+    requests, steps = torch.arange(rows, dtype=torch.int32).to(DEV), torch.zeros(rows, dtype=torch.int32).to(DEV)
+    took = [device_time(lambda: F().sample(x, 0.8, top_k, 7, requests, steps)) for x in (spread, equal, masked)]
+    assert took[1] < 4.6 * took[0] and took[2] < 4 * took[0], took
