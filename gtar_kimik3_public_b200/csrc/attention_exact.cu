@@ -441,7 +441,7 @@ size_t single_smem(int d, int group) {
 // Some 25 us a span of 1,024 keys (16/8 heads of 128, 32-bit), 2 of them the chain over the keys, 4 cycles each; the others are
 // the scores of one block of keys a warp, the exchange and its barriers, and the wait for the values.  Keys and values share a
 // place in shared memory, so that two blocks (three in bfloat16) are on an SM.  Measured (us; the wide kernel / here): one token after
-// 3,000: 1,262 / 78; sixteen: 2,451 / 191.  A token with no more than SHORT_KEYS keys takes a warp a head.
+// 3,000: 1,262 / 73; sixteen: 2,451 / 183.  A token with no more than SHORT_KEYS keys takes a warp a head.
 template <typename T, int GP>
 __global__ void __launch_bounds__(SINGLE_WARPS * 32, GP <= 8 ? 3 : 2) attention_exact_single_kernel(const Exact p) {
     constexpr int PAD = 16 / sizeof(T), LDK = K_PIECE + PAD, THREADS = SINGLE_WARPS * 32;
@@ -780,10 +780,10 @@ struct Route {
 };
 
 // single: up to two and a half turns of the clusters that are on the device at once.  Measured (us, single / warps; 16/8 heads of 128,
-//   32-bit; 16 tokens after 10, 1,000 and 3,000): 10.5, 66, 191 / 5.9, 202, 588; 32/8 heads of 64, bfloat16, 64 tokens after 10, 1,000
+//   32-bit; 16 tokens after 10, 1,000 and 3,000): 10.3, 64, 183 / 5.9, 202, 588; 32/8 heads of 64, bfloat16, 64 tokens after 10, 1,000
 //   and 3,000: 13.5, 115, 332 / 7.0, 158, 460.
 // tiles:  for steps beyond 16 warp units or 32 rows an SM, where a run can be long enough to fill tiles.  Measured (us, tiles /
-//   warps; 16/8 heads of 128, 32-bit): 512 tokens after 1,000: 372 / 975; 64 single tokens after 1,000 and a prompt of 512: 388 / 660;
+//   warps; 16/8 heads of 128, 32-bit): 512 tokens after 1,000: 372 / 975; 64 single tokens after 1,000 and a prompt of 512: 376 / 660;
 //   640 tokens in 16 runs of 40: 63 / 42; 16/1 heads of 128, 512 after 1,000: 381 / 559; 6/2 heads of 32, the same: 257 / 176.
 // The mixed step took 7,477 us with tiles that walk every run of theirs, 64 tokens after 10 141 us with a cluster each (here 7), and
 // the wide kernel for all of them 881 and 10.

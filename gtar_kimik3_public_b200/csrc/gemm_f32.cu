@@ -80,10 +80,9 @@ constexpr size_t tile_smem() {
     return (size_t)TILE_STAGES * (BM * (TILE_BK + 16 / sizeof(TA)) * sizeof(TA) + BN * (TILE_BK + 4) * sizeof(float));
 }
 
-// Bound by the register file and shared memory together: FFMAs issue in 57% of the cycles at 64 x 64, with the operands'
-// bank conflicts (dispatch stalls) and 16-byte reads (55% of shared memory's cycles) beside them; 41 TFLOP/s at 4,096^2.
-// What it measured, and what the one tile of 128 x 128 with plain loads between two barriers measured before, stands at
-// the launch rule.
+// Bound by the FP32 pipes, at a little over half of what two-number multiply-adds reach: one chain step an instruction, with the
+// 16-byte reads of both operands beside them.  41 TFLOP/s at 2,048 x 4,096 x 4,096.  What it measured, and what the one tile of
+// 128 x 128 with plain loads between two barriers measured before, stands at the launch rule.
 template <typename TA, typename TC, int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_f32_tile_kernel(const Product p) {
     constexpr int THREADS = (BM / TM) * (BN / TN), BK = TILE_BK, S = TILE_STAGES;

@@ -58,7 +58,8 @@ class RoutedExperts(FeedForward):
         self.w_shared_gate_up = self.w_shared_down = None
         self.w_gate_up = self.w_down = self.w_router = self.correction = None
         # from this many (token, expert) pairs on, a bfloat16 step sorts its pairs by expert and runs each expert's rows
-        # through one tensor-core product; below, every pair streams its expert's weights by itself
+        # through one tensor-core product; below, the library's own kernels take an expert's pairs together or one by one.  The
+        # number was set when they took every pair by itself
         self.grouped_from_pairs = 256
 
     def tensor_specs(self):

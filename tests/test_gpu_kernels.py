@@ -952,9 +952,9 @@ def device_time(step, repeats=5):
 
 
 @pytest.mark.parametrize("runs,parts", [
-    ([(1, 1000)] * 64 + [(512, 0)], ([(1, 1000)] * 64, [(512, 0)])),  # measured 2.1 times the larger part; a tile that walks its 32 runs: 30
-    ([(3, 1000)] * 64, ([(1, 1000)] * 64,) * 3),  # measured 0.5 of the parts' sum; tiles that walk ten runs each: 7
-    ([(1, 10)] * 64, ([(1, 10)],) * 4),  # measured 0.4; a cluster a token and kv head: 3.7
+    ([(1, 1000)] * 64 + [(512, 0)], ([(1, 1000)] * 64, [(512, 0)])),  # measured 1.0 times their sum; tiles that walk every run of theirs: 13
+    ([(3, 1000)] * 64, ([(1, 1000)] * 64,) * 3),  # measured 0.5; tiles that walk ten runs each: 2.4
+    ([(1, 10)] * 64, ([(1, 10)],) * 4),  # measured 0.3; a cluster a token and kv head: 3.5
 ])
 def test_attention_exact_of_many_sequences_does_not_walk_them_one_after_another(runs, parts):
     """A step takes at most twice as long as the steps that it could be cut into, one after another."""
