@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(TILE_WARPS * 32, 2) attention_exact_tile_kerne
 }
 
 // ------------------------------------------------------------------ single
-constexpr int SINGLE_WARPS = 8, SPAN = 1024, SPAN_BLOCKS = SPAN / KEYS, V_KEYS = 128, V_STAGES = 3, K_PIECE = 32, MAX_GROUP = 16, SHORT_KEYS = 64;
+constexpr int SINGLE_WARPS = 8, SPAN = 1024, SPAN_BLOCKS = SPAN / KEYS, V_KEYS = 128, V_STAGES = 3, K_PIECE = 32, MAX_GROUP = 16, SHORT_KEYS = 32;
 
 __host__ __device__ inline int single_ranks(int d) { return d <= 32 ? 1 : d <= 64 ? 2 : 4; }
 __host__ __device__ inline int single_slice(int d) { return (((d + single_ranks(d) - 1) / single_ranks(d)) + 7) / 8 * 8; }
@@ -441,7 +441,8 @@ size_t single_smem(int d, int group) {
 // Some 25 us a span of 1,024 keys (16/8 heads of 128, 32-bit), 2 of them the chain over the keys, 4 cycles each; the others are
 // the scores of one block of keys a warp, the exchange and its barriers, and the wait for the values.  Keys and values share a
 // place in shared memory, so that two blocks (three in bfloat16) are on an SM.  Measured (us; the wide kernel / here): one token after
-// 3,000: 1,262 / 73; sixteen: 2,451 / 183.  A token with no more than SHORT_KEYS keys takes a warp a head.
+// 3,000: 1,262 / 73; sixteen: 2,451 / 183.  A token whose keys lie in one block of them
+// takes a warp a head; with two blocks that is slower (a prompt of 64, 6/2 heads of 32: 6.9 against 6.2).
 template <typename T, int GP>
 __global__ void __launch_bounds__(SINGLE_WARPS * 32, GP <= 8 ? 3 : 2) attention_exact_single_kernel(const Exact p) {
     constexpr int PAD = 16 / sizeof(T), LDK = K_PIECE + PAD, THREADS = SINGLE_WARPS * 32;
