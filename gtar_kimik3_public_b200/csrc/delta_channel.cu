@@ -1,0 +1,762 @@
+// The gated delta rule with a decay per head and key channel (see delta_rule.cu) over many tokens at once, for bfloat16 steps:
+// everything between the layer's input projections and its output projection in three kernels.
+//
+// With S0 the state before a chunk of 64 tokens and G_t = g_0 * .. * g_t per channel, the writes u_t solve
+//     u_t = beta_t (v_t - (k_t G_t)^T S0 - sum_{j<t} (k_t . (k_j g_{j+1} .. g_t)) u_j)
+// so with A_tj = beta_t sum_c k_tc k_jc g_{j+1,c} .. g_tc below the diagonal
+//     u  = U - W S0                   U = (1 + A)^-1 diag(beta) V,   W = (1 + A)^-1 diag(beta) (K o G)
+//     o  = (Q o G) S0 + P u           P_tj = sum_c q_tc k_jc g_{j+1,c} .. g_tc for j <= t
+//     S1 = diag(G_last) S0 + (K o g_{t+1} .. g_last)^T u
+// (the chunked form of the delta rule: S. Yang, B. Wang, Y. Zhang, Y. Shen, Y. Kim, "Parallelizing Linear Transformers with the
+// Delta Rule over Sequence Length"; decays per channel by blocks inside a chunk: S. Yang, B. Wang, Y. Shen, R. Panda, Y. Kim, "Gated
+// Linear Attention Transformers with Hardware-Efficient Training".)
+//
+// Products of decays are never divided: between two blocks of 16 tokens a term's decays are (from the later block's start to t) x
+// (whole blocks between) x (from j to the end of j's block), all at most one; inside a block they are multiplied up token by token.
+// So nothing overflows however strong the decays, and no logarithm is taken.
+//
+//   inner   a block per chunk and head: convolutions, SiLU, unit lengths, decays, beta; A, P, W, U and the scaled keys and queries
+//   walk    a block per head and 8 value columns, the chunks in sequence: 128 x 8 numbers of state in the accumulators of eight warps
+//   read    a block per chunk and head: o, RMS norm over a head, weight and gate
+//
+// Every matrix product takes 32-bit operands: each number is split into two TF32 numbers (rounded, and the rounded rest), three
+// mma.sync a product, what is left out is 2^-24 of it; the large parts are added up by 32-bit additions outside the tensor core,
+// whose own sums are cut and not rounded (H. Ootomo, R. Yokota, "Recovering single precision accuracy from Tensor Cores while
+// surpassing the FP32 theoretical peak performance").  FFMA instead would be bound by what shared memory can deliver.
+//
+// Measured (us, the kernels that go token by token / here; heads of 128): one prompt of 2,048, 8 heads: 620 / 189; 1,024 + 500 + 77
+// tokens, 16 heads: 537 / 341; 100 + 40 + 900, 8 heads: 304 / 142.  Error of the states against 64 bits, relative: 4.07e-7 both ways at the
+// first, 3.2e-7 / 3.3e-7 at the second, 1.6e-7 / 2.0e-7 after 16 tokens; of the bfloat16 read-outs 1.66e-3 both ways.  `inner` is bound by latency (57 us
+// of the 189: its phases follow one another, two blocks an SM), `walk` by its two products and three barriers a chunk (2 us).
+
+#include "common.cuh"
+
+namespace {
+
+typedef __nv_bfloat16 bf16;
+
+constexpr int CHUNK = 64, SUB = 16, STRIP = 8;
+constexpr int THREADS = 256;
+constexpr int MAX_TAPS = 4;
+constexpr int TILE16 = SUB * SUB;
+
+// 32-bit numbers a chunk and head leaves in the workspace
+template <int D>
+struct Unit {
+    static constexpr int W = 0;                    // left operand of the walk's first product, in fragments [4][D/8][32] of four
+    static constexpr int K = W + CHUNK * D;        // left operand of its second product, in fragments [D/16][8][32]
+    static constexpr int Q = K + CHUNK * D;        // left operand of the read-out, in fragments [4][D/8][32]
+    static constexpr int P = Q + CHUNK * D;        // and within the chunk, in fragments [4][8][32]; what lies above the diagonal is not written
+    static constexpr int G = P + CHUNK * CHUNK;    // decays over the whole chunk
+    static constexpr int U = G + D;                // [64][dv]: U, then u
+    static constexpr int S = U + CHUNK * D;        // [D][dv]: the state before the chunk
+    static constexpr int SIZE = S + D * D;
+};
+
+// Quotients without the branch that a rounded division carries for numbers out of range, so that a thread's many are worked out side by side
+__device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + expf(fminf(-z, 80.f))); }
+__device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.f, 1.f + expf(fminf(-z, 80.f))); }
+__device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+
+__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// To the nearest number of ten fraction bits, ties away from zero.  (The conversion instruction does the same at an eighth of the rate of
+// these two.)
+__device__ __forceinline__ uint32_t tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
+__device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
+    hi = tf32(x);
+    lo = tf32(x - __uint_as_float(hi));
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Left operand, 16 x 8: lane 4 r + c holds rows r, r + 8 of two columns, in the order (r, first), (r + 8, first), (r, second),
+// (r + 8, second).  Which two columns is free as long as the right operand's two rows are the same ones: 2c and 2c + 1 where an
+// accumulator becomes an operand (no exchange between lanes), c and c + 4 where rows lie four banks apart.
+struct Left {
+    uint32_t hi[4], lo[4];
+    __device__ __forceinline__ Left(float a, float b, float c, float d) {
+        split(a, hi[0], lo[0]);
+        split(b, hi[1], lo[1]);
+        split(c, hi[2], lo[2]);
+        split(d, hi[3], lo[3]);
+    }
+};
+struct Sum {
+    float acc[4], low[4];  // the large parts, and the small ones, whose sums may be the tensor core's own
+    __device__ __forceinline__ Sum() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = low[i] = 0.f;
+    }
+    __device__ __forceinline__ void add(const Left& a, uint32_t h0, uint32_t h1, uint32_t l0, uint32_t l1) {
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        mma(c, a.hi, h0, h1);
+        mma(low, a.lo, h0, h1);
+        mma(low, a.hi, l0, l1);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] += c[i];
+    }
+    __device__ __forceinline__ void add(const Left& a, float b0, float b1) {
+        uint32_t h0, h1, l0, l1;
+        split(b0, h0, l0);
+        split(b1, h1, l1);
+        add(a, h0, h1, l0, l1);
+    }
+    __device__ __forceinline__ float at(int i) const { return acc[i] + low[i]; }
+};
+
+// entry (t, j) of a 16 x 16 block in shared memory: pairs of columns turned so that eight rows' pairs fall into different banks
+__device__ __forceinline__ int at16(int t, int j) { return t * SUB + 2 * ((j >> 1) ^ (((t >> 1) & 1) << 2)) + (j & 1); }
+
+template <int N>
+__device__ __forceinline__ void load_row(const bf16* src, float (&x)[N]) {
+    if constexpr (N == 4) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(src);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        x[0] = a.x, x[1] = a.y, x[2] = b.x, x[3] = b.y;
+    } else {
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src));
+        x[0] = a.x, x[1] = a.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_row(const float* src, float (&x)[N]) {
+    if constexpr (N == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(src);
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+    } else {
+        const float2 a = *reinterpret_cast<const float2*>(src);
+        x[0] = a.x, x[1] = a.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_row(float* dst, const float (&x)[N]) {
+    if constexpr (N == 4) *reinterpret_cast<float4*>(dst) = make_float4(x[0], x[1], x[2], x[3]);
+    else *reinterpret_cast<float2*>(dst) = make_float2(x[0], x[1]);
+}
+
+struct Inputs {
+    const bf16* proj;        // [T, ld]: q | k | v | b
+    const float* low;        // [T, ld_low]: decays | gate
+    const float* conv_w;     // [channels, taps]
+    float* conv_state;       // [slots, taps - 1, channels]
+    const float *a_log, *dt_bias, *norm;
+    const int *cu_q, *slots;
+    long long ld, ld_low;
+    int n_heads, n_kv, dv, taps, chunk0, wave;
+};
+
+// Eight consecutive tokens' convolution and SiLU of N neighbouring channels from column c on; s0: the first token's place in the
+// step, `live` of the eight are there.  Inputs before the step come from the sequence's convolution state.
+template <int N>
+__device__ __forceinline__ void conv_eight(const Inputs& in, int tok, int s0, int live, size_t slot, int c, int channels, float (&y)[8][N]) {
+    const int taps = in.taps;
+    float w[MAX_TAPS][N], x[8 + MAX_TAPS - 1][N];
+#pragma unroll
+    for (int j = 0; j < MAX_TAPS; ++j)
+#pragma unroll
+        for (int e = 0; e < N; ++e) w[j][e] = j < taps ? in.conv_w[(size_t)(c + e) * taps + taps - 1 - j] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 8 + MAX_TAPS - 1; ++i) {
+        const int back = i - (MAX_TAPS - 1), s = s0 + back;
+#pragma unroll
+        for (int e = 0; e < N; ++e) x[i][e] = 0.f;
+        if (back >= live || -back >= taps) continue;
+        if (s >= 0) load_row<N>(in.proj + (long long)(tok + back) * in.ld + c, x[i]);
+        else if (taps - 1 + s >= 0) load_row<N>(in.conv_state + (slot * (taps - 1) + (taps - 1 + s)) * channels + c, x[i]);
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            float z = 0.f;
+#pragma unroll
+            for (int j = 0; j < MAX_TAPS; ++j)
+                if (j < taps) z = fmaf(w[j][e], x[t + MAX_TAPS - 1 - j][e], z);
+            y[t][e] = t < live ? silu_f(z) : 0.f;
+        }
+}
+
+template <int D>
+struct InnerSmem {
+    static constexpr int LD = D + 4;  // rows four banks apart
+    float k[CHUNK][LD], g[CHUNK][LD], q[CHUNK][LD];
+    float blk[10][TILE16];            // (1 + A)^-1 of the four blocks on the diagonal, then the six of A below it
+    float total[4][D];                // decays over a block
+    float beta[CHUNK];
+};
+
+template <int D>
+__global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, float* __restrict__ work) {
+    constexpr int N = D / 32, KS = D / 8, LD = InnerSmem<D>::LD;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    InnerSmem<D>& sm = *reinterpret_cast<InnerSmem<D>*>(smem_raw);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.y, seq = blockIdx.z, hk = head / (in.n_heads / in.n_kv), dv = in.dv;
+    const int t0 = in.cu_q[seq], len = in.cu_q[seq + 1] - t0;
+    const int first = (in.chunk0 + blockIdx.x) * CHUNK;
+    if (first >= len) return;
+    const int n = min(CHUNK, len - first), tok0 = t0 + first;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c2 = lane & 3;
+    const int qk = in.n_kv * D, channels = 2 * qk + in.n_heads * dv;
+    const size_t slot = in.slots[seq];
+    float* mine = work + (((size_t)seq * in.wave + blockIdx.x) * in.n_heads + head) * Unit<D>::SIZE;
+
+    // ---- queries, keys, values, decays, beta: a warp has eight tokens, a lane N channels.  (Loops stay loops wherever registers allow:
+    //      the kernel runs through its code once, and code that is not in the instruction cache yet costs more than the branches.)
+    for (int i = tid; i < CHUNK * D / 4; i += THREADS) {  // what the decays are made of, on its way meanwhile
+        const int t = i / (D / 4), c = i % (D / 4) * 4;
+        if (t < n) cp_async_16(&sm.g[t][c], in.low + (long long)(tok0 + t) * in.ld_low + head * D + c);
+    }
+    cp_async_commit();
+    {
+        const int w0 = warp * 8, live = min(8, n - w0), at = lane * N;
+#pragma unroll 1
+        for (int part = 0; part < 3; ++part) {
+            const bool values = part == 2;
+            if (values && at >= dv) break;
+            float y[8][N];
+            conv_eight<N>(in, tok0 + w0, first + w0, live, slot, (values ? 2 * qk + head * dv : part * qk + hk * D) + at, channels, y);
+            if (values) {  // for now where their solutions will be
+#pragma unroll
+                for (int t = 0; t < 8; ++t) store_row<N>(mine + Unit<D>::U + (w0 + t) * dv + at, y[t]);
+                break;
+            }
+            float* to = (part == 0 ? &sm.q[w0][0] : &sm.k[w0][0]) + at;
+            float squares = 0.f;  // of token `lane`
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                float ss = 0.f;
+#pragma unroll
+                for (int e = 0; e < N; ++e) ss = fmaf(y[t][e], y[t][e], ss);
+                ss = warp_sum(ss);
+                if (lane == t) squares = ss;
+            }
+            float unit = 1.f / sqrtf(squares + 1e-6f);
+            if (part == 0) unit *= 1.f / sqrtf((float)D);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                const float mine_t = __shfl_sync(0xffffffffu, unit, t);
+#pragma unroll
+                for (int e = 0; e < N; ++e) y[t][e] *= mine_t;
+                store_row<N>(to + t * LD, y[t]);
+            }
+        }
+        if (tid < CHUNK) sm.beta[tid] = tid < n ? sigmoid_f(to_float(in.proj[(long long)(tok0 + tid) * in.ld + channels + head])) : 0.f;
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    {
+        const float rate = -expf(in.a_log[head]);
+        const int c = tid % D;
+        const float bias = in.dt_bias[head * D + c];
+#pragma unroll 2
+        for (int t = tid / D; t < CHUNK; t += THREADS / D) sm.g[t][c] = t < n ? expf(rate * softplus_f(sm.g[t][c] + bias)) : 1.f;
+    }
+    __syncthreads();
+
+    // ---- blocks on the diagonal, token by token: a warp has every other key of a block, decayed on from token to token
+    {
+        const int b = warp >> 1, odd = warp & 1, at = lane * N;
+        float held[8][N];
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+#pragma unroll
+            for (int e = 0; e < N; ++e) held[m][e] = 0.f;
+        const int value = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
+        const int j = 2 * (value & 7) + odd;
+#pragma unroll 1
+        for (int t = 0; t < SUB; ++t) {
+            float g[N], k[N], q[N], v[16];
+            load_row<N>(&sm.g[b * SUB + t][at], g);
+            load_row<N>(&sm.k[b * SUB + t][at], k);
+            load_row<N>(&sm.q[b * SUB + t][at], q);
+#pragma unroll
+            for (int m = 0; m < 8; ++m) {
+                v[m] = v[8 + m] = 0.f;
+                const bool meets = 2 * m + odd == t;  // zero until then
+#pragma unroll
+                for (int e = 0; e < N; ++e) {
+                    held[m][e] = meets ? k[e] : held[m][e] * g[e];
+                    v[m] = fmaf(k[e], held[m][e], v[m]);
+                    v[8 + m] = fmaf(q[e], held[m][e], v[8 + m]);
+                }
+            }
+            // sixteen sums over the lanes: a lane keeps half of its values at every exchange
+#pragma unroll
+            for (int o = 16, half = 8; half >= 1; o >>= 1, half >>= 1) {
+                const bool upper = (lane & o) != 0;
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                    const float send = upper ? v[i] : v[i + half], keep = upper ? v[i + half] : v[i];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            if ((lane & 1) == 0) {
+                if (value < 8) sm.blk[b][at16(t, j)] = j < t ? sm.beta[b * SUB + t] * v[0] : 0.f;
+                else mine[Unit<D>::P + ((b * 8 + 2 * b + (j >> 3)) * 32 + (t & 7) * 4 + ((j & 7) >> 1)) * 4 + (j & 1) * 2 + (t >> 3)] = v[0];
+            }
+        }
+    }
+    __syncthreads();
+    if (warp < 4) {  // (1 + A)^-1 of a block, a column a lane
+        float x[SUB];
+        float* A = sm.blk[warp];
+#pragma unroll
+        for (int i = 0; i < SUB; ++i) {
+            float p[2] = {0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < i; j += 2) {
+                const float2 a = *reinterpret_cast<const float2*>(A + at16(i, j));
+                p[0] = fmaf(a.x, x[j], p[0]);
+                if (j + 1 < i) p[1] = fmaf(a.y, x[j + 1], p[1]);
+            }
+            x[i] = (i == (lane & 15) ? 1.f : 0.f) - (p[0] + p[1]);
+        }
+        __syncwarp();
+        if (lane < SUB)
+#pragma unroll
+            for (int i = 0; i < SUB; ++i) A[at16(i, lane)] = x[i];
+    } else {  // decays from a block's start into keys and queries, and keys with the decays to the block's end in the place of the decays
+        for (int item = tid - 128; item < 4 * D; item += 128) {
+            const int c = item % D, b = item / D;
+            float g[SUB], k[SUB], run = 1.f;
+#pragma unroll
+            for (int t = 0; t < SUB; ++t) {
+                g[t] = sm.g[b * SUB + t][c];
+                k[t] = sm.k[b * SUB + t][c];
+            }
+#pragma unroll
+            for (int t = 0; t < SUB; ++t) {
+                run *= g[t];
+                sm.k[b * SUB + t][c] = k[t] * run;
+                sm.q[b * SUB + t][c] *= run;
+            }
+            sm.total[b][c] = run;
+            run = 1.f;
+#pragma unroll
+            for (int t = SUB - 1; t >= 0; --t) {
+                sm.g[b * SUB + t][c] = k[t] * run;
+                run *= g[t];
+            }
+        }
+    }
+    __syncthreads();
+
+    // ---- blocks below the diagonal: 24 products of 16 x 8 (six blocks, two halves, keys and queries), three a warp
+#pragma unroll 1
+    for (int task = warp; task < 24; task += 8) {
+        const bool queries = task >= 12;
+        const int pair = (task % 12) >> 1, nt = task & 1;
+        const int I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair - I * (I - 1) / 2;
+        const float* a = (queries ? &sm.q[I * SUB + r][0] : &sm.k[I * SUB + r][0]) + c2;
+        const float* b = &sm.g[J * SUB + nt * 8 + r][0] + c2;
+        Sum s;
+#pragma unroll 4
+        for (int ks = 0; ks < KS; ++ks) {
+            float b0 = b[8 * ks], b1 = b[8 * ks + 4];
+            for (int between = J + 1; between < I; ++between) {
+                b0 *= sm.total[between][8 * ks + c2];
+                b1 *= sm.total[between][8 * ks + c2 + 4];
+            }
+            s.add(Left(a[8 * ks], a[8 * ks + 8 * LD], a[8 * ks + 4], a[8 * ks + 8 * LD + 4]), b0, b1);
+        }
+        if (queries) {
+            reinterpret_cast<float4*>(mine + Unit<D>::P)[(I * 8 + J * 2 + nt) * 32 + lane] = make_float4(s.at(0), s.at(2), s.at(1), s.at(3));
+        } else {
+            float* to = sm.blk[4 + pair];
+            const float b0 = sm.beta[I * SUB + r], b1 = sm.beta[I * SUB + r + 8];
+            const int j = nt * 8 + 2 * c2;
+            *reinterpret_cast<float2*>(to + at16(r, j)) = make_float2(b0 * s.at(0), b0 * s.at(1));
+            *reinterpret_cast<float2*>(to + at16(r + 8, j)) = make_float2(b1 * s.at(2), b1 * s.at(3));
+        }
+    }
+    // ---- queries and keys with their decays, in the order of the operands they become
+    for (int i = warp; i < 4 * KS; i += 8) {
+        const int I = i / KS, c = (i % KS) * 8 + 2 * c2;
+        float2 x = *reinterpret_cast<const float2*>(&sm.q[I * SUB + r][c]), y = *reinterpret_cast<const float2*>(&sm.q[I * SUB + r + 8][c]);
+        for (int b = 0; b < I; ++b) {
+            const float2 f = *reinterpret_cast<const float2*>(&sm.total[b][c]);
+            x.x *= f.x, x.y *= f.y, y.x *= f.x, y.y *= f.y;
+        }
+        reinterpret_cast<float4*>(mine + Unit<D>::Q)[i * 32 + lane] = make_float4(x.x, y.x, x.y, y.y);
+    }
+    for (int i = warp; i < D / 16 * 8; i += 8) {
+        const int c = (i >> 3) * 16 + r, t = (i & 7) * 8 + 2 * c2;
+        float x[4] = {sm.g[t][c], sm.g[t][c + 8], sm.g[t + 1][c], sm.g[t + 1][c + 8]};
+        for (int b = (t >> 4) + 1; b < 4; ++b) {
+            const float f0 = sm.total[b][c], f1 = sm.total[b][c + 8];
+            x[0] *= f0, x[1] *= f1, x[2] *= f0, x[3] *= f1;
+        }
+        reinterpret_cast<float4*>(mine + Unit<D>::K)[i * 32 + lane] = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    if (tid < D) mine[Unit<D>::G + tid] = sm.total[0][tid] * sm.total[1][tid] * sm.total[2][tid] * sm.total[3][tid];
+    __syncthreads();
+
+    // ---- (1 + A)^-1 of beta K G and of beta V, block after block: a warp has 16 columns of each, which meet no others.  The transposed
+    //      system: an accumulator is the next product's left operand as it stands
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        if (warp * 16 >= (part == 0 ? D : dv)) continue;
+        const int c = warp * 16 + r;
+        const float* src = part == 0 ? &sm.k[0][0] : mine + Unit<D>::U;
+        const int ld_src = part == 0 ? LD : dv;
+        float pre[2] = {1.f, 1.f}, x[8][4];
+#pragma unroll
+        for (int I = 0; I < 4; ++I) {
+            float rest[2][4];
+            {
+                Sum s[2];
+#pragma unroll
+                for (int J = 0; J < I; ++J)
+#pragma unroll
+                    for (int ks = 0; ks < 2; ++ks) {
+                        const float* xs = x[2 * J + ks];
+                        const Left a(xs[0], xs[2], xs[1], xs[3]);
+#pragma unroll
+                        for (int nt = 0; nt < 2; ++nt) {
+                            const float2 b = *reinterpret_cast<const float2*>(&sm.blk[4 + I * (I - 1) / 2 + J][at16(nt * 8 + r, ks * 8 + 2 * c2)]);
+                            s[nt].add(a, b.x, b.y);
+                        }
+                    }
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int t = I * SUB + nt * 8 + 2 * c2 + (e & 1);
+                        rest[nt][e] = src[t * ld_src + c + 8 * (e >> 1)] * pre[e >> 1] * sm.beta[t] - s[nt].at(e);
+                    }
+            }
+            Sum s[2];
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+                const Left a(rest[ks][0], rest[ks][2], rest[ks][1], rest[ks][3]);
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    const float2 b = *reinterpret_cast<const float2*>(&sm.blk[I][at16(nt * 8 + r, ks * 8 + 2 * c2)]);
+                    s[nt].add(a, b.x, b.y);
+                }
+            }
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[2 * I + nt][e] = s[nt].at(e);
+            if (part == 0) {
+                pre[0] *= sm.total[I][c];
+                pre[1] *= sm.total[I][c + 8];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int t = i * 8 + 2 * c2 + (e & 1), col = c + 8 * (e >> 1);
+                if (part == 0) sm.k[t][col] = x[i][e];  // nobody else reads these columns
+                else mine[Unit<D>::U + t * dv + col] = x[i][e];
+            }
+    }
+    __syncthreads();
+    for (int i = warp; i < 4 * KS; i += 8) {
+        const int t = (i / KS) * SUB + r, c = (i % KS) * 8 + 2 * c2;
+        const float2 x = *reinterpret_cast<const float2*>(&sm.k[t][c]), y = *reinterpret_cast<const float2*>(&sm.k[t + 8][c]);
+        reinterpret_cast<float4*>(mine + Unit<D>::W)[i * 32 + lane] = make_float4(x.x, y.x, x.y, y.y);
+    }
+}
+
+template <int D>
+struct WalkSmem {
+    float4 ring[3][8][8][32];                // a warp's pieces of three tiles: a lane reads back what it copied itself
+    float state[2][STRIP][D + 8];            // rounded, rest: rows of value columns, eight banks apart
+    float u[2][STRIP][CHUNK + 8];
+    float4 part[4][32];                      // the second half of the first product's sums
+};
+
+template <int D>
+__global__ void __launch_bounds__(THREADS, 2) channel_walk_kernel(Inputs in, float* __restrict__ work, float* __restrict__ state) {
+    constexpr int HALF = D / 16;  // steps of eight channels that a warp has of the first product
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    WalkSmem<D>& sm = *reinterpret_cast<WalkSmem<D>*>(smem_raw);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.y, seq = blockIdx.z, v0 = blockIdx.x * STRIP, dv = in.dv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c2 = lane & 3;
+    const int t0 = in.cu_q[seq], len = in.cu_q[seq + 1] - t0;
+    const size_t slot = in.slots[seq];
+    if (in.chunk0 == 0 && in.taps > 1 && len > 0) {
+        // the convolution state moves on by the step's inputs: a channel a thread, rows upward, so every row is read before it is written
+        const int rows = in.taps - 1, channels = 2 * in.n_kv * D + in.n_heads * dv;
+        for (int c = (blockIdx.y * gridDim.x + blockIdx.x) * THREADS + threadIdx.x; c < channels; c += gridDim.x * gridDim.y * THREADS) {
+            float* mine = in.conv_state + slot * rows * channels + c;
+            for (int i = 0; i < rows; ++i) {
+                const int at = len - rows + i;
+                mine[(size_t)i * channels] = at >= 0 ? to_float(in.proj[(long long)(t0 + at) * in.ld + c]) : mine[(size_t)(i + len) * channels];
+            }
+        }
+    }
+    const int here = min(in.wave, (len + CHUNK - 1) / CHUNK - in.chunk0);
+    if (here <= 0) return;
+    const size_t step = (size_t)in.n_heads * Unit<D>::SIZE;
+    float* unit = work + ((size_t)seq * in.wave * in.n_heads + head) * Unit<D>::SIZE;
+    const bool owns = warp < D / 16;       // of the state: channels 16 warp + r and + 8, columns 2 c2 and + 1
+    const int mt = warp & 3, kh = warp >> 2;
+    auto issue = [&](int i) {
+        if (i < 2 * here) {
+            const float* u = unit + (i >> 1) * step;
+            if ((i & 1) == 0) {
+                const float4* src = reinterpret_cast<const float4*>(u + Unit<D>::W) + (mt * (D / 8) + kh * HALF) * 32 + lane;
+#pragma unroll
+                for (int ks = 0; ks < HALF; ++ks) cp_async_16(&sm.ring[i % 3][warp][ks][lane], src + ks * 32);
+            } else if (owns) {
+                const float4* src = reinterpret_cast<const float4*>(u + Unit<D>::K) + warp * 8 * 32 + lane;
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks) cp_async_16(&sm.ring[i % 3][warp][ks][lane], src + ks * 32);
+            }
+        }
+        cp_async_commit();
+    };
+    issue(0);
+    issue(1);
+    float* saved = state + (slot * in.n_heads + head) * (size_t)D * dv + v0 + 2 * c2;
+    float S[4] = {0.f, 0.f, 0.f, 0.f};
+    const int ch = warp * 16 + r;
+    if (owns) {
+        const float2 a = *reinterpret_cast<const float2*>(saved + (size_t)ch * dv), b = *reinterpret_cast<const float2*>(saved + (size_t)(ch + 8) * dv);
+        S[0] = a.x, S[1] = a.y, S[2] = b.x, S[3] = b.y;
+    }
+    const int tok = mt * 16 + r;
+    float2 next_u[2] = {};
+    float next_g[2] = {};
+    auto fetch = [&](int i) {  // what the chunk needs beside its tiles
+        if (i >= here) return;
+        const float* u = unit + i * step;
+        if (kh == 0) {
+            next_u[0] = *reinterpret_cast<const float2*>(u + Unit<D>::U + tok * dv + v0 + 2 * c2);
+            next_u[1] = *reinterpret_cast<const float2*>(u + Unit<D>::U + (tok + 8) * dv + v0 + 2 * c2);
+        }
+        if (owns) {
+            next_g[0] = u[Unit<D>::G + ch];
+            next_g[1] = u[Unit<D>::G + ch + 8];
+        }
+    };
+    fetch(0);
+    for (int i = 0; i < here; ++i) {
+        float* mine = unit + i * step;
+        if (owns) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint32_t hi, lo;
+                split(S[e], hi, lo);
+                sm.state[0][2 * c2 + (e & 1)][ch + 8 * (e >> 1)] = __uint_as_float(hi);
+                sm.state[1][2 * c2 + (e & 1)][ch + 8 * (e >> 1)] = __uint_as_float(lo);
+            }
+            *reinterpret_cast<float2*>(mine + Unit<D>::S + ch * dv + v0 + 2 * c2) = make_float2(S[0], S[1]);
+            *reinterpret_cast<float2*>(mine + Unit<D>::S + (ch + 8) * dv + v0 + 2 * c2) = make_float2(S[2], S[3]);
+        }
+        const float2 u0 = next_u[0], u1 = next_u[1];
+        const float g0 = next_g[0], g1 = next_g[1];
+        fetch(i + 1);
+        issue(2 * i + 2);
+        cp_async_wait<2>();
+        __syncthreads();  // the state before the chunk is there
+        {
+            Sum s;
+#pragma unroll
+            for (int ks = 0; ks < HALF; ++ks) {
+                const float4 a = sm.ring[(2 * i) % 3][warp][ks][lane];
+                const int at = (kh * HALF + ks) * 8 + 2 * c2;
+                const uint2 hi = *reinterpret_cast<const uint2*>(&sm.state[0][r][at]), lo = *reinterpret_cast<const uint2*>(&sm.state[1][r][at]);
+                s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
+            }
+            // the two halves meet: 64 threads a barrier
+            if (kh == 1) {
+                sm.part[mt][lane] = make_float4(s.at(0), s.at(1), s.at(2), s.at(3));
+                asm volatile("bar.arrive %0, 64;" ::"r"(1 + mt) : "memory");
+            } else {
+                asm volatile("bar.sync %0, 64;" ::"r"(1 + mt) : "memory");
+                const float4 p = sm.part[mt][lane];
+                const float u[4] = {u0.x - (s.at(0) + p.x), u0.y - (s.at(1) + p.y), u1.x - (s.at(2) + p.z), u1.y - (s.at(3) + p.w)};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    uint32_t hi, lo;
+                    split(u[e], hi, lo);
+                    sm.u[0][2 * c2 + (e & 1)][tok + 8 * (e >> 1)] = __uint_as_float(hi);
+                    sm.u[1][2 * c2 + (e & 1)][tok + 8 * (e >> 1)] = __uint_as_float(lo);
+                }
+                *reinterpret_cast<float2*>(mine + Unit<D>::U + tok * dv + v0 + 2 * c2) = make_float2(u[0], u[1]);
+                *reinterpret_cast<float2*>(mine + Unit<D>::U + (tok + 8) * dv + v0 + 2 * c2) = make_float2(u[2], u[3]);
+            }
+        }
+        issue(2 * i + 3);
+        cp_async_wait<2>();
+        __syncthreads();  // u is there, and nobody reads the state before the chunk any more
+        if (owns) {
+            Sum s;
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks) {
+                const float4 a = sm.ring[(2 * i + 1) % 3][warp][ks][lane];
+                const uint2 hi = *reinterpret_cast<const uint2*>(&sm.u[0][r][ks * 8 + 2 * c2]), lo = *reinterpret_cast<const uint2*>(&sm.u[1][r][ks * 8 + 2 * c2]);
+                s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
+            }
+            S[0] = fmaf(S[0], g0, s.at(0));
+            S[1] = fmaf(S[1], g0, s.at(1));
+            S[2] = fmaf(S[2], g1, s.at(2));
+            S[3] = fmaf(S[3], g1, s.at(3));
+        }
+    }
+    cp_async_wait<0>();
+    if (owns) {
+        *reinterpret_cast<float2*>(saved + (size_t)ch * dv) = make_float2(S[0], S[1]);
+        *reinterpret_cast<float2*>(saved + (size_t)(ch + 8) * dv) = make_float2(S[2], S[3]);
+    }
+}
+
+template <int D>
+struct ReadSmem {
+    static constexpr int LD = 132;  // two rows are eight banks apart
+    float state[D][LD], u[CHUNK][LD];
+    float squares[2][CHUNK];
+};
+
+template <int D>
+__global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, const float* __restrict__ work, bf16* __restrict__ out, float eps) {
+    constexpr int LD = ReadSmem<D>::LD;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    ReadSmem<D>& sm = *reinterpret_cast<ReadSmem<D>*>(smem_raw);
+    pdl_launch_dependents();
+    pdl_wait();
+    const int head = blockIdx.y, seq = blockIdx.z, dv = in.dv;
+    const int t0 = in.cu_q[seq], len = in.cu_q[seq + 1] - t0;
+    const int first = (in.chunk0 + blockIdx.x) * CHUNK;
+    if (first >= len) return;
+    const int n = min(CHUNK, len - first), tok0 = t0 + first;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c2 = lane & 3, mt = warp & 3, nh = warp >> 2;
+    const float* mine = work + (((size_t)seq * in.wave + blockIdx.x) * in.n_heads + head) * Unit<D>::SIZE;
+    const int pieces = dv / 4;
+    for (int i = threadIdx.x; i < D * pieces; i += THREADS) cp_async_16(&sm.state[i / pieces][(i % pieces) * 4], mine + Unit<D>::S + i * 4);
+    for (int i = threadIdx.x; i < CHUNK * pieces; i += THREADS) cp_async_16(&sm.u[i / pieces][(i % pieces) * 4], mine + Unit<D>::U + i * 4);
+    cp_async_commit();
+    const int tiles = dv / 16, v0 = nh * (dv / 2);
+    Sum s[8];
+    cp_async_wait<0>();
+    __syncthreads();
+    auto product = [&](const float4* left, int steps, const float(*right)[LD]) {
+        float4 ahead[4];  // from L2, four steps ahead
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ahead[i] = i < steps ? left[i * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int k4 = 0; k4 < steps; k4 += 4)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int ks = k4 + i;
+                if (ks >= steps) break;
+                const Left a(ahead[i].x, ahead[i].y, ahead[i].z, ahead[i].w);
+                if (ks + 4 < steps) ahead[i] = left[(ks + 4) * 32 + lane];
+                const float *b0 = &right[ks * 8 + 2 * c2][v0 + r], *b1 = b0 + LD;
+#pragma unroll
+                for (int nt = 0; nt < 8; ++nt)
+                    if (nt < tiles) s[nt].add(a, b0[nt * 8], b1[nt * 8]);
+            }
+    };
+    product(reinterpret_cast<const float4*>(mine + Unit<D>::Q) + mt * (D / 8) * 32, D / 8, sm.state);
+    product(reinterpret_cast<const float4*>(mine + Unit<D>::P) + mt * 8 * 32, 2 * (mt + 1), sm.u);
+    float ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            s[nt].acc[e] = nt < tiles ? s[nt].at(e) : 0.f;
+            ss[e >> 1] = fmaf(s[nt].acc[e], s[nt].acc[e], ss[e >> 1]);
+        }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 1);
+        ss[h] += __shfl_xor_sync(0xffffffffu, ss[h], 2);
+        if (c2 == 0) sm.squares[nh][mt * 16 + r + 8 * h] = ss[h];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int t = mt * 16 + r + 8 * h;
+        if (t >= n) continue;
+        const float unit = 1.f / sqrtf((sm.squares[0][t] + sm.squares[1][t]) / (float)dv + eps);
+        const float* gate = in.low + (long long)(tok0 + t) * in.ld_low + (long long)in.n_heads * D + head * dv + v0 + 2 * c2;
+        bf16* to = out + ((size_t)(tok0 + t) * in.n_heads + head) * dv + v0 + 2 * c2;
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+            if (nt >= tiles) continue;
+            const float2 z = *reinterpret_cast<const float2*>(gate + nt * 8), w = *reinterpret_cast<const float2*>(in.norm + v0 + nt * 8 + 2 * c2);
+            const float x = s[nt].acc[2 * h] * unit * w.x * sigmoid_f(z.x), y = s[nt].acc[2 * h + 1] * unit * w.y * sigmoid_f(z.y);
+            *reinterpret_cast<__nv_bfloat162*>(to + nt * 8) = __floats2bfloat162_rn(x, y);
+        }
+    }
+}
+
+}  // namespace
+
+static bool channel_fits(int d, int dv, int taps) { return (d == 64 || d == 128) && dv > 0 && dv % 16 == 0 && dv <= d && taps >= 1 && taps <= MAX_TAPS; }
+GK_EXPORT int gk_delta_channel_fits(int d, int dv, int taps) { return channel_fits(d, dv, taps); }
+// 32-bit numbers of workspace per sequence, chunk of a wave and head
+GK_EXPORT int gk_delta_channel_work(int d) { return d == 64 ? Unit<64>::SIZE : Unit<128>::SIZE; }
+
+// proj [T, ld] bfloat16: q (G d) | k (G d) | v (H dv) | b (H) | ..; low [T, ld_low] 32-bit: a (H d) | gate (H dv); out [T, H dv] bfloat16;
+// state [slots, H, d, dv] and conv_state [slots, taps - 1, channels] are moved on by the step's tokens.  max_len bounds the sequences'
+// token counts; `wave` chunks of every sequence are in flight at a time.
+GK_EXPORT int gk_delta_channel(const void* proj, long long ld, const float* low, long long ld_low, const float* conv_w, float* conv_state,
+                               const float* a_log, const float* dt_bias, const float* norm, float eps, float* state, float* work, void* out,
+                               const int* cu_q, const int* slots, int n_seqs, int n_heads, int n_kv, int d, int dv, int taps, int max_len,
+                               int wave, void* stream) {
+    GK_REQUIRE(n_heads > 0 && n_heads <= 65535 && n_kv > 0 && n_heads % n_kv == 0 && n_seqs >= 0 && n_seqs <= 65535, "delta_channel: bad counts");
+    GK_REQUIRE(channel_fits(d, dv, taps), "delta_channel: heads of %d / %d with %d taps do not fit", d, dv, taps);
+    GK_REQUIRE(taps == 1 || conv_state != nullptr, "delta_channel: a convolution of several taps needs its state");
+    GK_REQUIRE(max_len >= 0 && wave > 0 && work != nullptr, "delta_channel: bad sizes");
+    GK_REQUIRE(ld % 8 == 0 && ld_low % 4 == 0, "delta_channel: rows must start on 16 bytes");
+    GK_REQUIRE((((uintptr_t)proj | (uintptr_t)low | (uintptr_t)work | (uintptr_t)state | (uintptr_t)conv_state | (uintptr_t)dt_bias | (uintptr_t)norm |
+                 (uintptr_t)out) & 15) == 0, "delta_channel: tensors must start on 16 bytes");
+    if (n_seqs == 0 || max_len == 0) return GK_OK;
+    static bool prepared = false;
+    if (!prepared) {
+#define GK_ATTR(KERNEL, BYTES)                                                                                  \
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)) != cudaSuccess) \
+        return gk_fail(GK_CUDA_ERROR, "delta_channel: shared memory")
+        GK_ATTR(channel_inner_kernel<64>, sizeof(InnerSmem<64>));
+        GK_ATTR(channel_inner_kernel<128>, sizeof(InnerSmem<128>));
+        GK_ATTR(channel_walk_kernel<64>, sizeof(WalkSmem<64>));
+        GK_ATTR(channel_walk_kernel<128>, sizeof(WalkSmem<128>));
+        GK_ATTR(channel_read_kernel<64>, sizeof(ReadSmem<64>));
+        GK_ATTR(channel_read_kernel<128>, sizeof(ReadSmem<128>));
+#undef GK_ATTR
+        prepared = true;
+    }
+    cudaStream_t s = (cudaStream_t)stream;
+    const int chunks = (max_len + CHUNK - 1) / CHUNK;
+    for (int chunk0 = 0; chunk0 < chunks; chunk0 += wave) {
+        const int here = chunks - chunk0 < wave ? chunks - chunk0 : wave;
+        const Inputs in{(const bf16*)proj, low, conv_w, conv_state, a_log, dt_bias, norm, cu_q, slots, ld, ld_low, n_heads, n_kv, dv, taps, chunk0, wave};
+#define GK_CHANNEL(D)                                                                                                                  \
+    gk_launch(channel_inner_kernel<D>, dim3(here, n_heads, n_seqs), dim3(THREADS), sizeof(InnerSmem<D>), s, in, work);                 \
+    gk_launch_behind(channel_walk_kernel<D>, dim3(dv / STRIP, n_heads, n_seqs), dim3(THREADS), sizeof(WalkSmem<D>), s, in, work, state);      \
+    gk_launch_behind(channel_read_kernel<D>, dim3(here, n_heads, n_seqs), dim3(THREADS), sizeof(ReadSmem<D>), s, in, (const float*)work, (bf16*)out, eps)
+        if (d == 64) {
+            GK_CHANNEL(64);
+        } else {
+            GK_CHANNEL(128);
+        }
+#undef GK_CHANNEL
+    }
+    GK_CHECK_LAUNCH("delta_channel");
+    return GK_OK;
+}

@@ -1343,6 +1343,59 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
     return out
 
 
+# The longest run of a step from which on the chunks are the faster way: their three kernels take 73 us for one chunk and some two more
+# a chunk, the kernels that go token by token 0.3 us a token behind 13 (8 heads of 128, one prompt: 33 tokens: 75 / 23 us, 2,048: 189 / 620).
+DELTA_CHANNEL_MIN_TOKENS = 256
+
+
+def delta_channel_ok(proj: torch.Tensor, low: torch.Tensor, dt_bias: torch.Tensor, norm_w: torch.Tensor, conv_state: torch.Tensor | None,
+                     state: torch.Tensor, d: int, dv: int, taps: int) -> bool:
+    """Whether :func:`delta_channel` takes these operands: bfloat16 projections, heads of 64 or 128 with values no wider, at most
+    four taps, rows and tensors that start on 16 bytes."""
+    if proj.dtype != torch.bfloat16 or low.dtype != torch.float32 or proj.shape[1] % 8 or low.shape[1] % 4:
+        return False
+    tensors = (proj, low, dt_bias, norm_w, state) + (() if conv_state is None else (conv_state,))
+    return all(t.data_ptr() % 16 == 0 for t in tensors) and bool(library().gk_delta_channel_fits(d, dv, taps))
+
+
+def delta_channel(proj: torch.Tensor, low: torch.Tensor, conv_w: torch.Tensor, conv_state: torch.Tensor | None, a_log: torch.Tensor,
+                  dt_bias: torch.Tensor, norm_w: torch.Tensor, eps: float, state: torch.Tensor, cu_q: torch.Tensor, slots: torch.Tensor,
+                  n_seqs: int, max_q_len: int, n_heads: int, n_kv: int, d: int, dv: int, taps: int) -> torch.Tensor:
+    """What :func:`delta_prepare`, :func:`conv_roll`, :func:`delta_scan` and :func:`head_norm_gate` (gate behind the decays in ``low``)
+    do in turn, in chunks of 64 tokens on the tensor cores with 32-bit operands (each number as two TF32 numbers); ``max_q_len``
+    bounds the sequences' token counts in this step.  Returns the gated read-outs ``[T, n_heads dv]`` (bfloat16)."""
+    require_device(proj.device)
+    _check(proj, "proj", torch.bfloat16, 2)
+    _check(low, "low", torch.float32, 2)
+    T, channels = proj.shape[0], 2 * n_kv * d + n_heads * dv
+    if proj.shape[1] < channels + n_heads or low.shape[1] < n_heads * (d + dv) or low.shape[0] != T:
+        raise KernelError(f"projections {tuple(proj.shape)} / {tuple(low.shape)} are too narrow for these sizes")
+    _check(conv_w, "conv_w", torch.float32, 2)
+    _check(state, "state", torch.float32, 4)
+    if tuple(conv_w.shape) != (channels, taps) or tuple(state.shape[1:]) != (n_heads, d, dv):
+        raise KernelError(f"conv_w {tuple(conv_w.shape)} or the state {tuple(state.shape)} have other sizes than the heads")
+    if taps > 1:
+        _check(conv_state, "conv_state", torch.float32, 3)
+        if tuple(conv_state.shape[1:]) != (taps - 1, channels):
+            raise KernelError(f"conv_state is {tuple(conv_state.shape)}, expected [slots, {taps - 1}, {channels}]")
+    for name, t, size in (("a_log", a_log, n_heads), ("dt_bias", dt_bias, n_heads * d), ("norm_w", norm_w, dv)):
+        _check(t, name, torch.float32, 1)
+        if t.shape[0] != size:
+            raise KernelError(f"{name} has {t.shape[0]} entries, expected {size}")
+    for name, t in (("cu_q", cu_q), ("slots", slots)):
+        _check(t, name, torch.int32, 1)
+    dev = proj.device
+    unit = library().gk_delta_channel_work(d)
+    chunks = max(1, -(-int(max_q_len) // DELTA_CHUNK))
+    wave = max(1, min(chunks, DELTA_WORKSPACE_BYTES // max(1, 4 * unit * n_seqs * n_heads)))
+    work = torch.empty((max(1, n_seqs) * wave * n_heads * unit,), dtype=torch.float32, device=dev)
+    out = torch.empty((T, n_heads * dv), dtype=torch.bfloat16, device=dev)
+    call("gk_delta_channel", ptr(proj), proj.shape[1], ptr(low), low.shape[1], ptr(conv_w), ptr(conv_state) if taps > 1 else None, ptr(a_log),
+         ptr(dt_bias), ptr(norm_w), float(eps), ptr(state), ptr(work), ptr(out), ptr(cu_q), ptr(slots), int(n_seqs), n_heads, n_kv, d, dv,
+         taps, int(max_q_len), wave, stream_ptr())
+    return out
+
+
 def head_norm_gate(o: torch.Tensor, weight: torch.Tensor, gate: torch.Tensor, gate_at: int, eps: float, out_dtype: torch.dtype) -> torch.Tensor:
     """``o [T, H, dv]`` (32-bit) divided by each head's root mean square, times ``weight [dv]``, times the sigmoid of
     ``gate[:, gate_at : gate_at + H dv]``.  Returns ``[T, H dv]`` in ``out_dtype``."""
