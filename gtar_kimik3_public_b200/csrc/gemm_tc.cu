@@ -22,9 +22,8 @@
 // *error_flag and leaves its loop; the block still drains its own copies, frees its tensor memory
 // and returns.
 
-#include <cuda.h>
 
-#include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
@@ -1044,35 +1043,9 @@ __global__ void __launch_bounds__(PERSISTENT_THREADS, 1) gemm_tc_pair_kernel(con
 }
 
 // ---------------------------------------------------------------- host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult result;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &result) == cudaSuccess &&
-            result == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(ptr);
-    }
-    return fn;
-}
-
 // A K-major matrix [rows, k] of bfloat16 with `ld` elements between rows; boxes of box_rows x 64.
 int make_map(CUtensorMap* map, const void* base, int rows, int k, long long ld, int box_rows) {
-    EncodeTiledFn fn = encode_tiled();
-    if (!fn) return gk_fail(GK_CUDA_ERROR, "gemm_tc: the driver does not offer cuTensorMapEncodeTiled");
-    cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(__nv_bfloat16)};
-    cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-    cuuint32_t elem[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return gk_fail(GK_CUDA_ERROR, "gemm_tc: cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return GK_OK;
+    return gk_matrix_map(map, base, rows, k, ld, BK, box_rows, true);
 }
 
 template <int BN, int STAGES>

@@ -27,11 +27,23 @@
 #include <algorithm>
 #include <cmath>
 
-#include "common.cuh"
+#include "tensor_map.cuh"
 
 namespace {
 
 constexpr int ROUTE_WARPS = 4;
+
+__device__ __forceinline__ void score_copy16(void* smem, const void* gmem, bool in) {  // zeros where `in` is false
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(in ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 
 // Loads of several elements want their address on as many bytes: a row length that is a multiple of them says so only where the
@@ -110,14 +122,55 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_scores_kernel(const T*
         }
 }
 
+// The same where tokens are few: a block has eight tokens and two rows of the router, all of which it asks for at once (the kernel
+// above goes back to memory for every fourth of a row, on a handful of SMs), a warp four tokens and one row.  Rows of a multiple
+// of eight entries; the sums are those of the kernel above bit for bit.  Bound by its launch and one trip to memory.
+// Measured (us, scores and choice, cold, 1 to 128 tokens; the kernel above / here): 64 experts of 2,048: 23.6 / 13.3, 32 of 1,024: 17.4 /
+// 11.3, 16 of 4,096: 32 / 11.3; 8 of 256: 11.3 / 9.2.
+constexpr int FEW_TOKENS = 8, FEW_EXPERTS = 2;
+template <typename T>
+__global__ void __launch_bounds__(128) route_scores_few_kernel(const T* __restrict__ h, const float* __restrict__ w_router, float* __restrict__ z,
+                                                               int n_tokens, int width, int n_experts) {
+    extern __shared__ __align__(16) unsigned char few_smem[];  // router rows [FEW_EXPERTS][width], tokens [FEW_TOKENS][width]
+    float* ws = reinterpret_cast<float*>(few_smem);
+    T* xs = reinterpret_cast<T*>(ws + FEW_EXPERTS * width);
+    pdl_launch_dependents();
+    const int e0 = blockIdx.x * FEW_EXPERTS, t0 = blockIdx.y * FEW_TOKENS, tokens = min(FEW_TOKENS, n_tokens - t0), rows = min(FEW_EXPERTS, n_experts - e0);
+    for (int i = threadIdx.x * 4; i < rows * width; i += 128 * 4) cp_async_16(ws + i, w_router + (size_t)e0 * width + i);  // no kernel in flight writes them
+    pdl_wait();
+    constexpr int PIECE = 16 / sizeof(T);
+    for (int i = threadIdx.x * PIECE; i < tokens * width; i += 128 * PIECE) cp_async_16(xs + i, h + (size_t)t0 * width + i);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = warp & 1, first = (warp >> 1) * 4;
+    if (row >= rows || first >= tokens) return;
+    const float* w = ws + row * width;
+    const T* x = xs + first * width;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int i = lane * 4; i < width; i += 128) {
+        float wv[4], xv[4][4];
+        load_four(w + i, true, wv);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) load_four(x + a * width + i, first + a < tokens, xv[a]);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[a] = fmaf(xv[a][e], wv[e], acc[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const float sum = warp_sum(acc[a]);
+        if (lane == 0 && first + a < tokens) z[(size_t)(t0 + first + a) * n_experts + e0 + row] = sum;
+    }
+}
+
 // The same for many bfloat16 tokens: a block has 16 tokens and 16 NJ rows of the router, the reduction in pieces of 64 entries
 // that come through a two-stage cp.async ring.  Its threads are four groups of 64 that take a quarter of every piece each, a
 // thread 4 tokens x NJ rows; the groups' sums meet at the end in their order.  A score depends on the token's row alone.
 constexpr int SCORE_K = 64, SCORE_ROWS = 16, SCORE_LDW = SCORE_K + 4, SCORE_LDH = SCORE_K + 8;
 
-__device__ __forceinline__ void score_copy16(void* smem, const void* gmem, bool in) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem), "r"(in ? 16 : 0) : "memory");
-}
 
 template <int NJ>
 __global__ void __launch_bounds__(256) route_scores_tiled_kernel(const __nv_bfloat16* __restrict__ h, const float* __restrict__ w_router,
@@ -243,6 +296,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_choose_kernel(
     if (n_groups > 1 && keep < n_groups) {
         for (int gidx = lane; gidx < n_groups; gidx += 32) {
             float first = -INFINITY, second = -INFINITY;
+#pragma unroll 8
             for (int e = gidx * per; e < (gidx + 1) * per; ++e) {
                 const float c = choice[e];
                 if (c > first) { second = first; first = c; }
@@ -254,6 +308,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_choose_kernel(
         // the groups that are not among the best `keep` lose their experts
         for (int gidx = lane; gidx < n_groups; gidx += 32) {
             int better = 0;
+#pragma unroll 8
             for (int o = 0; o < n_groups; ++o)
                 better += (group_score[o] > group_score[gidx]) || (group_score[o] == group_score[gidx] && o < gidx);
             if (better >= keep)
@@ -261,27 +316,33 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) route_choose_kernel(
         }
         __syncwarp();
     }
-    for (int pick = 0; pick < top; ++pick) {
-        float best = -INFINITY;
-        int arg = 0x7fffffff;
+    // A lane keeps the best of its own experts, as a number that orders like the score (zero: none left); two reductions of the warp
+    // find the largest and, where several are equal, the lowest expert.
+    unsigned int best = 0;
+    int arg = 0x7fffffff;
+    const auto own_best = [&]() {
+        best = 0, arg = 0x7fffffff;
         for (int e = lane; e < n_experts; e += 32) {
-            const float c = choice[e];
-            if (c > best) { best = c; arg = e; }
+            const float c = choice[e] + 0.f;  // one zero
+            const unsigned int bits = __float_as_uint(c), key = c > -INFINITY ? (bits & 0x80000000u ? ~bits : bits | 0x80000000u) : 0u;
+            if (key > best) best = key, arg = e;
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
-            if (ob > best || (ob == best && oa < arg)) { best = ob; arg = oa; }
-        }
-        if (arg == 0x7fffffff) arg = 0;  // nothing left to choose from: cannot happen when top <= allowed experts
+    };
+    own_best();
+    for (int pick = 0; pick < top; ++pick) {
+        const unsigned int most = __reduce_max_sync(0xffffffffu, best);
+        int chosen = (int)__reduce_min_sync(0xffffffffu, best == most ? (unsigned int)arg : 0x7fffffffu);
+        if (chosen == 0x7fffffff) chosen = 0;  // nothing left to choose from: cannot happen when top <= allowed experts
         if (lane == 0) {
-            ids[(size_t)t * ld_pairs + pick] = arg;
-            weights[(size_t)t * ld_pairs + pick] = logits || (flags & ROUTE_RENORMALISE) ? s[arg] : s[arg] * scale;
-            choice[arg] = -INFINITY;
+            ids[(size_t)t * ld_pairs + pick] = chosen;
+            weights[(size_t)t * ld_pairs + pick] = logits || (flags & ROUTE_RENORMALISE) ? s[chosen] : s[chosen] * scale;
         }
-        __syncwarp();
+        if (lane == (chosen & 31)) {
+            choice[chosen] = -INFINITY;
+            own_best();
+        }
     }
+    __syncwarp();
     if ((flags & ROUTE_RENORMALISE) && lane == 0) {
         float* w = weights + (size_t)t * ld_pairs;
         float sum = 0.f;
@@ -619,14 +680,18 @@ __global__ void __launch_bounds__(UP_WARPS * 32) token_down_kernel(const T* __re
 // at once (16 bytes) and they serve as its fragments of two products; the tokens' rows lie in shared memory and are read the
 // same way.  What remains is the stream of the weights, an expert's rows once for sixteen of its tokens (for eight where rows are longer
 // than some 1,500 entries: two blocks an SM would not hold sixteen) and for every list of 512 pairs.  Blocks stay
-// and take equal runs of (expert, sixteen rows) units: the experts that were chosen are listed by every block for itself, and a
-// warp asks for its first rows of the next unit before it adds up this one's.  (One block a pair and chunk of rows, most of
-// which found that another had their expert, spent their time in the chain ids - list - weights - tokens: 60 us where the
-// weights take 21.)  (Tensor-memory products would want 128 rows a tile and the weights through shared memory, for a
-// step that does next to no arithmetic.)
-// Measured (us; up, down and join; 6 of 64 experts of 2,048 x 1,024), every pair by itself on the FP32 pipes and here: 4 tokens 93 / 88,
-// 8: 170 / 121 (experts drawn at random), 16: 319 / 173, 42: 763 / 248; 4 of 32 experts of 1,024 x 768: 8 tokens 43 / 38, 63: 265 / 66.
-constexpr int MMA_WARPS = 4, MMA_STEPS = 2, MMA_TOKENS = 16, MMA_LIST = 512;
+// and take equal runs of (expert, sixteen rows) units: the experts that were chosen are listed by every block for itself.  (One block a pair
+// and chunk of rows, most of which found that another had their expert, spent their time in the chain ids - list - weights - tokens.)
+//
+// The weights come by TMA, boxes of sixteen rows x 64 entries into a ring of every warp's own that runs on across the ends of units, 48 KB
+// of them a block and two blocks an SM.  (Loads into registers had four pieces in flight that ended with every unit, and went through
+// the load unit 64 bytes of a row at a time: 400 cycles a piece and warp, which also held for copies of 16 bytes into a ring.)
+// (Tensor-memory products would want 128 rows a tile, for a step that does next to no arithmetic.)
+// Measured (us, cold; up, down and join; loads into registers / here): 6 of 64 experts of 2,048 x 1,024: 4 tokens 91 / 65, 8: 95 / 77,
+// 16: 114 / 81, 42: 175 / 142; 4 of 32 of 1,024 x 768: 8 tokens 46 / 34, 63: 69 / 65; 2 of 8 of 6,144 x 512: 16 tokens 108 / 81.
+// Every pair by itself on the FP32 pipes: 8 tokens 170 and 43, 42 and 63 tokens 763 and 265.  Bound by the weights (4.6 TB/s of them in
+// the up product of 8 tokens) with 6 us of launch and list before the first of them.
+constexpr int MMA_WARPS = 4, MMA_TOKENS = 16, MMA_LIST = 512;
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
@@ -637,78 +702,74 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1
 // together (two rows, four pieces) fall into different banks
 __host__ __device__ constexpr int mma_stride(int k) { return (k * 2 + 127) / 128 * 128 + 64; }
 
-// MMA_STEPS pieces of 32 entries of a lane's two rows (`k` entries a row, eight rows apart) of each matrix
-template <int NM>
-struct MmaBatch {
-    uint4 lo[MMA_STEPS][NM], hi[MMA_STEPS][NM];
-    __device__ __forceinline__ void load(const __nv_bfloat16* const (&row0)[NM], int k, int i, int end) {
-#pragma unroll
-        for (int u = 0; u < MMA_STEPS; ++u)
-            if (i + u < end) {
-#pragma unroll
-                for (int m = 0; m < NM; ++m) {
-                    const __nv_bfloat16* at = row0[m] + (i + u) * 32;
-                    lo[u][m] = *reinterpret_cast<const uint4*>(at);
-                    hi[u][m] = *reinterpret_cast<const uint4*>(at + (size_t)8 * k);
-                }
-            }
-    }
-    template <int NB>
-    __device__ __forceinline__ void multiply(const unsigned char* x_at, int stride, int i, int end, float (&sums)[NM][NB][4]) const {
-#pragma unroll
-        for (int u = 0; u < MMA_STEPS; ++u)
-            if (i + u < end) {
-#pragma unroll
-                for (int b = 0; b < NB; ++b) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(x_at + b * 8 * stride + (i + u) * 64);
-#pragma unroll
-                    for (int m = 0; m < NM; ++m) {
-                        mma_bf16(sums[m][b], lo[u][m].x, hi[u][m].x, lo[u][m].y, hi[u][m].y, x.x, x.y);
-                        mma_bf16(sums[m][b], lo[u][m].z, hi[u][m].z, lo[u][m].w, hi[u][m].w, x.z, x.w);
-                    }
-                }
-            }
-    }
-};
-
 // rows of `source` (`divide` pairs share one) for pairs[0 .. count - 1] into shared memory; what stands in the rows behind them
 // is multiplied into columns that nobody reads
 __device__ __forceinline__ void mma_stage(unsigned char* xs, int stride, const __nv_bfloat16* __restrict__ source, const int* pairs, int count, int divide, int k) {
     const int pieces = k / 8;
+#pragma unroll 8
     for (int i = threadIdx.x; i < count * pieces; i += MMA_WARPS * 32) {
         const int t = i / pieces, c = i - t * pieces;
         *reinterpret_cast<uint4*>(xs + t * stride + c * 16) = *reinterpret_cast<const uint4*>(source + (size_t)(pairs[t] / divide) * k + c * 8);
     }
 }
 
-// Sixteen rows of NM matrices times the staged tokens, this warp's quarter: part[(m NB + b) 4 + e][lane].  `first`: the batch that
-// this warp has already asked for.
-template <int NM, int NB>
-__device__ __forceinline__ void mma_tile(MmaBatch<NM>& first, const __nv_bfloat16* const (&row0)[NM], int k, int begin, int end, const unsigned char* xs, int stride,
-                                         float (*part)[32]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
-    const unsigned char* x_at = xs + g * stride + q * 16;
-    float sums[NM][NB][4];
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) sums[m][b][e] = 0.f;
-    for (int i = begin; i < end; i += 2 * MMA_STEPS) {
-        MmaBatch<NM> second;
-        second.load(row0, k, i + MMA_STEPS, end);
-        first.template multiply<NB>(x_at, stride, i, end, sums);
-        first.load(row0, k, i + 2 * MMA_STEPS, end);
-        second.template multiply<NB>(x_at, stride, i + MMA_STEPS, end, sums);
+// ---- TMA: a warp's boxes of sixteen rows, each waited for on a barrier of its own; waits are bounded
+constexpr uint32_t EXPERT_SPINS = 1u << 24;
+
+__device__ __forceinline__ uint32_t smem_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool box_wait(uint64_t* bar, uint32_t parity) {
+    for (uint32_t i = 0; i < EXPERT_SPINS; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(smem_address(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
     }
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-#pragma unroll
-        for (int b = 0; b < NB; ++b)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) part[(m * NB + b) * 4 + e][lane] = sums[m][b][e];
+    return false;
 }
+
+// A warp's boxes of 16 rows x `box_k` entries (64, or 32 where rows have no more) of NM matrices, DEPTH of them ahead of the products
+// and across the ends of units.
+template <int NM, int DEPTH>
+struct BoxRing {
+    static constexpr int SLOT = NM * 16 * 128;  // bytes
+    unsigned char* slots;
+    uint64_t* full;
+    int asked = 0, taken = 0, put = 0, take = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    // one lane asks; the whole warp has read what stood in the place before
+    __device__ __forceinline__ void ask(const CUtensorMap* map, int k, int row, int rows_apart, int box_k, bool elected) {
+        if (elected) {
+            const uint32_t bar = smem_address(full + put);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(NM * 16 * box_k * 2) : "memory");
+#pragma unroll
+            for (int m = 0; m < NM; ++m)
+                asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                                 smem_address(slots + put * SLOT + m * 16 * 128)),
+                             "l"(reinterpret_cast<uint64_t>(map)), "r"(k), "r"(row + m * rows_apart), "r"(bar)
+                             : "memory");
+        }
+        ++asked;
+        put = put + 1 == DEPTH ? 0 : put + 1;
+    }
+    __device__ __forceinline__ const unsigned char* next() {
+        if (ok) ok = box_wait(full + take, phase);
+        return slots + take * SLOT;
+    }
+    __device__ __forceinline__ void done() {
+        ++taken;
+        take = take + 1 == DEPTH ? 0 : take + 1;
+        if (take == 0) phase ^= 1;
+    }
+    __device__ __forceinline__ void drain() {  // nothing may land in shared memory after the block is gone
+        for (; taken < asked; done()) box_wait(full + take, phase);
+    }
+};
 
 // the sum of one entry over the warps
 template <int N>
@@ -791,62 +852,117 @@ __device__ __forceinline__ int mma_list(const int* __restrict__ ids, int first, 
     return *n_runs;
 }
 
-// UP: gate and up rows, act[pair] = silu(gate) * up; else rows of w_down, parts[pair].  k entries a row, n_rows rows a matrix.
-template <bool UP>
-__global__ void __launch_bounds__(MMA_WARPS * 32, UP ? 3 : 4) experts_mma_kernel(
-    const __nv_bfloat16* __restrict__ source, const __nv_bfloat16* __restrict__ weights, const int* __restrict__ ids, __nv_bfloat16* __restrict__ act,
-    float* __restrict__ parts, int n_pairs, int k, int n_rows, int divide, int n_experts, int at_once) {
+// UP: gate and up rows, act[pair] = silu(gate) * up; else rows of w_down, parts[pair].  k entries a row, n_rows rows a matrix; `map`: all
+// experts' rows one after another.
+template <bool UP, int DEPTH>
+__global__ void __launch_bounds__(MMA_WARPS * 32) experts_mma_kernel(
+    const __grid_constant__ CUtensorMap map, const __nv_bfloat16* __restrict__ source, const int* __restrict__ ids, __nv_bfloat16* __restrict__ act,
+    float* __restrict__ parts, int n_pairs, int k, int n_rows, int divide, int n_experts, int at_once, int staged_bytes, int box_k, int* error_flag) {
     constexpr int NM = UP ? 2 : 1, ENTRIES = NM * MMA_TOKENS / 8 * 4;
-    extern __shared__ __align__(16) unsigned char expert_smem[];  // the tokens' rows [at_once][stride]; before that, counts
+    extern __shared__ __align__(128) unsigned char ring_smem[];  // the rings [MMA_WARPS][DEPTH]; the tokens' rows [at_once][stride], before that counts
     __shared__ int list[MMA_LIST], n_runs;
     __shared__ MmaRun runs[MMA_LIST];
     __shared__ float part[MMA_WARPS][ENTRIES][32];
+    __shared__ __align__(8) uint64_t full[MMA_WARPS][DEPTH];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    if (threadIdx.x < MMA_WARPS * DEPTH) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_address(&full[0][0] + threadIdx.x)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     pdl_launch_dependents();
     pdl_wait();
+    unsigned char* staged_rows = ring_smem + MMA_WARPS * DEPTH * BoxRing<NM, DEPTH>::SLOT;
     const int first_pair = blockIdx.z * MMA_LIST, last_pair = min(first_pair + MMA_LIST, n_pairs);
     const int tiles = n_rows / 16;
-    const long long units = (long long)mma_list(ids, first_pair, last_pair, n_experts, at_once, (int*)expert_smem, list, runs, &n_runs) * tiles;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
-    const int stride = mma_stride(k), pieces = k / 32, share = (pieces + MMA_WARPS - 1) / MMA_WARPS;
+    // (a barrier of the block stands in here)
+    const long long units = (long long)mma_list(ids, first_pair, last_pair, n_experts, at_once, (int*)staged_rows, list, runs, &n_runs) * tiles;
+    const int stride = mma_stride(k), pieces = k / 32, share = (pieces + MMA_WARPS - 1) / MMA_WARPS, per = box_k / 32, pitch = box_k * 2;
     const int begin = min(warp * share, pieces), end = min(begin + share, pieces);
     int unit = (int)(units * blockIdx.x / gridDim.x);
     const int unit_end = (int)(units * (blockIdx.x + 1) / gridDim.x);
-    const __nv_bfloat16* rows[NM];
-    const auto point = [&](int u) {
-        const __nv_bfloat16* at = weights + (size_t)runs[u / tiles].expert * NM * n_rows * k + (size_t)((u % tiles) * 16 + g) * k + q * 8;
-#pragma unroll
-        for (int m = 0; m < NM; ++m) rows[m] = at + (size_t)m * n_rows * k;
+    BoxRing<NM, DEPTH> ring{ring_smem + warp * DEPTH * BoxRing<NM, DEPTH>::SLOT, full[warp]};
+    int ahead = begin < end ? unit : unit_end, piece = begin, row = 0;  // what is asked for next
+    const auto point = [&]() {
+        if (ahead < unit_end) row = runs[ahead / tiles].expert * NM * n_rows + (ahead % tiles) * 16;
     };
-    MmaBatch<NM> first;
-    if (unit < unit_end) {
-        point(unit);
-        first.load(rows, k, begin, end);
-    }
+    const auto ask = [&]() {
+        if (ahead >= unit_end) return;
+        ring.ask(&map, piece * 32, row, n_rows, box_k, lane == 0);
+        piece += per;
+        if (piece >= end) {
+            piece = begin;
+            ++ahead;
+            point();
+        }
+    };
+    point();
+    for (int i = 0; i < DEPTH; ++i) ask();
     for (int staged = -1; unit < unit_end; ++unit) {
         const int at = unit / tiles, tile = unit % tiles, count = runs[at].count, NB = count <= 8 ? 1 : 2;
         const int* pairs = list + runs[at].start;
         if (at != staged) {  // all warps are through with the rows of before: they stand behind the barrier after their sums
-            mma_stage(expert_smem, stride, source, pairs, count, divide, k);
+            mma_stage(staged_rows, stride, source, pairs, count, divide, k);
             staged = at;
         }
         __syncthreads();
-        if (NB == 1) mma_tile<NM, 1>(first, rows, k, begin, end, expert_smem, stride, part[warp]);
-        else mma_tile<NM, 2>(first, rows, k, begin, end, expert_smem, stride, part[warp]);
-        if (unit + 1 < unit_end) {
-            point(unit + 1);
-            first.load(rows, k, begin, end);
+        const unsigned char* x = staged_rows + g * stride + q * 16;
+        float sums[NM][2][4];
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sums[m][b][e] = 0.f;
+        for (int i = begin; i < end; i += per) {
+            const unsigned char* box = ring.next() + g * pitch + q * 16;
+            const int here = min(per, end - i);
+            uint4 lo[2][NM], hi[2][NM], v[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u >= here) continue;
+#pragma unroll
+                for (int m = 0; m < NM; ++m) {
+                    lo[u][m] = *reinterpret_cast<const uint4*>(box + m * 16 * 128 + u * 64);
+                    hi[u][m] = *reinterpret_cast<const uint4*>(box + m * 16 * 128 + u * 64 + 8 * pitch);
+                }
+                v[u][0] = *reinterpret_cast<const uint4*>(x + (i + u) * 64);
+                if (NB == 2) v[u][1] = *reinterpret_cast<const uint4*>(x + (i + u) * 64 + 8 * stride);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                if (u >= here) continue;
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    if (b >= NB) continue;
+#pragma unroll
+                    for (int m = 0; m < NM; ++m) {
+                        mma_bf16(sums[m][b], lo[u][m].x, hi[u][m].x, lo[u][m].y, hi[u][m].y, v[u][b].x, v[u][b].y);
+                        mma_bf16(sums[m][b], lo[u][m].z, hi[u][m].z, lo[u][m].w, hi[u][m].w, v[u][b].z, v[u][b].w);
+                    }
+                }
+            }
+            ring.done();
+            __syncwarp();  // the place is free
+            ask();
         }
+#pragma unroll
+        for (int m = 0; m < NM; ++m)
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (b < NB) part[warp][(m * NB + b) * 4 + e][lane] = sums[m][b][e];
         __syncthreads();
         // entry (b, i) of lane (g, q): token 8 b + 2 q + i % 2, row g + 8 (i / 2)
         for (int entry = warp; entry < NB * 4; entry += MMA_WARPS) {
-            const int t = (entry >> 2) * 8 + q * 2 + (entry & 1), row = tile * 16 + g + ((entry >> 1) & 1) * 8;
+            const int t = (entry >> 2) * 8 + q * 2 + (entry & 1), row_out = tile * 16 + g + ((entry >> 1) & 1) * 8;
             if (t >= count) continue;
             const float sum = mma_sum<ENTRIES>(part, entry, lane);
-            if constexpr (UP) act[(size_t)pairs[t] * n_rows + row] = __float2bfloat16_rn(sum / (1.f + expf(-sum)) * mma_sum<ENTRIES>(part, NB * 4 + entry, lane));
-            else parts[(size_t)pairs[t] * n_rows + row] = sum;
+            if constexpr (UP) act[(size_t)pairs[t] * n_rows + row_out] = __float2bfloat16_rn(sum / (1.f + expf(-sum)) * mma_sum<ENTRIES>(part, NB * 4 + entry, lane));
+            else parts[(size_t)pairs[t] * n_rows + row_out] = sum;
         }
         // the next unit's first barrier stands before `part` is written again
     }
+    if (!ring.ok && lane == 0) atomicExch(error_flag, 41);
+    ring.drain();
 }
 
 // ---- the same for so few pairs that their experts are nearly all different: no list, no third kernel, and a pair's row is the
@@ -1100,13 +1216,18 @@ GK_EXPORT int gk_route_groups(const void* h, int dtype, const float* w_router, c
         else GK_TILED(4);
 #undef GK_TILED
     } else GK_DISPATCH_DTYPE(dtype, T, {
-        if (per_warp == 8)
+        const size_t few = (size_t)width * (FEW_EXPERTS * sizeof(float) + FEW_TOKENS * sizeof(T));
+        if (!many && width % 8 == 0 && (((uintptr_t)h | (uintptr_t)w_router) & 15) == 0 && few <= 160 * 1024) {
+            if (few > 48 * 1024) cudaFuncSetAttribute(route_scores_few_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+            gk_launch(route_scores_few_kernel<T>, dim3((n_scores + FEW_EXPERTS - 1) / FEW_EXPERTS, (n_tokens + FEW_TOKENS - 1) / FEW_TOKENS), dim3(128), few, s,
+                      (const T*)h, w_router, z, n_tokens, width, n_scores);
+        } else if (per_warp == 8)
             gk_launch(route_scores_kernel<T, 8, 4>, score_grid, dim3(ROUTE_WARPS * 32), 0, s, (const T*)h, w_router, z, n_tokens, width, n_scores);
         else
             gk_launch(route_scores_kernel<T, 2, 4>, score_grid, dim3(ROUTE_WARPS * 32), 0, s, (const T*)h, w_router, z, n_tokens, width, n_scores);
     })
     GK_CHECK_LAUNCH("route_scores");
-    gk_launch(route_choose_kernel, dim3((n_tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem, s, (const float*)z,
+    gk_launch_behind(route_choose_kernel, dim3((n_tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem, s, (const float*)z,
               correction, ids, weights, n_tokens, n_experts, top, n_groups, keep, scale, flags, n_scores, ld_pairs, shared_weight);
     GK_CHECK_LAUNCH("route_groups");
     return GK_OK;
@@ -1154,19 +1275,44 @@ bool mma_suits(int k, int n_rows, int n_experts) {
     return k % 32 == 0 && n_rows % 16 == 0 && 8 * (size_t)mma_stride(k) <= 160 * 1024 && n_experts <= 4096;
 }
 
-constexpr size_t MMA_STATIC_SMEM = MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + MMA_WARPS * 2 * (MMA_TOKENS / 8 * 4) * 32 * sizeof(float) + 64;
+constexpr size_t ring_bytes(bool up, int depth) { return (size_t)MMA_WARPS * depth * (up ? 2 : 1) * 16 * 128; }
+constexpr size_t MMA_STATIC_SMEM = MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + MMA_WARPS * 2 * (MMA_TOKENS / 8 * 4) * 32 * sizeof(float) + 1024;
+
+struct MmaStep {
+    const void *source, *weights;
+    const int* ids;
+    void* act;
+    float* parts;
+    long long pairs;
+    int n_tokens, k, n_rows, divide, n_experts;
+    int* error_flag;
+};
+
+template <bool UP, int DEPTH>
+int launch_ring(const MmaStep& p, int at_once, size_t staged, int blocks, cudaStream_t s) {
+    CUtensorMap map;
+    const int box_k = p.k < 64 ? 32 : 64;
+    const int status = gk_matrix_map(&map, p.weights, (long long)p.n_experts * (UP ? 2 : 1) * p.n_rows, p.k, p.k, box_k, 16, false);
+    if (status) return status;
+    const long long most = std::min(p.pairs, (long long)MMA_LIST) * (p.n_rows / 16);
+    cudaFuncSetAttribute(experts_mma_kernel<UP, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - MMA_STATIC_SMEM));
+    // the down product stands behind the up product of the same call
+    gk_launch_with(!UP || g_gk_pdl != 0, experts_mma_kernel<UP, DEPTH>,
+                   dim3((unsigned)std::min(most, (long long)blocks * sm_count()), 1, (unsigned)((p.pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32),
+                   staged + ring_bytes(UP, DEPTH), s, dim3(1, 1, 1), map, (const __nv_bfloat16*)p.source, p.ids, (__nv_bfloat16*)p.act, p.parts, (int)p.pairs,
+                   p.k, p.n_rows, p.divide, p.n_experts, at_once, (int)staged, box_k, p.error_flag);
+    return GK_OK;
+}
 
 template <bool UP>
-void launch_mma(const void* source, const void* weights, const int* ids, void* act, float* parts, long long pairs, int n_tokens, int k, int n_rows, int divide,
-                int n_experts, cudaStream_t s) {
-    const int at_once = n_tokens > 8 && MMA_TOKENS * (size_t)mma_stride(k) <= 48 * 1024 ? MMA_TOKENS : 8;
-    const size_t rows = (size_t)at_once * mma_stride(k), counts = (2 * (size_t)n_experts + MMA_LIST) * 4, smem = rows > counts ? rows : counts;
-    // as many blocks as stay on the device at once: by their registers (the bound above) and by shared memory
-    const long long blocks = std::max(1LL, std::min(UP ? 3LL : 4LL, (long long)(227 * 1024 / (smem + MMA_STATIC_SMEM + 1024))));
-    const long long most = std::min(pairs, (long long)MMA_LIST) * (n_rows / 16), places = blocks * sm_count();
-    if (smem > 16 * 1024) cudaFuncSetAttribute(experts_mma_kernel<UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    gk_launch(experts_mma_kernel<UP>, dim3((unsigned)std::min(most, places), 1, (unsigned)((pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32), smem, s,
-              (const __nv_bfloat16*)source, (const __nv_bfloat16*)weights, ids, (__nv_bfloat16*)act, parts, (int)pairs, k, n_rows, divide, n_experts, at_once);
+int launch_mma(const MmaStep& p, cudaStream_t s) {
+    // 48 KB of rings and two blocks an SM; beside longer tokens' rows one block with 128 KB, or 32 KB where the rows leave no more
+    constexpr int TWO = UP ? 3 : 6, DEEP = UP ? 8 : 16, FLAT = UP ? 2 : 4;
+    const int at_once = p.n_tokens > 8 && MMA_TOKENS * (size_t)mma_stride(p.k) <= 48 * 1024 ? MMA_TOKENS : 8;
+    const size_t rows = (size_t)at_once * mma_stride(p.k), counts = (2 * (size_t)p.n_experts + MMA_LIST) * 4, staged = ((rows > counts ? rows : counts) + 127) / 128 * 128;
+    if (staged + ring_bytes(UP, TWO) + MMA_STATIC_SMEM <= 112 * 1024) return launch_ring<UP, TWO>(p, at_once, staged, 2, s);
+    if (staged + ring_bytes(UP, DEEP) + MMA_STATIC_SMEM <= 227 * 1024) return launch_ring<UP, DEEP>(p, at_once, staged, 1, s);
+    return launch_ring<UP, FLAT>(p, at_once, staged, 1, s);
 }
 
 // Megabytes of weights that the pairs of a step fetch and that they would not if every expert came once (a token's experts are all
@@ -1187,34 +1333,36 @@ struct ExpertStep {
     void* act;     // [n_tokens * top, ff] in the run's type
     float* out;
     int n_tokens, width, ff, top, n_experts;
+    int* error_flag;
 };
 
 template <typename T>
 void launch_join(const ExpertStep& p, cudaStream_t s) {
-    gk_launch(experts_join_kernel<T>, dim3(p.n_tokens, (p.width + 255) / 256), dim3(256), 0, s, (const float*)p.parts, p.weights, (const T*)p.add,
+    gk_launch_behind(experts_join_kernel<T>, dim3(p.n_tokens, (p.width + 255) / 256), dim3(256), 0, s, (const float*)p.parts, p.weights, (const T*)p.add,
               p.add_weight, p.out, p.width, p.top);
 }
 
 // up: inner values of all pairs; down: their products and the sums.  Each on the tensor cores where its sizes are whole tiles, and
 // each either a pair by itself or an expert's pairs together.
-void up_mma(const ExpertStep& p, bool few, cudaStream_t s) {
+int up_mma(const ExpertStep& p, bool few, cudaStream_t s) {
     const long long pairs = (long long)p.n_tokens * p.top;
-    if (few)
-        gk_launch(pair_up_mma_kernel, dim3((unsigned)pairs, p.ff / 16), dim3(MMA_WARPS * 32), 0, s, (const __nv_bfloat16*)p.h, (const __nv_bfloat16*)p.w_gate_up,
-                  p.ids, (__nv_bfloat16*)p.act, p.width, p.ff, p.top);
-    else
-        launch_mma<true>(p.h, p.w_gate_up, p.ids, p.act, nullptr, pairs, p.n_tokens, p.width, p.ff, p.top, p.n_experts, s);
+    if (!few) return launch_mma<true>(MmaStep{p.h, p.w_gate_up, p.ids, p.act, nullptr, pairs, p.n_tokens, p.width, p.ff, p.top, p.n_experts, p.error_flag}, s);
+    gk_launch(pair_up_mma_kernel, dim3((unsigned)pairs, p.ff / 16), dim3(MMA_WARPS * 32), 0, s, (const __nv_bfloat16*)p.h, (const __nv_bfloat16*)p.w_gate_up,
+              p.ids, (__nv_bfloat16*)p.act, p.width, p.ff, p.top);
+    return GK_OK;
 }
 
-void down_mma(const ExpertStep& p, bool few, cudaStream_t s) {
+int down_mma(const ExpertStep& p, bool few, cudaStream_t s) {
     if (few) {
         const int turns = (p.top + TOKEN_PAIRS - 1) / TOKEN_PAIRS, groups = (p.top + turns - 1) / turns;
         gk_launch(token_down_mma_kernel, dim3(p.n_tokens, p.width / 16), dim3(groups * MMA_WARPS * 32), 0, s, (const __nv_bfloat16*)p.act,
                   (const __nv_bfloat16*)p.w_down, p.ids, p.weights, (const __nv_bfloat16*)p.add, p.add_weight, p.out, p.ff, p.width, p.top);
-        return;
+        return GK_OK;
     }
-    launch_mma<false>(p.act, p.w_down, p.ids, nullptr, p.parts, (long long)p.n_tokens * p.top, p.n_tokens, p.ff, p.width, 1, p.n_experts, s);
+    const int status = launch_mma<false>(MmaStep{p.act, p.w_down, p.ids, nullptr, p.parts, (long long)p.n_tokens * p.top, p.n_tokens, p.ff, p.width, 1, p.n_experts, p.error_flag}, s);
+    if (status) return status;
     launch_join<__nv_bfloat16>(p, s);
+    return GK_OK;
 }
 
 template <typename T, typename TW>
@@ -1270,10 +1418,13 @@ int experts(const ExpertStep& p, cudaStream_t s) {
     const bool few_mma = (repeated <= 8 || (double)pairs * 3e-6 * third <= 32) && p.width / 16 <= 65535 && p.ff / 16 <= 65535;
     const bool few_up = repeated <= 64 || expert_grid(pairs, p.n_experts, p.ff, p.width, UP_ROWS).blocks() < 2LL * sm_count();
     const bool few_down = repeated <= 64 || expert_grid(pairs, p.n_experts, p.width, p.ff, DOWN_ROWS).blocks() < 2LL * sm_count();
-    if (mma_up) up_mma(p, few_mma, s);
+    int status = GK_OK;
+    if (mma_up) status = up_mma(p, few_mma, s);
     else GK_DISPATCH_DTYPE(p.dtype, T, { GK_DISPATCH_DTYPE(p.w_dtype, TW, { up_fp32<T, TW>(p, few_up, s); }) })
-    if (mma_down) down_mma(p, few_mma, s);
+    if (status) return status;
+    if (mma_down) status = down_mma(p, few_mma, s);
     else GK_DISPATCH_DTYPE(p.dtype, T, { GK_DISPATCH_DTYPE(p.w_dtype, TW, { down_fp32<T, TW>(p, few_down, s); }) })
+    if (status) return status;
     GK_CHECK_LAUNCH("experts");
     return GK_OK;
 }
@@ -1284,9 +1435,10 @@ int experts(const ExpertStep& p, cudaStream_t s) {
 // tokens than that go in several turns.
 GK_EXPORT int gk_experts(const void* h, int dtype, const void* w_gate_up, const void* w_down, int w_dtype, const int* ids, const float* weights,
                          const void* add, const float* add_weight, float* work, float* out, int n_tokens, int at_once, int width, int ff, int top,
-                         int n_experts, void* stream) {
+                         int n_experts, int* error_flag, void* stream) {
     GK_REQUIRE(GK_VALID_DTYPE(dtype) && GK_VALID_DTYPE(w_dtype), "experts: bad dtype");
     GK_REQUIRE(at_once > 0 && width > 0 && ff > 0 && top > 0 && n_experts > 0 && (add != nullptr || add_weight == nullptr), "experts: bad sizes");
+    GK_REQUIRE(error_flag != nullptr, "experts: error_flag is required");
     if (n_tokens == 0) return GK_OK;
     // a token's inner values stand in shared memory in the down product of few pairs
     GK_REQUIRE((size_t)width * sizeof(float) <= 200 * 1024, "experts: rows of %d are longer than the kernels stage", width);
@@ -1297,7 +1449,7 @@ GK_EXPORT int gk_experts(const void* h, int dtype, const void* w_gate_up, const 
         const size_t row = (size_t)at * width;
         const ExpertStep p{(const char*)h + row * size, w_gate_up, w_down, dtype, w_dtype, ids + (size_t)at * top, weights + (size_t)at * top,
                            add ? (const char*)add + row * size : nullptr, add_weight ? add_weight + at : nullptr, work, work + (size_t)at_once * top * width,
-                           out + row, std::min(at_once, n_tokens - at), width, ff, top, n_experts};
+                           out + row, std::min(at_once, n_tokens - at), width, ff, top, n_experts, error_flag};
         const int status = experts(p, (cudaStream_t)stream);
         if (status != GK_OK) return status;
     }

@@ -1629,7 +1629,7 @@ def experts_pairwise(h: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Ten
     at_once = max(1, min(T, EXPERT_PAIRS_AT_ONCE // max(top, 1)))
     work = torch.empty((at_once * top * (4 * width + ff * h.element_size()),), dtype=torch.uint8, device=h.device)
     call("gk_experts", ptr(h), dtype_code(h.dtype), ptr(w_gate_up), ptr(w_down), dtype_code(w_gate_up.dtype), ptr(ids), ptr(weights), ptr(add),
-         ptr(add_weight), ptr(work), ptr(out), T, at_once, width, ff, top, E, stream_ptr())
+         ptr(add_weight), ptr(work), ptr(out), T, at_once, width, ff, top, E, ptr(error_flag(h.device)), stream_ptr())
     return out
 
 

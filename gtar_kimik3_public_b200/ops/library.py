@@ -81,7 +81,7 @@ _SIGNATURES: dict[str, list] = {
     "gk_delta_channel": [P, L, P, L, P, P, P, P, P, F, P, P, P, P, P, I, I, I, I, I, I, I, I, P],
     "gk_head_norm_gate": [P, P, P, I, L, P, I, L, I, I, F, P],
     "gk_route_groups": [P, I, P, P, P, P, P, I, I, I, I, I, I, F, I, I, P, P],
-    "gk_experts": [P, I, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, P],
+    "gk_experts": [P, I, P, P, I, P, P, P, P, P, P, I, I, I, I, I, I, P, P],
     "gk_experts_sort": [P, I, I, P, P, P, P],
     "gk_gather_rows": [P, I, P, P, I, I, I, P],
     "gk_experts_combine": [P, I, P, P, P, P, P, I, I, I, P],
