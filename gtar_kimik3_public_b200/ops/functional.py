@@ -381,8 +381,11 @@ def split_k_for(m: int, n: int, k: int) -> int:
         return 1
     tiles = -(-n // 128) * -(-m // min(SKINNY_BN_MAX, 16 if m <= 16 else 32 if m <= 32 else 64))
     by_blocks = SPLIT_TARGET_BLOCKS // tiles
-    if tiles * 8 <= SPLIT_TARGET_BLOCKS + 32:
-        by_blocks = 8  # 17 to 20 tiles: eight ways (up to 160 blocks) beat four (2,560 rows of 9,728: 14.0 against 17.2 us)
+    # 17 to 20 tiles: with up to 16 tokens eight ways (up to 160 blocks, two on an SM) beat four (2,560 rows of 9,728: 14.0 against 17.2
+    # us).  With more tokens a block's ring is larger and two on an SM have half of it each, so eight ways only where every block has an
+    # SM of its own (the same rows, 32 tokens: 26.6 us eight ways, 22.5 four ways; 64 tokens: 29.6 and 23.6, cold weights)
+    if tiles * 8 <= SPLIT_TARGET_BLOCKS + (32 if m <= 16 else 16):
+        by_blocks = 8
     limit = min(by_blocks, (k // 64) // SPLIT_MIN_K_BLOCKS, 8)
     return 8 if limit >= 8 else 4 if limit >= 4 else 2 if limit >= 2 else 1
 

@@ -162,3 +162,12 @@ def test_exact_attention_routes_at_measured_points():
                     got = route(tokens, seqs, longest, n_q, n_kv, d, dtype)
                     assert got in (SINGLE, WARPS, TILES, TILES | WARPS), (n_q, n_kv, d, seqs, longest, got)
                     assert got != TILES or seqs == 1, (n_q, n_kv, d, seqs, longest)
+
+
+def test_split_k_of_more_than_sixteen_tokens_leaves_every_block_an_sm():
+    # a block of 17 tokens and more has the deep ring only where no other block shares its SM
+    assert split_k_for(16, 2560, 9728) == 8 and split_k_for(17, 2560, 9728) == 4 and split_k_for(64, 2560, 9728) == 4
+    for m in (17, 32, 64):
+        for n in range(128, 2700, 128):
+            splits = split_k_for(m, n, 9728)
+            assert splits < 8 or -(-n // 128) * splits <= 148
