@@ -24,10 +24,11 @@
 // whose own sums are cut and not rounded (H. Ootomo, R. Yokota, "Recovering single precision accuracy from Tensor Cores while
 // surpassing the FP32 theoretical peak performance").  FFMA instead would be bound by what shared memory can deliver.
 //
-// Measured (us, the kernels that go token by token / here; heads of 128): one prompt of 2,048, 8 heads: 620 / 189; 1,024 + 500 + 77
-// tokens, 16 heads: 537 / 341; 100 + 40 + 900, 8 heads: 304 / 142.  Error of the states against 64 bits, relative: 4.07e-7 both ways at the
-// first, 3.2e-7 / 3.3e-7 at the second, 1.6e-7 / 2.0e-7 after 16 tokens; of the bfloat16 read-outs 1.66e-3 both ways.  `inner` is bound by latency (57 us
-// of the 189: its phases follow one another, two blocks an SM), `walk` by its two products and three barriers a chunk (2 us).
+// Measured (us, the kernels that go token by token / here; heads of 128): one prompt of 2,048, 8 heads: 620 / 137; 1,024 + 500 + 77
+// tokens, 16 heads: 537 / 283; 100 + 40 + 900, 8 heads: 305 / 126; 32 prompts of 40: 154 / 136.  Error of the states against 64 bits,
+// relative: 4.07e-7 / 4.09e-7 at the first, 3.15e-7 / 3.31e-7 at the second, 1.6e-7 / 2.0e-7 after 16 tokens; of the bfloat16 read-outs
+// 1.66e-3 both ways.  `inner` is bound by latency (some 50 us of the 137: its phases follow one another, two blocks an SM), `walk` by its two products and
+// three barriers a chunk (1.5 us).
 
 #include "common.cuh"
 
@@ -56,7 +57,12 @@ struct Unit {
 // Quotients without the branch that a rounded division carries for numbers out of range, so that a thread's many are worked out side by side
 __device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + expf(fminf(-z, 80.f))); }
 __device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.f, 1.f + expf(fminf(-z, 80.f))); }
-__device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+// log(1 + e^z) = max(z, 0) + log(1 + u), u = e^-|z|; with w = 1 + u as rounded, log(1 + u) = log(w) u / (w - 1) to a few last places (D.
+// Goldberg, "What Every Computer Scientist Should Know About Floating-Point Arithmetic", theorem 4).
+__device__ __forceinline__ float softplus_f(float z) {
+    const float u = expf(-fabsf(z)), w = 1.f + u;
+    return fmaxf(z, 0.f) + (w == 1.f ? u : logf(w) * __fdividef(u, w - 1.f));
+}
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -81,6 +87,13 @@ __device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint3
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// the same with nothing to add to
+__device__ __forceinline__ void mma_alone(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // Left operand, 16 x 8: lane 4 r + c holds rows r, r + 8 of two columns, in the order (r, first), (r + 8, first), (r, second),
 // (r + 8, second).  Which two columns is free as long as the right operand's two rows are the same ones: 2c and 2c + 1 where an
 // accumulator becomes an operand (no exchange between lanes), c and c + 4 where rows lie four banks apart.
@@ -93,17 +106,23 @@ struct Left {
         split(d, hi[3], lo[3]);
     }
 };
-struct Sum {
-    float acc[4], low[4];  // the large parts, and the small ones, whose sums may be the tensor core's own
-    __device__ __forceinline__ Sum() {
+// CHAINS: of the small parts' products, which the tensor core adds up itself, one after another
+template <int CHAINS>
+struct SumOf {
+    float acc[4], low[CHAINS][4];
+    __device__ __forceinline__ SumOf() {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] = low[i] = 0.f;
+        for (int i = 0; i < 4; ++i) {
+            acc[i] = 0.f;
+#pragma unroll
+            for (int j = 0; j < CHAINS; ++j) low[j][i] = 0.f;
+        }
     }
     __device__ __forceinline__ void add(const Left& a, uint32_t h0, uint32_t h1, uint32_t l0, uint32_t l1) {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        mma(c, a.hi, h0, h1);
-        mma(low, a.lo, h0, h1);
-        mma(low, a.hi, l0, l1);
+        float c[4];
+        mma_alone(c, a.hi, h0, h1);
+        mma(low[0], a.lo, h0, h1);
+        mma(low[CHAINS - 1], a.hi, l0, l1);
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[i] += c[i];
     }
@@ -113,24 +132,37 @@ struct Sum {
         split(b1, h1, l1);
         add(a, h0, h1, l0, l1);
     }
-    __device__ __forceinline__ float at(int i) const { return acc[i] + low[i]; }
+    __device__ __forceinline__ float at(int i) const { return acc[i] + (CHAINS > 1 ? low[0][i] + low[CHAINS - 1][i] : low[0][i]); }
 };
+typedef SumOf<1> Sum;
 
 // entry (t, j) of a 16 x 16 block in shared memory: pairs of columns turned so that eight rows' pairs fall into different banks
 __device__ __forceinline__ int at16(int t, int j) { return t * SUB + 2 * ((j >> 1) ^ (((t >> 1) & 1) << 2)) + (j & 1); }
 
+// N (4 or 2) bfloat16 numbers as they lie in memory
 template <int N>
-__device__ __forceinline__ void load_row(const bf16* src, float (&x)[N]) {
-    if constexpr (N == 4) {
-        const uint2 raw = *reinterpret_cast<const uint2*>(src);
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-        x[0] = a.x, x[1] = a.y, x[2] = b.x, x[3] = b.y;
-    } else {
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src));
-        x[0] = a.x, x[1] = a.y;
+struct Raw {
+    uint32_t pairs[N / 2];
+    __device__ __forceinline__ void numbers(float (&x)[N]) const {
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pairs[i]));
+            x[2 * i] = f.x, x[2 * i + 1] = f.y;
+        }
     }
-}
+};
+template <>
+struct __align__(8) Raw<4> {
+    uint32_t pairs[2];
+    __device__ __forceinline__ void numbers(float (&x)[4]) const {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pairs[i]));
+            x[2 * i] = f.x, x[2 * i + 1] = f.y;
+        }
+    }
+};
+
 template <int N>
 __device__ __forceinline__ void load_row(const float* src, float (&x)[N]) {
     if constexpr (N == 4) {
@@ -160,22 +192,38 @@ struct Inputs {
 
 // Eight consecutive tokens' convolution and SiLU of N neighbouring channels from column c on; s0: the first token's place in the
 // step, `live` of the eight are there.  Inputs before the step come from the sequence's convolution state.
-template <int N>
+template <int N, bool USUAL>
 __device__ __forceinline__ void conv_eight(const Inputs& in, int tok, int s0, int live, size_t slot, int c, int channels, float (&y)[8][N]) {
-    const int taps = in.taps;
-    float w[MAX_TAPS][N], x[8 + MAX_TAPS - 1][N];
+    const int taps = USUAL ? MAX_TAPS : in.taps;
+    constexpr int ROWS = 8 + MAX_TAPS - 1;
+    float w[MAX_TAPS][N], x[ROWS][N];
+    Raw<N> raw[ROWS];  // all of them asked for before the first is looked at
 #pragma unroll
-    for (int j = 0; j < MAX_TAPS; ++j)
+    for (int i = 0; i < ROWS; ++i) {
+        const int back = i - (MAX_TAPS - 1);
+        const bool there = back < live && -back < taps && s0 + back >= 0;
+        raw[i] = there ? *reinterpret_cast<const Raw<N>*>(in.proj + (long long)(tok + back) * in.ld + c) : Raw<N>{};
+    }
+    if (USUAL) {
 #pragma unroll
-        for (int e = 0; e < N; ++e) w[j][e] = j < taps ? in.conv_w[(size_t)(c + e) * taps + taps - 1 - j] : 0.f;
+        for (int e = 0; e < N; ++e) {
+            const float4 four = *reinterpret_cast<const float4*>(in.conv_w + (size_t)(c + e) * MAX_TAPS);
+            w[3][e] = four.x, w[2][e] = four.y, w[1][e] = four.z, w[0][e] = four.w;
+        }
+    } else {
 #pragma unroll
-    for (int i = 0; i < 8 + MAX_TAPS - 1; ++i) {
-        const int back = i - (MAX_TAPS - 1), s = s0 + back;
+        for (int j = 0; j < MAX_TAPS; ++j)
 #pragma unroll
-        for (int e = 0; e < N; ++e) x[i][e] = 0.f;
-        if (back >= live || -back >= taps) continue;
-        if (s >= 0) load_row<N>(in.proj + (long long)(tok + back) * in.ld + c, x[i]);
-        else if (taps - 1 + s >= 0) load_row<N>(in.conv_state + (slot * (taps - 1) + (taps - 1 + s)) * channels + c, x[i]);
+            for (int e = 0; e < N; ++e) w[j][e] = j < taps ? in.conv_w[(size_t)(c + e) * taps + taps - 1 - j] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) raw[i].numbers(x[i]);
+    if (s0 < taps - 1 && live > 0) {  // the step's first tokens
+#pragma unroll
+        for (int i = 0; i < MAX_TAPS - 1; ++i) {
+            const int s = s0 + i - (MAX_TAPS - 1);
+            if (s < 0 && taps - 1 + s >= 0) load_row<N>(in.conv_state + (slot * (taps - 1) + (taps - 1 + s)) * channels + c, x[i]);
+        }
     }
 #pragma unroll
     for (int t = 0; t < 8; ++t)
@@ -194,18 +242,20 @@ struct InnerSmem {
     static constexpr int LD = D + 4;  // rows four banks apart
     float k[CHUNK][LD], g[CHUNK][LD], q[CHUNK][LD];
     float blk[10][TILE16];            // (1 + A)^-1 of the four blocks on the diagonal, then the six of A below it
-    float total[4][D];                // decays over a block
+    float total[5][D];                // decays over a block, and ones
     float beta[CHUNK];
 };
 
-template <int D>
+// USUAL: four taps, values as wide as keys and tap weights on 16 bytes, known when the kernel is built: without branches on them a thread's
+// loads are asked for together.
+template <int D, bool USUAL>
 __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, float* __restrict__ work) {
     constexpr int N = D / 32, KS = D / 8, LD = InnerSmem<D>::LD;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     InnerSmem<D>& sm = *reinterpret_cast<InnerSmem<D>*>(smem_raw);
     pdl_launch_dependents();
     pdl_wait();
-    const int head = blockIdx.y, seq = blockIdx.z, hk = head / (in.n_heads / in.n_kv), dv = in.dv;
+    const int head = blockIdx.y, seq = blockIdx.z, hk = head / (in.n_heads / in.n_kv), dv = USUAL ? D : in.dv;
     const int t0 = in.cu_q[seq], len = in.cu_q[seq + 1] - t0;
     const int first = (in.chunk0 + blockIdx.x) * CHUNK;
     if (first >= len) return;
@@ -229,7 +279,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
             const bool values = part == 2;
             if (values && at >= dv) break;
             float y[8][N];
-            conv_eight<N>(in, tok0 + w0, first + w0, live, slot, (values ? 2 * qk + head * dv : part * qk + hk * D) + at, channels, y);
+            conv_eight<N, USUAL>(in, tok0 + w0, first + w0, live, slot, (values ? 2 * qk + head * dv : part * qk + hk * D) + at, channels, y);
             if (values) {  // for now where their solutions will be
 #pragma unroll
                 for (int t = 0; t < 8; ++t) store_row<N>(mine + Unit<D>::U + (w0 + t) * dv + at, y[t]);
@@ -255,6 +305,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
                 store_row<N>(to + t * LD, y[t]);
             }
         }
+        if (tid < D) sm.total[4][tid] = 1.f;
         if (tid < CHUNK) sm.beta[tid] = tid < n ? sigmoid_f(to_float(in.proj[(long long)(tok0 + tid) * in.ld + channels + head])) : 0.f;
     }
     cp_async_wait<0>();
@@ -263,7 +314,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
         const float rate = -expf(in.a_log[head]);
         const int c = tid % D;
         const float bias = in.dt_bias[head * D + c];
-#pragma unroll 2
+#pragma unroll 4
         for (int t = tid / D; t < CHUNK; t += THREADS / D) sm.g[t][c] = t < n ? expf(rate * softplus_f(sm.g[t][c] + bias)) : 1.f;
     }
     __syncthreads();
@@ -278,7 +329,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
             for (int e = 0; e < N; ++e) held[m][e] = 0.f;
         const int value = ((lane >> 4) & 1) * 8 + ((lane >> 3) & 1) * 4 + ((lane >> 2) & 1) * 2 + ((lane >> 1) & 1);
         const int j = 2 * (value & 7) + odd;
-#pragma unroll 1
+#pragma unroll 2
         for (int t = 0; t < SUB; ++t) {
             float g[N], k[N], q[N], v[16];
             load_row<N>(&sm.g[b * SUB + t][at], g);
@@ -365,14 +416,11 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
         const int I = pair == 0 ? 1 : pair < 3 ? 2 : 3, J = pair - I * (I - 1) / 2;
         const float* a = (queries ? &sm.q[I * SUB + r][0] : &sm.k[I * SUB + r][0]) + c2;
         const float* b = &sm.g[J * SUB + nt * 8 + r][0] + c2;
-        Sum s;
+        const float *f1 = sm.total[I - J > 1 ? J + 1 : 4] + c2, *f2 = sm.total[I - J > 2 ? J + 2 : 4] + c2;  // the blocks between
+        SumOf<2> s;
 #pragma unroll 4
         for (int ks = 0; ks < KS; ++ks) {
-            float b0 = b[8 * ks], b1 = b[8 * ks + 4];
-            for (int between = J + 1; between < I; ++between) {
-                b0 *= sm.total[between][8 * ks + c2];
-                b1 *= sm.total[between][8 * ks + c2 + 4];
-            }
+            const float b0 = b[8 * ks] * f1[8 * ks] * f2[8 * ks], b1 = b[8 * ks + 4] * f1[8 * ks + 4] * f2[8 * ks + 4];
             s.add(Left(a[8 * ks], a[8 * ks + 8 * LD], a[8 * ks + 4], a[8 * ks + 8 * LD + 4]), b0, b1);
         }
         if (queries) {
@@ -477,19 +525,20 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
     }
 }
 
-template <int D>
+// RING: tiles that a warp's pieces of are in flight or in use: six where a block has an SM to itself, three where two share one
+template <int D, int RING>
 struct WalkSmem {
-    float4 ring[3][8][8][32];                // a warp's pieces of three tiles: a lane reads back what it copied itself
+    float4 ring[RING][8][8][32];             // a warp's pieces of the tiles: a lane reads back what it copied itself
     float state[2][STRIP][D + 8];            // rounded, rest: rows of value columns, eight banks apart
     float u[2][STRIP][CHUNK + 8];
     float4 part[4][32];                      // the second half of the first product's sums
 };
 
-template <int D>
-__global__ void __launch_bounds__(THREADS, 2) channel_walk_kernel(Inputs in, float* __restrict__ work, float* __restrict__ state) {
+template <int D, int RING>
+__global__ void __launch_bounds__(THREADS, RING == 3 ? 2 : 1) channel_walk_kernel(Inputs in, float* __restrict__ work, float* __restrict__ state) {
     constexpr int HALF = D / 16;  // steps of eight channels that a warp has of the first product
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    WalkSmem<D>& sm = *reinterpret_cast<WalkSmem<D>*>(smem_raw);
+    WalkSmem<D, RING>& sm = *reinterpret_cast<WalkSmem<D, RING>*>(smem_raw);
     pdl_launch_dependents();
     pdl_wait();
     const int head = blockIdx.y, seq = blockIdx.z, v0 = blockIdx.x * STRIP, dv = in.dv;
@@ -519,17 +568,16 @@ __global__ void __launch_bounds__(THREADS, 2) channel_walk_kernel(Inputs in, flo
             if ((i & 1) == 0) {
                 const float4* src = reinterpret_cast<const float4*>(u + Unit<D>::W) + (mt * (D / 8) + kh * HALF) * 32 + lane;
 #pragma unroll
-                for (int ks = 0; ks < HALF; ++ks) cp_async_16(&sm.ring[i % 3][warp][ks][lane], src + ks * 32);
+                for (int ks = 0; ks < HALF; ++ks) cp_async_16(&sm.ring[i % RING][warp][ks][lane], src + ks * 32);
             } else if (owns) {
                 const float4* src = reinterpret_cast<const float4*>(u + Unit<D>::K) + warp * 8 * 32 + lane;
 #pragma unroll
-                for (int ks = 0; ks < 8; ++ks) cp_async_16(&sm.ring[i % 3][warp][ks][lane], src + ks * 32);
+                for (int ks = 0; ks < 8; ++ks) cp_async_16(&sm.ring[i % RING][warp][ks][lane], src + ks * 32);
             }
         }
         cp_async_commit();
     };
-    issue(0);
-    issue(1);
+    for (int i = 0; i < RING - 1; ++i) issue(i);
     float* saved = state + (slot * in.n_heads + head) * (size_t)D * dv + v0 + 2 * c2;
     float S[4] = {0.f, 0.f, 0.f, 0.f};
     const int ch = warp * 16 + r;
@@ -569,14 +617,14 @@ __global__ void __launch_bounds__(THREADS, 2) channel_walk_kernel(Inputs in, flo
         const float2 u0 = next_u[0], u1 = next_u[1];
         const float g0 = next_g[0], g1 = next_g[1];
         fetch(i + 1);
-        issue(2 * i + 2);
-        cp_async_wait<2>();
+        issue(2 * i + RING - 1);
+        cp_async_wait<RING - 1>();
         __syncthreads();  // the state before the chunk is there
         {
-            Sum s;
+            SumOf<2> s;
 #pragma unroll
             for (int ks = 0; ks < HALF; ++ks) {
-                const float4 a = sm.ring[(2 * i) % 3][warp][ks][lane];
+                const float4 a = sm.ring[(2 * i) % RING][warp][ks][lane];
                 const int at = (kh * HALF + ks) * 8 + 2 * c2;
                 const uint2 hi = *reinterpret_cast<const uint2*>(&sm.state[0][r][at]), lo = *reinterpret_cast<const uint2*>(&sm.state[1][r][at]);
                 s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
@@ -600,14 +648,14 @@ __global__ void __launch_bounds__(THREADS, 2) channel_walk_kernel(Inputs in, flo
                 *reinterpret_cast<float2*>(mine + Unit<D>::U + (tok + 8) * dv + v0 + 2 * c2) = make_float2(u[2], u[3]);
             }
         }
-        issue(2 * i + 3);
-        cp_async_wait<2>();
+        issue(2 * i + RING);
+        cp_async_wait<RING - 1>();
         __syncthreads();  // u is there, and nobody reads the state before the chunk any more
         if (owns) {
-            Sum s;
+            SumOf<2> s;
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks) {
-                const float4 a = sm.ring[(2 * i + 1) % 3][warp][ks][lane];
+                const float4 a = sm.ring[(2 * i + 1) % RING][warp][ks][lane];
                 const uint2 hi = *reinterpret_cast<const uint2*>(&sm.u[0][r][ks * 8 + 2 * c2]), lo = *reinterpret_cast<const uint2*>(&sm.u[1][r][ks * 8 + 2 * c2]);
                 s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
             }
@@ -631,14 +679,14 @@ struct ReadSmem {
     float squares[2][CHUNK];
 };
 
-template <int D>
+template <int D, bool USUAL>
 __global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, const float* __restrict__ work, bf16* __restrict__ out, float eps) {
     constexpr int LD = ReadSmem<D>::LD;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     ReadSmem<D>& sm = *reinterpret_cast<ReadSmem<D>*>(smem_raw);
     pdl_launch_dependents();
     pdl_wait();
-    const int head = blockIdx.y, seq = blockIdx.z, dv = in.dv;
+    const int head = blockIdx.y, seq = blockIdx.z, dv = USUAL ? D : in.dv;
     const int t0 = in.cu_q[seq], len = in.cu_q[seq + 1] - t0;
     const int first = (in.chunk0 + blockIdx.x) * CHUNK;
     if (first >= len) return;
@@ -695,13 +743,19 @@ __global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, con
         const float unit = 1.f / sqrtf((sm.squares[0][t] + sm.squares[1][t]) / (float)dv + eps);
         const float* gate = in.low + (long long)(tok0 + t) * in.ld_low + (long long)in.n_heads * D + head * dv + v0 + 2 * c2;
         bf16* to = out + ((size_t)(tok0 + t) * in.n_heads + head) * dv + v0 + 2 * c2;
+        float2 z[8], w[8];  // all asked for before the first is used
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-            if (nt >= tiles) continue;
-            const float2 z = *reinterpret_cast<const float2*>(gate + nt * 8), w = *reinterpret_cast<const float2*>(in.norm + v0 + nt * 8 + 2 * c2);
-            const float x = s[nt].acc[2 * h] * unit * w.x * sigmoid_f(z.x), y = s[nt].acc[2 * h + 1] * unit * w.y * sigmoid_f(z.y);
-            *reinterpret_cast<__nv_bfloat162*>(to + nt * 8) = __floats2bfloat162_rn(x, y);
-        }
+        for (int nt = 0; nt < 8; ++nt)
+            if (nt < tiles) {
+                z[nt] = *reinterpret_cast<const float2*>(gate + nt * 8);
+                w[nt] = *reinterpret_cast<const float2*>(in.norm + v0 + nt * 8 + 2 * c2);
+            }
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+            if (nt < tiles) {
+                const float x = s[nt].acc[2 * h] * unit * w[nt].x * sigmoid_f(z[nt].x), y = s[nt].acc[2 * h + 1] * unit * w[nt].y * sigmoid_f(z[nt].y);
+                *reinterpret_cast<__nv_bfloat162*>(to + nt * 8) = __floats2bfloat162_rn(x, y);
+            }
     }
 }
 
@@ -727,35 +781,54 @@ GK_EXPORT int gk_delta_channel(const void* proj, long long ld, const float* low,
     GK_REQUIRE((((uintptr_t)proj | (uintptr_t)low | (uintptr_t)work | (uintptr_t)state | (uintptr_t)conv_state | (uintptr_t)dt_bias | (uintptr_t)norm |
                  (uintptr_t)out) & 15) == 0, "delta_channel: tensors must start on 16 bytes");
     if (n_seqs == 0 || max_len == 0) return GK_OK;
-    static bool prepared = false;
-    if (!prepared) {
+    static int sms = 0;
+    if (sms == 0) {
 #define GK_ATTR(KERNEL, BYTES)                                                                                  \
     if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BYTES)) != cudaSuccess) \
         return gk_fail(GK_CUDA_ERROR, "delta_channel: shared memory")
-        GK_ATTR(channel_inner_kernel<64>, sizeof(InnerSmem<64>));
-        GK_ATTR(channel_inner_kernel<128>, sizeof(InnerSmem<128>));
-        GK_ATTR(channel_walk_kernel<64>, sizeof(WalkSmem<64>));
-        GK_ATTR(channel_walk_kernel<128>, sizeof(WalkSmem<128>));
-        GK_ATTR(channel_read_kernel<64>, sizeof(ReadSmem<64>));
-        GK_ATTR(channel_read_kernel<128>, sizeof(ReadSmem<128>));
+#define GK_ATTRS(D)                                                  \
+    GK_ATTR((channel_inner_kernel<D, false>), sizeof(InnerSmem<D>)); \
+    GK_ATTR((channel_inner_kernel<D, true>), sizeof(InnerSmem<D>));  \
+    GK_ATTR((channel_walk_kernel<D, 3>), sizeof(WalkSmem<D, 3>));    \
+    GK_ATTR((channel_walk_kernel<D, 6>), sizeof(WalkSmem<D, 6>));    \
+    GK_ATTR((channel_read_kernel<D, false>), sizeof(ReadSmem<D>));   \
+    GK_ATTR((channel_read_kernel<D, true>), sizeof(ReadSmem<D>))
+        GK_ATTRS(64);
+        GK_ATTRS(128);
+#undef GK_ATTRS
 #undef GK_ATTR
-        prepared = true;
+        int device = 0, n = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) n = 148;
+        sms = n;
     }
     cudaStream_t s = (cudaStream_t)stream;
     const int chunks = (max_len + CHUNK - 1) / CHUNK;
+    const bool usual = taps == MAX_TAPS && dv == d && ((uintptr_t)conv_w & 15) == 0;
+    const dim3 strips(dv / STRIP, n_heads, n_seqs);
+    const bool alone = (long long)strips.x * strips.y * strips.z <= sms;
     for (int chunk0 = 0; chunk0 < chunks; chunk0 += wave) {
         const int here = chunks - chunk0 < wave ? chunks - chunk0 : wave;
         const Inputs in{(const bf16*)proj, low, conv_w, conv_state, a_log, dt_bias, norm, cu_q, slots, ld, ld_low, n_heads, n_kv, dv, taps, chunk0, wave};
-#define GK_CHANNEL(D)                                                                                                                  \
-    gk_launch(channel_inner_kernel<D>, dim3(here, n_heads, n_seqs), dim3(THREADS), sizeof(InnerSmem<D>), s, in, work);                 \
-    gk_launch_behind(channel_walk_kernel<D>, dim3(dv / STRIP, n_heads, n_seqs), dim3(THREADS), sizeof(WalkSmem<D>), s, in, work, state);      \
-    gk_launch_behind(channel_read_kernel<D>, dim3(here, n_heads, n_seqs), dim3(THREADS), sizeof(ReadSmem<D>), s, in, (const float*)work, (bf16*)out, eps)
+        const dim3 units(here, n_heads, n_seqs);
+#define GK_INNER(D, USUAL) gk_launch(channel_inner_kernel<D, USUAL>, units, dim3(THREADS), sizeof(InnerSmem<D>), s, in, work)
+#define GK_WALK(D, RING) gk_launch_behind(channel_walk_kernel<D, RING>, strips, dim3(THREADS), sizeof(WalkSmem<D, RING>), s, in, work, state)
+#define GK_READ(D, USUAL) gk_launch_behind(channel_read_kernel<D, USUAL>, units, dim3(THREADS), sizeof(ReadSmem<D>), s, in, (const float*)work, (bf16*)out, eps)
+#define GK_CHANNEL(D)              \
+    if (usual) GK_INNER(D, true);  \
+    else GK_INNER(D, false);       \
+    if (alone) GK_WALK(D, 6);      \
+    else GK_WALK(D, 3);            \
+    if (usual) GK_READ(D, true);   \
+    else GK_READ(D, false)
         if (d == 64) {
             GK_CHANNEL(64);
         } else {
             GK_CHANNEL(128);
         }
 #undef GK_CHANNEL
+#undef GK_READ
+#undef GK_WALK
+#undef GK_INNER
     }
     GK_CHECK_LAUNCH("delta_channel");
     return GK_OK;

@@ -1346,9 +1346,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
     return out
 
 
-# The longest run of a step from which on the chunks are the faster way: their three kernels take 73 us for one chunk and some two more
-# a chunk, the kernels that go token by token 0.3 us a token behind 13 (8 heads of 128, one prompt: 33 tokens: 75 / 23 us, 2,048: 189 / 620).
-DELTA_CHANNEL_MIN_TOKENS = 256
+# The longest run of a step from which on the chunks are the faster way: their three kernels take 57 us for one chunk and some 2.5 more
+# a chunk, the kernels that go token by token 0.27 us a token behind 14 (8 heads of 128, one prompt: 33 tokens: 57 / 23 us, 2,048: 137 / 620).
+DELTA_CHANNEL_MIN_TOKENS = 192
 
 
 def delta_channel_ok(proj: torch.Tensor, low: torch.Tensor, dt_bias: torch.Tensor, norm_w: torch.Tensor, conv_state: torch.Tensor | None,

@@ -19,7 +19,7 @@ What a sequence keeps between steps: the states of all heads and the convolution
 A step's kernels: the packed projection q | k | v | b; the packed first halves of the two low-rank paths and one product
 for their second halves (a block-diagonal matrix); one kernel for convolutions, activations, unit lengths, decays and
 beta; one that moves the convolution state on; the recurrence; norm and gate; the output projection.  Prompts,
-portions of prompts and single tokens take the same path in 32-bit runs; bfloat16 steps with a run of 256 tokens and more
+portions of prompts and single tokens take the same path in 32-bit runs; bfloat16 steps with a run of 192 tokens and more
 (heads of 64 or 128) do everything between the projections in chunks of 64 tokens on the tensor cores, with 32-bit operands.
 
 The second, ``head_delta``, has one decay number per head, ``g_t = exp(-exp(A_h) * softplus(W_a x + dt_bias_h))``, and its gate is
