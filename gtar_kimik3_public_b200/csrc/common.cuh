@@ -37,6 +37,9 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 extern int g_gk_pdl;  // set through gk_set_pdl(): launch kernels with programmatic stream serialization
+// gk_chain(): this thread is launching the kernels of one layer.  1: none of them yet (the first waits for all that is in front of
+// it, as ever), 2: the later ones, which may start early like those of a captured step.
+extern thread_local int t_gk_chain;
 void gk_prepare_kernel(const void* kernel);  // once per kernel: its preferred L1 / shared-memory split
 
 // Launches `kernel` on `stream` as thread-block clusters of `cluster` blocks (where that is more than one), with the
@@ -72,7 +75,9 @@ inline cudaError_t gk_launch_with(bool early, void (*kernel)(KArgs...), dim3 gri
 template <typename... KArgs, typename... Args>
 inline cudaError_t gk_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                      dim3 cluster, Args... args) {
-    return gk_launch_with(g_gk_pdl != 0, kernel, grid, block, smem, stream, cluster, args...);
+    const bool early = g_gk_pdl != 0 || t_gk_chain == 2;
+    if (t_gk_chain == 1) t_gk_chain = 2;
+    return gk_launch_with(early, kernel, grid, block, smem, stream, cluster, args...);
 }
 
 template <typename... KArgs, typename... Args>

@@ -40,6 +40,16 @@ GK_EXPORT int gk_set_pdl(int on) {
     return before;
 }
 
+thread_local int t_gk_chain = 0;
+
+// on = 1: the calls of this thread up to the one with 0 launch the kernels of one layer, which read nothing before pdl_wait() that one of
+// them writes; all but the first may start early.  Returns the state before (0: outside a layer).
+GK_EXPORT int gk_chain(int on) {
+    const int before = t_gk_chain;
+    t_gk_chain = on ? 1 : 0;
+    return before;
+}
+
 GK_EXPORT const char* gk_last_error() { return g_last_error; }
 
 // Interface revision: the Python side refuses a library built from other sources.

@@ -8,6 +8,7 @@ reason.  Nothing here falls back to the CPU or to a library's model code.
 from __future__ import annotations
 
 import ctypes
+import functools
 import threading
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
@@ -52,6 +53,7 @@ _SIGNATURES: dict[str, list] = {
     "gk_gemv_bf16": [P, I, I, L, P, I, L, P, I, I, F, F, P],
     "gk_gemv_bf16_stream": [P, I, I, L, P, I, L, P, I, I, P, L, P, I, F, P, L, P],
     "gk_set_pdl": [I],
+    "gk_chain": [I],
     "gk_attention_decode_resident_clusters": [I, I],
     "gk_set_gemm_pairs": [I],
     "gk_set_attention_prefill_keys": [I],
@@ -190,3 +192,22 @@ def call(name: str, *args) -> None:
         entry = _entries[name] = getattr(library(), name)
     if entry(*args) != 0:
         raise KernelError(f"{name}: {library().gk_last_error().decode(errors='replace')}")
+
+
+def one_layer(forward):
+    """For a method that launches the kernels of one layer of a model, called outside captured steps too: the library's kernels behind
+    the first may take their places on the SMs, and fetch weights, while the one in front of them drains, as in a captured step.  They read
+    nothing early that a kernel of the layer writes; the first waits for everything in front of it.  The mark is the calling thread's
+    own.  (Measured, called as a program calls a layer: a feed-forward of 4B sizes at 8 tokens 36.9 us without the mark and 33.2 with it, of 8B
+    sizes at 64 tokens 70.3 and 66.7.)"""
+
+    @functools.wraps(forward)
+    def marked(*args, **kwargs):
+        chain = library().gk_chain
+        chain(1)
+        try:
+            return forward(*args, **kwargs)
+        finally:
+            chain(0)
+
+    return marked

@@ -14,6 +14,7 @@ import torch
 from ..ops import attention as attention_ops
 from ..ops import functional as F
 from ..ops.linear import linear, linear_normed, linear_on_stream_ok, linear_residual
+from ..ops.library import one_layer
 from .base import KVRequest, Mixer, PositionEncoding, StepContext, TensorSpec, register_part
 
 
@@ -73,6 +74,7 @@ class GQAAttention(Mixer):
                 "has_qk_norm": self.q_norm is not None, "eps_qk": self.qk_norm_eps or 1.0,
                 "qk_dtype": None if self.q_norm is None else self.q_norm.dtype, "rope": rope, "scale": self.scale}
 
+    @one_layer
     def forward(self, x, ctx: StepContext, cache: F.PagedKV) -> torch.Tensor:
         cos = sin = None
         if self.position is not None:

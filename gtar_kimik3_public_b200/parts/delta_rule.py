@@ -35,6 +35,7 @@ import torch
 
 from ..ops import functional as F
 from ..ops.linear import linear
+from ..ops.library import one_layer
 from .base import Mixer, ProjectedMixer, StateRequest, StepContext, TensorSpec, register_part
 
 _NAMES = {"q": "q", "k": "k", "v": "v", "q_conv": "q.conv", "k_conv": "k.conv", "v_conv": "v.conv", "b": "b", "a_log": "A_log",
@@ -112,6 +113,7 @@ class ChannelDeltaRule(Mixer):
             requests.append(StateRequest((self.taps - 1, self.channels), torch.float32))
         return requests
 
+    @one_layer
     def forward(self, x, ctx: StepContext, cache) -> torch.Tensor:
         if ctx.extras.get("cache_read_only", False):
             raise ValueError("a recurrent mixer advances its state at every step: it cannot run on another entry's storage")

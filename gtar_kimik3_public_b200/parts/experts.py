@@ -31,6 +31,7 @@ import torch
 
 from ..ops import functional as F
 from ..ops.linear import grouped_product_ok, linear, linear_grouped
+from ..ops.library import one_layer
 from .base import FeedForward, StepContext, TensorSpec, register_part
 
 
@@ -115,6 +116,7 @@ class RoutedExperts(FeedForward):
                               renormalise=self.renormalise,
                               shared=("pair" if self.shared_as_expert else "weight") if self.shared_gate else None)
 
+    @one_layer
     def forward_added(self, x: torch.Tensor, ctx: StepContext, add: torch.Tensor | None) -> torch.Tensor:
         """``add + experts(x)`` as one 32-bit sum (``add``: another branch's output for the same tokens, or None)."""
         add_weight = None

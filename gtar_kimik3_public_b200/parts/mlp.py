@@ -9,6 +9,7 @@ import torch
 
 from ..ops import functional as F
 from ..ops.linear import linear, linear_normed, linear_on_stream_ok, linear_residual
+from ..ops.library import one_layer
 from .base import FeedForward, StepContext, TensorSpec, register_part
 
 
@@ -41,6 +42,7 @@ class SwiGLUFeedForward(FeedForward):
         return {"kind": "swiglu", "hidden": self.hidden_size, "inter": self.intermediate_size, "w_gu": self.w_gate_up,
                 "w_down": self.w_down}
 
+    @one_layer
     def forward(self, x, ctx: StepContext) -> torch.Tensor:
         return linear(linear(x, self.w_gate_up, swiglu=True), self.w_down)
 
