@@ -110,21 +110,62 @@ __device__ __forceinline__ void scan_slice(const float* __restrict__ row, int be
     for (int i = vec_begin + 4 * n_vec + threadIdx.x; i < end; i += blockDim.x) visit(row[i], i);
 }
 
+// What a scan of the whole slice leaves for one of its few large elements: the largest key of each thread's turns of sixteen
+// elements, `per` turns together, [MARKS][blockDim.x] in shared memory.
+constexpr int MARKS = 8;
+__device__ __forceinline__ int turns_a_mark(int n_vec) { return (n_vec + (int)blockDim.x * 4 * MARKS - 1) / ((int)blockDim.x * 4 * MARKS); }
+
+// The largest key among the thread's elements of row[begin .. end), and of each group of its turns.
+__device__ __forceinline__ unsigned int scan_largest(const float* __restrict__ row, int begin, int end, unsigned int* marks) {
+    const int lead = min((int)((16 - ((uintptr_t)(row + begin) & 15)) & 15) / 4, max(end - begin, 0));
+    const int vec_begin = begin + lead, n_vec = max(end - vec_begin, 0) / 4, rest = vec_begin + 4 * n_vec, per = turns_a_mark(n_vec);
+    const float4* vec = reinterpret_cast<const float4*>(row + vec_begin);
+    unsigned int largest = 0, group = 0;
+    if ((int)threadIdx.x < lead) largest = float_key(row[begin + threadIdx.x]);
+    if ((int)threadIdx.x < end - rest) largest = max(largest, float_key(row[rest + threadIdx.x]));
+    int left = per;
+    unsigned int* mark = marks + threadIdx.x;
+    for (int v0 = threadIdx.x; v0 < n_vec; v0 += blockDim.x * 4) {
+        float4 got[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int v = v0 + u * (int)blockDim.x;
+            if (v < n_vec) got[u] = vec[v];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (v0 + u * (int)blockDim.x < n_vec)
+                group = max(group, max(max(float_key(got[u].x), float_key(got[u].y)), max(float_key(got[u].z), float_key(got[u].w))));
+        if (--left == 0) {
+            *mark = group;
+            mark += blockDim.x;
+            largest = max(largest, group);
+            group = 0, left = per;
+        }
+    }
+    if (left != per) *mark = group;
+    return max(largest, group);
+}
+
 // The same for the elements whose key reaches `least`, of which there are few: what is done with one stands in the code once and
-// fetches it again, instead of sixteen times behind the loads.
+// fetches it again, instead of sixteen times behind the loads.  With `marks` (scan_largest's) only the turns among which there is one
+// are fetched.
 template <typename Visit>
-__device__ __forceinline__ void scan_reaching(const float* __restrict__ row, int begin, int end, unsigned int least, Visit visit) {
+__device__ __forceinline__ void scan_reaching(const float* __restrict__ row, int begin, int end, unsigned int least, Visit visit, const unsigned int* marks = nullptr) {
     const int lead = min((int)((16 - ((uintptr_t)(row + begin) & 15)) & 15) / 4, max(end - begin, 0));
     const int vec_begin = begin + lead, n_vec = max(end - vec_begin, 0) / 4, rest = vec_begin + 4 * n_vec;
     const float4* vec = reinterpret_cast<const float4*>(row + vec_begin);
     const float least_value = key_float(least);
     const auto maybe = [&](float x) { return !(x < least_value); };  // true for all that reach it, for a zero of the other sign and for NaN
     constexpr int IN_FLIGHT = 4;
+    const int per = marks != nullptr ? turns_a_mark(n_vec) : 0;
+    int turn = 0;
     // the last turn of all threads is for the elements beside the whole pieces: at most three in front and three behind
-    for (int v0 = threadIdx.x;; v0 += blockDim.x * IN_FLIGHT) {
+    for (int v0 = threadIdx.x;; v0 += blockDim.x * IN_FLIGHT, ++turn) {
         unsigned int hits = 0;
         int first = vec_begin + 4 * v0, step = 4 * (int)blockDim.x;
         const bool last = v0 >= n_vec;
+        if (marks != nullptr && !last && marks[turn / per * (int)blockDim.x + (int)threadIdx.x] < least) continue;
         if (!last) {
             float4 got[IN_FLIGHT];
 #pragma unroll
@@ -395,8 +436,9 @@ __global__ void __launch_bounds__(SELECT_THREADS, 3) sample_top_k_kernel(
     __shared__ SelectShared sh;
     __shared__ Best scratch[32], block_result;
     __shared__ __align__(16) unsigned int keys[CANDIDATES];  // first the groups' largest keys, then the candidates' keys
-    __shared__ unsigned int own_keys[MAX_KEYS], enough[2][16], in_front[MAX_KEYS], bounds[2], n_above;
+    __shared__ unsigned int own_keys[MAX_KEYS], enough[2][16], in_front[MAX_KEYS], bounds[2], n_above, counts[SELECT_BLOCKS];
     __shared__ CandidateList list;
+    __shared__ unsigned int marks[MARKS * SELECT_THREADS];
     pdl_launch_dependents();
     pdl_wait();
     uint32_t n_ranks_raw;
@@ -416,8 +458,7 @@ __global__ void __launch_bounds__(SELECT_THREADS, 3) sample_top_k_kernel(
     if (2 * top_k <= n_ranks * groups) {  // so it is for every top_k that comes here, up to half of MAX_KEYS
         if (threadIdx.x == 0) list.count = 0, n_above = 0, bounds[0] = bounds[1] = 0xffffffffu;
         in_front[threadIdx.x] = 0;
-        unsigned int largest = 0;  // below every key but that of the NaN of all ones
-        scan_slice(row, begin, end, [&](float x, int) { largest = max(largest, float_key(x)); });
+        unsigned int largest = scan_largest(row, begin, end, marks);
         for (int o = 1; o < lanes; o <<= 1) largest = max(largest, __shfl_xor_sync(0xffffffffu, largest, o));
         if (threadIdx.x % lanes == 0) own_keys[threadIdx.x / lanes] = largest;
         cluster_barrier();
@@ -433,30 +474,31 @@ __global__ void __launch_bounds__(SELECT_THREADS, 3) sample_top_k_kernel(
             reach = 0xffffffffu;
             for (int b = 0; b < n_ranks; ++b) reach = min(reach, remote_read(&bounds[0], b));
         }
-        const uint32_t first_list = remote_address(&list, 0);
+        // into the block's own list: a request of another SM for every few of them would be most of this scan
         bool full = false;
         unsigned int above = 0;
         scan_reaching(row, begin, end, reach, [&](float x, int i) {
             above += float_key(x) > reach;
             if (full) return;
-            // one request for all lanes that stand here together
-            const unsigned int here = __activemask(), leader = __ffs(here) - 1, lane = threadIdx.x & 31;
-            unsigned int at;
-            if (lane == leader) asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at) : "r"(first_list + (uint32_t)offsetof(CandidateList, count)), "r"(__popc(here)) : "memory");
-            at = __shfl_sync(here, at, leader) + __popc(here & ((1u << lane) - 1));
-            if (at < CANDIDATES) {
-                asm volatile("st.shared::cluster.v2.b32 [%0], {%1, %2};" ::"r"(first_list + 8 * at), "r"(__float_as_uint(x)), "r"(i) : "memory");
-            } else {
-                full = true;
-            }
-        });
+            const unsigned int at = atomicAdd(&list.count, 1u);
+            if (at < CANDIDATES) list.entries[at] = make_int2(__float_as_int(x), i);
+            else full = true;
+        }, marks);
         for (int o = 1; o < 32; o <<= 1) above += __shfl_xor_sync(0xffffffffu, above, o);
         if ((threadIdx.x & 31) == 0) atomicAdd(&n_above, above);
         cluster_barrier();
-        const int n = (int)remote_read(&list.count, 0);
+        if ((int)threadIdx.x < n_ranks) counts[threadIdx.x] = remote_read(&list.count, threadIdx.x);
+        __syncthreads();
+        int n = 0;
+        for (int b = 0; b < n_ranks; ++b) n += (int)counts[b];
         settled = n <= CANDIDATES;
-        if (settled && rank == 0) {
-            for (int i = threadIdx.x; i < n; i += SELECT_THREADS) keys[i] = float_key(__int_as_float(list.entries[i].x));
+        if (settled && rank == 0) {  // the others' lists behind this block's own
+            for (int i = threadIdx.x; i < n; i += SELECT_THREADS) {
+                int b = 0, at = i;
+                while (at >= (int)counts[b]) at -= (int)counts[b++];
+                if (b > 0) list.entries[i] = make_int2((int)remote_read(&list.entries[at].x, b), (int)remote_read(&list.entries[at].y, b));
+                keys[i] = float_key(__int_as_float(list.entries[i].x));
+            }
             __syncthreads();
             const unsigned int kth = n <= MAX_KEYS ? least_of_first(keys, n, top_k, 0, n, in_front, &bounds[1]) : kth_of_many(keys, n, top_k, enough);
             const Draw draw = key_of_row();
