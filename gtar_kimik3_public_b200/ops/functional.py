@@ -745,6 +745,42 @@ def attention_decode_fused(
     return out
 
 
+def attention_decode_layer(x: torch.Tensor, w_qkv: torch.Tensor, w_o: torch.Tensor, n_q: int, n_kv: int, head_dim: int,
+                           q_weight: torch.Tensor | None, k_weight: torch.Tensor | None, eps: float, cos: torch.Tensor | None,
+                           sin: torch.Tensor | None, kv: PagedKV, kv_len: torch.Tensor, slots: torch.Tensor, max_position: int, scale: float,
+                           window: int, n_splits: int, write_kv: bool) -> torch.Tensor:
+    """``gemv(attention_decode_fused(gemv(x, w_qkv), ...), w_o)`` as one call into the library: the same three kernels."""
+    require_device(x.device)
+    for name, t, dims in (("x", x, 2), ("w_qkv", w_qkv, 2), ("w_o", w_o, 2), ("k pages", kv.k, 4), ("v pages", kv.v, 4)):
+        _check(t, name, torch.bfloat16, dims)
+    _check(kv_len, "kv_len", torch.int32, 1)
+    _check(slots, "slots", torch.int32, 1)
+    n, hidden = x.shape
+    if w_qkv.shape != ((n_q + 2 * n_kv) * head_dim, hidden) or w_o.shape[1] != n_q * head_dim or n > GEMV_MAX_TOKENS_SHORT_K:
+        raise KernelError(f"x is {tuple(x.shape)} but the weights are {tuple(w_qkv.shape)} and {tuple(w_o.shape)}")
+    if kv.k.shape[1] != n_kv or kv.k.shape[3] != head_dim:
+        raise KernelError(f"pages {tuple(kv.k.shape)} do not fit n_kv={n_kv}, head_dim={head_dim}")
+    weight_code = 0
+    if q_weight is not None:
+        _check(q_weight, "q_weight", dims=1)
+        _check(k_weight, "k_weight", q_weight.dtype, 1)
+        weight_code = dtype_code(q_weight.dtype)
+    table_positions = 0
+    if cos is not None:
+        _check(cos, "cos", torch.float32, 2)
+        _check(sin, "sin", torch.float32, 2)
+        if cos.shape[1] != head_dim // 2 or sin.shape != cos.shape:
+            raise KernelError("rotary tables must be [positions, head_dim / 2]")
+        table_positions = cos.shape[0]
+    scratch = torch.empty((n * 2 * (n_q + n_kv) * head_dim,), dtype=torch.bfloat16, device=x.device)
+    out = torch.empty((n, w_o.shape[0]), dtype=torch.bfloat16, device=x.device)
+    call("gk_attention_decode_layer_bf16", ptr(x), n, hidden, ptr(w_qkv), ptr(w_o), w_o.shape[0], ptr(scratch), ptr(out), ptr(q_weight), ptr(k_weight),
+         weight_code, int(q_weight is not None), float(eps), ptr(cos), ptr(sin), table_positions, int(max_position), int(write_kv), ptr(kv.k), ptr(kv.v),
+         ptr(kv_len), ptr(slots), ptr(kv.block_table), n_q, n_kv, head_dim, kv.max_pages, kv.page_size, float(scale), int(window), int(n_splits),
+         stream_ptr())
+    return out
+
+
 @functools.lru_cache(maxsize=None)
 def decode_flat_places(head_dim: int, sm_count: int) -> int:
     """How many blocks of the evenly dealt decode attention kernel the device holds at once: the most pieces that

@@ -87,8 +87,26 @@ class GQAAttention(Mixer):
                               ctx.max_position, write_kv)
             o = attention_ops.paged_attention(q, cache, ctx, self.scale, self.window or 0)
             return linear(o.view(ctx.n_tokens, self.n_q * self.head_dim), self.w_o)
+        splits = self._decode_layer_splits(x, ctx, cache)
+        if splits:
+            return F.attention_decode_layer(x, self.w_qkv, self.w_o, self.n_q, self.n_kv, self.head_dim, self.q_norm, self.k_norm, self.qk_norm_eps or 1.0,
+                                            cos, sin, cache, ctx.kv_len, ctx.slots, ctx.max_position, self.scale, self.window or 0, splits, write_kv)
         o = self._attend(linear(x, self.w_qkv), ctx, cache, cos, sin, write_kv)
         return linear(o.view(ctx.n_tokens, self.n_q * self.head_dim), self.w_o)
+
+    def _decode_layer_splits(self, x: torch.Tensor, ctx: StepContext, cache) -> int:
+        """How many blocks share a sequence where the step is the one that ``_attend`` between two few-token products would take through
+        its kernel with norm, rotation and cache write inside, so that the layer is one call; 0 where it is not."""
+        w_qkv, w_o = self.w_qkv, self.w_o
+        if not (ctx.all_single and x.dtype == torch.bfloat16 and w_qkv.dtype == torch.bfloat16 and w_o.dtype == torch.bfloat16
+                and isinstance(cache, F.PagedKV) and attention_ops.fused_decode_ok(x, cache, self.n_q, self.n_kv, self.head_dim)):
+            return 0
+        m, hidden = x.shape
+        if (hidden % 8 or (x.data_ptr() | w_qkv.data_ptr() | w_o.data_ptr()) % 16 or not F.gemv_suits(m, w_qkv.shape[0], hidden, x.device)
+                or not F.gemv_suits(m, w_o.shape[0], w_o.shape[1], x.device) or attention_ops.decode_flat_preferred(ctx, self.n_kv, cache)):
+            return 0
+        splits = attention_ops.decode_split_count(ctx, self.n_kv, cache)
+        return splits if splits <= 8 else 0
 
     def on_stream_ok(self, h: torch.Tensor, norm_weight, ctx: StepContext, cache) -> bool:
         """Whether ``forward_on_stream`` takes this step: a few tokens, one each, bfloat16 matrices of sizes the
