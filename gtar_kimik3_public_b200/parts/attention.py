@@ -96,9 +96,10 @@ class GQAAttention(Mixer):
 
     def _decode_layer_splits(self, x: torch.Tensor, ctx: StepContext, cache) -> int:
         """How many blocks share a sequence where the step is the one that ``_attend`` between two few-token products would take through
-        its kernel with norm, rotation and cache write inside, so that the layer is one call; 0 where it is not."""
+        its kernel with norm, rotation and cache write inside, so that the layer is one call; 0 where it is not.  A step that is run for
+        its capture (its launches are sized for a range of lengths) pays the host's part once and goes call by call."""
         w_qkv, w_o = self.w_qkv, self.w_o
-        if not (ctx.all_single and x.dtype == torch.bfloat16 and w_qkv.dtype == torch.bfloat16 and w_o.dtype == torch.bfloat16
+        if not (ctx.all_single and not ctx.typical_kv_len and x.dtype == torch.bfloat16 and w_qkv.dtype == torch.bfloat16 and w_o.dtype == torch.bfloat16
                 and isinstance(cache, F.PagedKV) and attention_ops.fused_decode_ok(x, cache, self.n_q, self.n_kv, self.head_dim)):
             return 0
         m, hidden = x.shape
