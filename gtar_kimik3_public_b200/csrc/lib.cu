@@ -50,6 +50,13 @@ GK_EXPORT int gk_chain(int on) {
     return before;
 }
 
+// `bytes` from pinned host memory to the device, in stream order.
+GK_EXPORT int gk_copy_to_device(void* dst, const void* src, long long bytes, void* stream) {
+    const cudaError_t err = cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyHostToDevice, (cudaStream_t)stream);
+    if (err != cudaSuccess) return gk_fail(GK_CUDA_ERROR, "copy_to_device: %s", cudaGetErrorString(err));
+    return GK_OK;
+}
+
 GK_EXPORT const char* gk_last_error() { return g_last_error; }
 
 // Interface revision: the Python side refuses a library built from other sources.

@@ -103,15 +103,18 @@ class Engine:
         q_lens = [len(e.tokens) for e in entries]
         if min(q_lens) == 0:
             raise ValueError(f"request {entries[q_lens.index(0)].id!r} brings no token")
-        parts = [_token_array(e.tokens) for e in entries]
-        if any(part.ndim != 1 for part in parts):
-            raise ValueError("tokens must be a flat list of ids")
-        flat = parts[0] if len(parts) == 1 else np.concatenate(parts)
-        if flat.min() < 0 or flat.max() >= vocab:
-            for entry, part in zip(entries, parts):
-                wrong = part[(part < 0) | (part >= vocab)]
-                if wrong.size:
-                    raise ValueError(f"request {entry.id!r}: token id {int(wrong[0])} is outside the vocabulary of {vocab}")
+        if all([n == 1 and type(e.tokens) is list and type(e.tokens[0]) is int and 0 <= e.tokens[0] < vocab for n, e in zip(q_lens, entries)]):
+            parts = [e.tokens for e in entries]  # a decode step of plain numbers: nothing to convert, and looked at already
+        else:
+            parts = [_token_array(e.tokens) for e in entries]
+            if any(part.ndim != 1 for part in parts):
+                raise ValueError("tokens must be a flat list of ids")
+            flat = parts[0] if len(parts) == 1 else np.concatenate(parts)
+            if flat.min() < 0 or flat.max() >= vocab:
+                for entry, part in zip(entries, parts):
+                    wrong = part[(part < 0) | (part >= vocab)]
+                    if wrong.size:
+                        raise ValueError(f"request {entry.id!r}: token id {int(wrong[0])} is outside the vocabulary of {vocab}")
         for entry, n in zip(entries, q_lens):
             for place in entry.want:
                 if not 0 <= int(place) < n:
@@ -144,8 +147,9 @@ class Engine:
         self.steps_run += 1
         if self.graphs is not None:
             packed = pack_step(sequences, vocab, check_tokens=False)
-            if packed.n_want > 0 and self.graphs.wants_graph(packed):
-                logits = self.graphs.run(packed)
+            key = self.graphs.key_of(packed)
+            if packed.n_want > 0 and self.graphs.wants_graph(packed, key):
+                logits = self.graphs.run(packed, key=key)
                 return logits.clone() if keep_output else logits
         ctx = plan_step(sequences, self.model.dtype, self.model.device, vocab)
         return self.model.step(ctx, self.cache)

@@ -34,7 +34,8 @@ from collections import OrderedDict
 import numpy as np
 import torch
 
-from ..ops.functional import set_pdl
+from ..ops import library
+from ..ops.functional import copy_to_device, set_pdl
 from .step import PackedStep, context_from_views
 
 
@@ -80,17 +81,16 @@ class StepGraphs:
         overwritten by the host."""
         turn = self.turn
         self.turn = (turn + 1) % self.RING
-        if self.events[turn] is not None:
-            self.events[turn].synchronize()
-        buf, pinned = self.host_np[turn], self.host[turn]
-        offsets = self.offsets(packed)
-        for offset, field in zip(offsets, packed.fields):
-            buf[offset:offset + len(field)] = field
-        begin = offsets[1] if skip_tokens else 0  # the token ids come from the device in that case
-        self.meta[begin:offsets[-1]].copy_(pinned[begin:offsets[-1]], non_blocking=True)
-        event = torch.cuda.Event()
+        event = self.events[turn]
+        if event is None:
+            event = self.events[turn] = torch.cuda.Event()
+        else:
+            event.synchronize()
+        total = sum(map(len, packed.fields))
+        np.concatenate(packed.fields, out=self.host_np[turn][:total])
+        begin = packed.n_tokens if skip_tokens else 0  # the token ids come from the device in that case
+        copy_to_device(self.meta, self.host[turn], begin, total)
         event.record()
-        self.events[turn] = event
 
     # ------------------------------------------------------------------ graphs
     def length_bounds(self, packed: PackedStep) -> tuple[int, int]:
@@ -114,9 +114,9 @@ class StepGraphs:
             return (packed.n_tokens, packed.n_seqs, packed.n_want, 1, self.length_bound(packed))
         return (packed.n_tokens, packed.n_seqs, packed.n_want, packed.max_q_len, 0)
 
-    def wants_graph(self, packed: PackedStep) -> bool:
+    def wants_graph(self, packed: PackedStep, key: tuple | None = None) -> bool:
         """Decode shapes always; other shapes from their second appearance on."""
-        key = self.key_of(packed)
+        key = key or self.key_of(packed)
         if key in self.graphs or packed.all_single:
             return True
         if key in self.seen:
@@ -126,10 +126,10 @@ class StepGraphs:
             self.seen.clear()
         return False
 
-    def run(self, packed: PackedStep, device_tokens: torch.Tensor | None = None) -> torch.Tensor:
+    def run(self, packed: PackedStep, device_tokens: torch.Tensor | None = None, key: tuple | None = None) -> torch.Tensor:
         """Logits ``[n_want, vocab]``.  The returned tensor is the graph's own output buffer: the next
         replay of the same shape overwrites it."""
-        key = self.key_of(packed)
+        key = key or self.key_of(packed)
         self.upload(packed, skip_tokens=device_tokens is not None)
         if device_tokens is not None:
             self.meta[0:packed.n_tokens].copy_(device_tokens)
@@ -138,16 +138,12 @@ class StepGraphs:
         self.graphs.move_to_end(key)
         graph, logits = self.graphs[key]
         graph.replay()
-        from ..ops import library
-
         library.launch_count += self.launches[key]
         return logits
 
     def _capture(self, key: tuple, packed: PackedStep) -> torch.Tensor:
         """Runs the step launch by launch, captures its launches for the steps to come, and returns the
         logits of the run (the capture itself executes nothing, so the step has run once)."""
-        from ..ops import library
-
         self.model.prepare(self.cache.max_seq_len - 1)
         # launch shapes inside a graph must not depend on the lengths of the day: a bound stands in
         bound, typical = self.length_bounds(packed)

@@ -100,7 +100,7 @@ def pack_step(sequences: list[SequenceStep], vocab_size: int, check_tokens: bool
             want_rows.append(int(starts[index]) + place)
     slots = [s.slot for s in sequences]
     fields = [
-        tokens.astype(np.int32), tok_pos.astype(np.int32), tok_seq, starts, np.asarray(slots, dtype=np.int32),
+        tokens.astype(np.int32), tok_pos.astype(np.int32, copy=False), tok_seq, starts, np.asarray(slots, dtype=np.int32),
         past_np + np.asarray(q_lens, dtype=np.int32), np.asarray(want_rows, dtype=np.int32),
     ]
     return PackedStep(fields, q_lens, past, slots)

@@ -390,6 +390,15 @@ def split_k_for(m: int, n: int, k: int) -> int:
     return 8 if limit >= 8 else 4 if limit >= 4 else 2 if limit >= 2 else 1
 
 
+def copy_to_device(device_ints: torch.Tensor, pinned_ints: torch.Tensor, begin: int, end: int) -> None:
+    """``device_ints[begin:end] = pinned_ints[begin:end]`` in stream order without waiting (int32, the host side in pinned memory that
+    stays as it is until the copy has run): the copy alone, where slicing both sides costs more than it."""
+    if not (0 <= begin <= end <= min(device_ints.numel(), pinned_ints.numel())):
+        raise KernelError(f"copy of {begin} to {end} does not fit {device_ints.numel()} and {pinned_ints.numel()} numbers")
+    if begin < end and library().gk_copy_to_device(device_ints.data_ptr() + 4 * begin, pinned_ints.data_ptr() + 4 * begin, 4 * (end - begin), stream_ptr()):
+        raise KernelError(library().gk_last_error().decode(errors="replace"))  # (no kernel: not among the launches that `call` counts)
+
+
 def set_pdl(on: bool) -> bool:
     """Switches programmatic dependent launch for all later kernel launches; returns the old setting."""
     from .library import library

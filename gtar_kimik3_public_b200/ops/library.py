@@ -54,6 +54,7 @@ _SIGNATURES: dict[str, list] = {
     "gk_gemv_bf16_stream": [P, I, I, L, P, I, L, P, I, I, P, L, P, I, F, P, L, P],
     "gk_set_pdl": [I],
     "gk_chain": [I],
+    "gk_copy_to_device": [P, P, L, P],
     "gk_attention_decode_resident_clusters": [I, I],
     "gk_set_gemm_pairs": [I],
     "gk_set_attention_prefill_keys": [I],
