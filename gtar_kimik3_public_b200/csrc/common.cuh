@@ -88,7 +88,8 @@ inline cudaError_t gk_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 
 // For the second and later kernels of one call of this library: the kernel in front is the call's own, which waits for what is in
 // front of it, and this one touches no memory before pdl_wait(); so it may take its place on the SMs early whatever the switch says.
-// (A gap of some 1.5 us between two kernels launched one by one.)
+// (What it saves where kernels are launched one by one: two products of a feed-forward, which start early in the same way, take 33.2 us
+// instead of 36.9.)
 template <typename... KArgs, typename... Args>
 inline cudaError_t gk_launch_behind(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     return gk_launch_with(true, kernel, grid, block, smem, stream, dim3(1, 1, 1), args...);
