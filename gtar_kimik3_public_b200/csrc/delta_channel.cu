@@ -19,16 +19,21 @@
 //   walk    a block per head and 8 value columns, the chunks in sequence: 128 x 8 numbers of state in the accumulators of eight warps
 //   read    a block per chunk and head: o, RMS norm over a head, weight and gate
 //
-// Every matrix product takes 32-bit operands: each number is split into two TF32 numbers (rounded, and the rounded rest), three
-// mma.sync a product, what is left out is 2^-24 of it; the large parts are added up by 32-bit additions outside the tensor core,
-// whose own sums are cut and not rounded (H. Ootomo, R. Yokota, "Recovering single precision accuracy from Tensor Cores while
-// surpassing the FP32 theoretical peak performance").  FFMA instead would be bound by what shared memory can deliver.
+// Every matrix product takes 32-bit operands: each number is split into three bfloat16 numbers whose sum it is, six mma.sync a product
+// (G. Henry, P. T. P. Tang, A. Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations");
+// what is left out is at most 2^-24 of a product, 2^-27.5 root mean square.  The large parts are added up by 32-bit additions outside the
+// tensor core, whose own sums are cut and not rounded (H. Ootomo, R. Yokota, "Recovering single precision accuracy from Tensor Cores while
+// surpassing the FP32 theoretical peak performance"); of their products of 16 bits little is cut.  FFMA instead would be bound by what
+// shared memory can deliver.
 //
-// Measured (us, the kernels that go token by token / here; heads of 128): one prompt of 2,048, 8 heads: 620 / 137; 1,024 + 500 + 77
-// tokens, 16 heads: 537 / 283; 100 + 40 + 900, 8 heads: 305 / 126; 32 prompts of 40: 154 / 136.  Error of the states against 64 bits,
-// relative: 4.07e-7 / 4.09e-7 at the first, 3.15e-7 / 3.31e-7 at the second, 1.6e-7 / 2.0e-7 after 16 tokens; of the bfloat16 read-outs
-// 1.66e-3 both ways.  `inner` is bound by latency (some 50 us of the 137: its phases follow one another, two blocks an SM), `walk` by its two products and
-// three barriers a chunk (1.5 us).
+// Error of the states against 64 bits, relative, the kernels that go token by token / here (heads of 128; activations and decays are formed
+// alike): one prompt of 2,048, 8 heads: 5.35e-7 / 5.15e-7; 1,024 + 500 + 77, 16 heads: 4.76e-7 / 4.62e-7; 192 after a state: 2.78e-7 / 2.70e-7;
+// smaller in each of 20 drawn steps of 33 to 1,100 tokens, by 3 to 10%; of the bfloat16 read-outs 1.66e-3 both ways.  Where decays leave
+// hardly anything of the token before (e^-2.7 a token) u has one rounding more: 1.20e-7 / 1.26e-7.  (Two TF32 numbers and three products, the same number
+// of instructions: 137 us instead of 146 at the first, but 2.93e-7 at the third.)
+// Measured (us, token by token / here): 2,048 tokens, 8 heads: 620 / 146; 1,024 + 500 + 77, 16 heads: 539 / 295; 512 + 300, 8 heads: 179 / 94.
+// `inner` is bound by latency (some 50 us of the 146: its phases follow one another, two blocks an SM), `walk` by its two products and three
+// barriers a chunk (1.5 us).
 
 #include "common.cuh"
 
@@ -54,15 +59,10 @@ struct Unit {
     static constexpr int SIZE = S + D * D;
 };
 
-// Quotients without the branch that a rounded division carries for numbers out of range, so that a thread's many are worked out side by side
-__device__ __forceinline__ float silu_f(float z) { return __fdividef(z, 1.f + expf(fminf(-z, 80.f))); }
-__device__ __forceinline__ float sigmoid_f(float z) { return __fdividef(1.f, 1.f + expf(fminf(-z, 80.f))); }
-// log(1 + e^z) = max(z, 0) + log(1 + u), u = e^-|z|; with w = 1 + u as rounded, log(1 + u) = log(w) u / (w - 1) to a few last places (D.
-// Goldberg, "What Every Computer Scientist Should Know About Floating-Point Arithmetic", theorem 4).
-__device__ __forceinline__ float softplus_f(float z) {
-    const float u = expf(-fabsf(z)), w = 1.f + u;
-    return fmaxf(z, 0.f) + (w == 1.f ? u : logf(w) * __fdividef(u, w - 1.f));
-}
+// As in the kernels that go token by token
+__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
+__device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -74,36 +74,59 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// To the nearest number of ten fraction bits, ties away from zero.  (The conversion instruction does the same at an eighth of the rate of
-// these two.)
-__device__ __forceinline__ uint32_t tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
-__device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
-    hi = tf32(x);
-    lo = tf32(x - __uint_as_float(hi));
+// Two 32-bit numbers as three pairs of bfloat16 numbers: the nearest one, the nearest one to the rest, and what then remains, which is one.
+__device__ __forceinline__ uint32_t bf16_pair(float x, float y) {
+    uint32_t d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(y), "f"(x));
+    return d;
 }
-__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+__device__ __forceinline__ void split(float x, float y, uint32_t (&part)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        part[i] = bf16_pair(x, y);
+        x -= __uint_as_float(part[i] << 16);
+        y -= __uint_as_float(part[i] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ void mma(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
 // the same with nothing to add to
-__device__ __forceinline__ void mma_alone(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+__device__ __forceinline__ void mma_alone(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
 }
 
-// Left operand, 16 x 8: lane 4 r + c holds rows r, r + 8 of two columns, in the order (r, first), (r + 8, first), (r, second),
-// (r + 8, second).  Which two columns is free as long as the right operand's two rows are the same ones: 2c and 2c + 1 where an
-// accumulator becomes an operand (no exchange between lanes), c and c + 4 where rows lie four banks apart.
+// Left operand, two pieces of 16 x 8: of a piece lane 4 r + c holds rows r, r + 8 of two columns, in the order (r, first), (r + 8, first), (r,
+// second), (r + 8, second).  Which two columns is free as long as the right operand's two rows are the same ones: 2c and 2c + 1 where an
+// accumulator becomes an operand (no exchange between lanes), c and c + 4 where rows lie four banks apart.  The instruction's pairs of
+// columns are one of each piece, so that where a thread has rows r and r + 8 of a right operand they are a pair.
 struct Left {
-    uint32_t hi[4], lo[4];
-    __device__ __forceinline__ Left(float a, float b, float c, float d) {
-        split(a, hi[0], lo[0]);
-        split(b, hi[1], lo[1]);
-        split(c, hi[2], lo[2]);
-        split(d, hi[3], lo[3]);
+    uint32_t part[3][4];
+    __device__ __forceinline__ Left(const float4& a, const float4& b) {
+        const float x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t p[3];
+            split(x[i], y[i], p);
+            part[0][i] = p[0], part[1][i] = p[1], part[2][i] = p[2];
+        }
+    }
+};
+struct Right {
+    uint32_t part[3][2];
+    __device__ __forceinline__ Right() {}
+    // the two rows of the first piece, then those of the second
+    __device__ __forceinline__ Right(float a0, float a1, float b0, float b1) {
+        uint32_t p[3], q[3];
+        split(a0, b0, p);
+        split(a1, b1, q);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) part[i][0] = p[i], part[i][1] = q[i];
     }
 };
 // CHAINS: of the small parts' products, which the tensor core adds up itself, one after another
@@ -118,19 +141,16 @@ struct SumOf {
             for (int j = 0; j < CHAINS; ++j) low[j][i] = 0.f;
         }
     }
-    __device__ __forceinline__ void add(const Left& a, uint32_t h0, uint32_t h1, uint32_t l0, uint32_t l1) {
+    __device__ __forceinline__ void add(const Left& a, const Right& b) {
         float c[4];
-        mma_alone(c, a.hi, h0, h1);
-        mma(low[0], a.lo, h0, h1);
-        mma(low[CHAINS - 1], a.hi, l0, l1);
+        mma_alone(c, a.part[0], b.part[0]);
+        mma(low[0], a.part[0], b.part[1]);
+        mma(low[CHAINS - 1], a.part[1], b.part[0]);
+        mma(low[0], a.part[0], b.part[2]);
+        mma(low[CHAINS - 1], a.part[2], b.part[0]);
+        mma(low[0], a.part[1], b.part[1]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[i] += c[i];
-    }
-    __device__ __forceinline__ void add(const Left& a, float b0, float b1) {
-        uint32_t h0, h1, l0, l1;
-        split(b0, h0, l0);
-        split(b1, h1, l1);
-        add(a, h0, h1, l0, l1);
     }
     __device__ __forceinline__ float at(int i) const { return acc[i] + (CHAINS > 1 ? low[0][i] + low[CHAINS - 1][i] : low[0][i]); }
 };
@@ -241,7 +261,7 @@ template <int D>
 struct InnerSmem {
     static constexpr int LD = D + 4;  // rows four banks apart
     float k[CHUNK][LD], g[CHUNK][LD], q[CHUNK][LD];
-    float blk[10][TILE16];            // (1 + A)^-1 of the four blocks on the diagonal, then the six of A below it
+    float blk[10][TILE16];            // (1 + A)^-1 - 1 of the four blocks on the diagonal, then the six of A below it
     float total[5][D];                // decays over a block, and ones
     float beta[CHUNK];
 };
@@ -381,7 +401,7 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
         __syncwarp();
         if (lane < SUB)
 #pragma unroll
-            for (int i = 0; i < SUB; ++i) A[at16(i, lane)] = x[i];
+            for (int i = 0; i < SUB; ++i) A[at16(i, lane)] = i == lane ? 0.f : x[i];  // the ones on the diagonal are added where it is used
     } else {  // decays from a block's start into keys and queries, and keys with the decays to the block's end in the place of the decays
         for (int item = tid - 128; item < 4 * D; item += 128) {
             const int c = item % D, b = item / D;
@@ -418,11 +438,10 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
         const float* b = &sm.g[J * SUB + nt * 8 + r][0] + c2;
         const float *f1 = sm.total[I - J > 1 ? J + 1 : 4] + c2, *f2 = sm.total[I - J > 2 ? J + 2 : 4] + c2;  // the blocks between
         SumOf<2> s;
-#pragma unroll 4
-        for (int ks = 0; ks < KS; ++ks) {
-            const float b0 = b[8 * ks] * f1[8 * ks] * f2[8 * ks], b1 = b[8 * ks + 4] * f1[8 * ks + 4] * f2[8 * ks + 4];
-            s.add(Left(a[8 * ks], a[8 * ks + 8 * LD], a[8 * ks + 4], a[8 * ks + 8 * LD + 4]), b0, b1);
-        }
+        const auto left = [&](int c) { return make_float4(a[c], a[c + 8 * LD], a[c + 4], a[c + 8 * LD + 4]); };
+        const auto right = [&](int c) { return b[c] * f1[c] * f2[c]; };
+#pragma unroll 2
+        for (int c = 0; c < D; c += 16) s.add(Left(left(c), left(c + 8)), Right(right(c), right(c + 4), right(c + 8), right(c + 12)));
         if (queries) {
             reinterpret_cast<float4*>(mine + Unit<D>::P)[(I * 8 + J * 2 + nt) * 32 + lane] = make_float4(s.at(0), s.at(2), s.at(1), s.at(3));
         } else {
@@ -464,23 +483,23 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
         const float* src = part == 0 ? &sm.k[0][0] : mine + Unit<D>::U;
         const int ld_src = part == 0 ? LD : dv;
         float pre[2] = {1.f, 1.f}, x[8][4];
+        const auto turned = [](const float(&a)[4], const float(&b)[4]) { return Left(make_float4(a[0], a[2], a[1], a[3]), make_float4(b[0], b[2], b[1], b[3])); };
+        const auto block = [&](int which, int nt) {
+            const float2 a = *reinterpret_cast<const float2*>(&sm.blk[which][at16(nt * 8 + r, 2 * c2)]);
+            const float2 b = *reinterpret_cast<const float2*>(&sm.blk[which][at16(nt * 8 + r, 8 + 2 * c2)]);
+            return Right(a.x, a.y, b.x, b.y);
+        };
 #pragma unroll
         for (int I = 0; I < 4; ++I) {
             float rest[2][4];
             {
                 Sum s[2];
 #pragma unroll
-                for (int J = 0; J < I; ++J)
+                for (int J = 0; J < I; ++J) {
+                    const Left a = turned(x[2 * J], x[2 * J + 1]);
 #pragma unroll
-                    for (int ks = 0; ks < 2; ++ks) {
-                        const float* xs = x[2 * J + ks];
-                        const Left a(xs[0], xs[2], xs[1], xs[3]);
-#pragma unroll
-                        for (int nt = 0; nt < 2; ++nt) {
-                            const float2 b = *reinterpret_cast<const float2*>(&sm.blk[4 + I * (I - 1) / 2 + J][at16(nt * 8 + r, ks * 8 + 2 * c2)]);
-                            s[nt].add(a, b.x, b.y);
-                        }
-                    }
+                    for (int nt = 0; nt < 2; ++nt) s[nt].add(a, block(4 + I * (I - 1) / 2 + J, nt));
+                }
 #pragma unroll
                 for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -490,19 +509,13 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
                     }
             }
             Sum s[2];
+            const Left a = turned(rest[0], rest[1]);
 #pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-                const Left a(rest[ks][0], rest[ks][2], rest[ks][1], rest[ks][3]);
+            for (int nt = 0; nt < 2; ++nt) {
+                s[nt].add(a, block(I, nt));
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    const float2 b = *reinterpret_cast<const float2*>(&sm.blk[I][at16(nt * 8 + r, ks * 8 + 2 * c2)]);
-                    s[nt].add(a, b.x, b.y);
-                }
+                for (int e = 0; e < 4; ++e) x[2 * I + nt][e] = rest[nt][e] + s[nt].at(e);
             }
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) x[2 * I + nt][e] = s[nt].at(e);
             if (part == 0) {
                 pre[0] *= sm.total[I][c];
                 pre[1] *= sm.total[I][c + 8];
@@ -525,12 +538,24 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
     }
 }
 
+// Sixteen rows of a column whose words are pairs already, the three parts `apart` bytes from one another.
+__device__ __forceinline__ Right right_at(const uint32_t* words, size_t apart) {
+    Right b;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        const uint2 two = *reinterpret_cast<const uint2*>(words + p * apart / 4);
+        b.part[p][0] = two.x, b.part[p][1] = two.y;
+    }
+    return b;
+}
+
 // RING: tiles that a warp's pieces of are in flight or in use: six where a block has an SM to itself, three where two share one
 template <int D, int RING>
 struct WalkSmem {
     float4 ring[RING][8][8][32];             // a warp's pieces of the tiles: a lane reads back what it copied itself
-    float state[2][STRIP][D + 8];            // rounded, rest: rows of value columns, eight banks apart
-    float u[2][STRIP][CHUNK + 8];
+    // rows of value columns, eight banks apart, in three parts: a word is channels (tokens) r and r + 8 of sixteen
+    uint32_t state[3][STRIP][D / 2 + 8];
+    uint32_t u[3][STRIP][CHUNK / 2 + 8];
     float4 part[4][32];                      // the second half of the first product's sums
 };
 
@@ -605,11 +630,11 @@ __global__ void __launch_bounds__(THREADS, RING == 3 ? 2 : 1) channel_walk_kerne
         float* mine = unit + i * step;
         if (owns) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                uint32_t hi, lo;
-                split(S[e], hi, lo);
-                sm.state[0][2 * c2 + (e & 1)][ch + 8 * (e >> 1)] = __uint_as_float(hi);
-                sm.state[1][2 * c2 + (e & 1)][ch + 8 * (e >> 1)] = __uint_as_float(lo);
+            for (int e = 0; e < 2; ++e) {
+                uint32_t part[3];
+                split(S[e], S[2 + e], part);
+#pragma unroll
+                for (int h = 0; h < 3; ++h) sm.state[h][2 * c2 + e][warp * 8 + r] = part[h];
             }
             *reinterpret_cast<float2*>(mine + Unit<D>::S + ch * dv + v0 + 2 * c2) = make_float2(S[0], S[1]);
             *reinterpret_cast<float2*>(mine + Unit<D>::S + (ch + 8) * dv + v0 + 2 * c2) = make_float2(S[2], S[3]);
@@ -623,12 +648,8 @@ __global__ void __launch_bounds__(THREADS, RING == 3 ? 2 : 1) channel_walk_kerne
         {
             SumOf<2> s;
 #pragma unroll
-            for (int ks = 0; ks < HALF; ++ks) {
-                const float4 a = sm.ring[(2 * i) % RING][warp][ks][lane];
-                const int at = (kh * HALF + ks) * 8 + 2 * c2;
-                const uint2 hi = *reinterpret_cast<const uint2*>(&sm.state[0][r][at]), lo = *reinterpret_cast<const uint2*>(&sm.state[1][r][at]);
-                s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
-            }
+            for (int ks = 0; ks < HALF; ks += 2)
+                s.add(Left(sm.ring[(2 * i) % RING][warp][ks][lane], sm.ring[(2 * i) % RING][warp][ks + 1][lane]), right_at(&sm.state[0][r][(kh * HALF + ks) * 4 + 2 * c2], sizeof(sm.state[0])));
             // the two halves meet: 64 threads a barrier
             if (kh == 1) {
                 sm.part[mt][lane] = make_float4(s.at(0), s.at(1), s.at(2), s.at(3));
@@ -638,11 +659,11 @@ __global__ void __launch_bounds__(THREADS, RING == 3 ? 2 : 1) channel_walk_kerne
                 const float4 p = sm.part[mt][lane];
                 const float u[4] = {u0.x - (s.at(0) + p.x), u0.y - (s.at(1) + p.y), u1.x - (s.at(2) + p.z), u1.y - (s.at(3) + p.w)};
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    uint32_t hi, lo;
-                    split(u[e], hi, lo);
-                    sm.u[0][2 * c2 + (e & 1)][tok + 8 * (e >> 1)] = __uint_as_float(hi);
-                    sm.u[1][2 * c2 + (e & 1)][tok + 8 * (e >> 1)] = __uint_as_float(lo);
+                for (int e = 0; e < 2; ++e) {
+                    uint32_t part[3];
+                    split(u[e], u[2 + e], part);
+#pragma unroll
+                    for (int h = 0; h < 3; ++h) sm.u[h][2 * c2 + e][mt * 8 + r] = part[h];
                 }
                 *reinterpret_cast<float2*>(mine + Unit<D>::U + tok * dv + v0 + 2 * c2) = make_float2(u[0], u[1]);
                 *reinterpret_cast<float2*>(mine + Unit<D>::U + (tok + 8) * dv + v0 + 2 * c2) = make_float2(u[2], u[3]);
@@ -654,11 +675,8 @@ __global__ void __launch_bounds__(THREADS, RING == 3 ? 2 : 1) channel_walk_kerne
         if (owns) {
             SumOf<2> s;
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) {
-                const float4 a = sm.ring[(2 * i + 1) % RING][warp][ks][lane];
-                const uint2 hi = *reinterpret_cast<const uint2*>(&sm.u[0][r][ks * 8 + 2 * c2]), lo = *reinterpret_cast<const uint2*>(&sm.u[1][r][ks * 8 + 2 * c2]);
-                s.add(Left(a.x, a.y, a.z, a.w), hi.x, hi.y, lo.x, lo.y);
-            }
+            for (int ks = 0; ks < 8; ks += 2)
+                s.add(Left(sm.ring[(2 * i + 1) % RING][warp][ks][lane], sm.ring[(2 * i + 1) % RING][warp][ks + 1][lane]), right_at(&sm.u[0][r][ks * 4 + 2 * c2], sizeof(sm.u[0])));
             S[0] = fmaf(S[0], g0, s.at(0));
             S[1] = fmaf(S[1], g0, s.at(1));
             S[2] = fmaf(S[2], g1, s.at(2));
@@ -708,15 +726,15 @@ __global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, con
 #pragma unroll 1
         for (int k4 = 0; k4 < steps; k4 += 4)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 4; i += 2) {
                 const int ks = k4 + i;
                 if (ks >= steps) break;
-                const Left a(ahead[i].x, ahead[i].y, ahead[i].z, ahead[i].w);
-                if (ks + 4 < steps) ahead[i] = left[(ks + 4) * 32 + lane];
+                const Left a(ahead[i], ahead[i + 1]);
+                if (ks + 4 < steps) ahead[i] = left[(ks + 4) * 32 + lane], ahead[i + 1] = left[(ks + 5) * 32 + lane];
                 const float *b0 = &right[ks * 8 + 2 * c2][v0 + r], *b1 = b0 + LD;
 #pragma unroll
                 for (int nt = 0; nt < 8; ++nt)
-                    if (nt < tiles) s[nt].add(a, b0[nt * 8], b1[nt * 8]);
+                    if (nt < tiles) s[nt].add(a, Right(b0[nt * 8], b1[nt * 8], b0[nt * 8 + 8 * LD], b1[nt * 8 + 8 * LD]));
             }
     };
     product(reinterpret_cast<const float4*>(mine + Unit<D>::Q) + mt * (D / 8) * 32, D / 8, sm.state);

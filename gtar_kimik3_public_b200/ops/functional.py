@@ -1392,7 +1392,7 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
 
 
 # The longest run of a step from which on the chunks are the faster way: their three kernels take 57 us for one chunk and some 2.5 more
-# a chunk, the kernels that go token by token 0.27 us a token behind 14 (8 heads of 128, one prompt: 33 tokens: 57 / 23 us, 2,048: 137 / 620).
+# a chunk, the kernels that go token by token 0.27 us a token behind 14 (8 heads of 128, one prompt: 33 tokens: 57 / 23 us, 2,048: 146 / 620).
 DELTA_CHANNEL_MIN_TOKENS = 192
 
 
@@ -1410,7 +1410,7 @@ def delta_channel(proj: torch.Tensor, low: torch.Tensor, conv_w: torch.Tensor, c
                   dt_bias: torch.Tensor, norm_w: torch.Tensor, eps: float, state: torch.Tensor, cu_q: torch.Tensor, slots: torch.Tensor,
                   n_seqs: int, max_q_len: int, n_heads: int, n_kv: int, d: int, dv: int, taps: int) -> torch.Tensor:
     """What :func:`delta_prepare`, :func:`conv_roll`, :func:`delta_scan` and :func:`head_norm_gate` (gate behind the decays in ``low``)
-    do in turn, in chunks of 64 tokens on the tensor cores with 32-bit operands (each number as two TF32 numbers); ``max_q_len``
+    do in turn, in chunks of 64 tokens on the tensor cores with 32-bit operands (each number as three bfloat16 numbers whose sum it is); ``max_q_len``
     bounds the sequences' token counts in this step.  Returns the gated read-outs ``[T, n_heads dv]`` (bfloat16)."""
     require_device(proj.device)
     _check(proj, "proj", torch.bfloat16, 2)

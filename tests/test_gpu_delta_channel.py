@@ -133,3 +133,16 @@ def test_a_prompt_in_waves_and_in_portions_is_the_whole_prompt(monkeypatch):
         at += n
     assert torch.equal(conv3, conv) and relative(state3, state) < 2e-6
     assert relative(torch.cat(parts), y) < 2e-3
+
+
+@pytest.mark.parametrize("lens,decay", [([192], -1.0), ([260, 40], -1.0), ([400], -2.0), ([192, 64], -9.0)])
+def test_states_are_no_further_from_64_bits_than_token_by_token(lens, decay):
+    """What a product leaves out (2^-27.5 of it, root mean square) is less than a rounded addition, and there are fewer additions than token by token."""
+    chunks = tokens = 0.0
+    for seed in range(1, 9):
+        layer = Layer(lens, 4, 4, 128, 128, 4, decay, seed=seed)
+        _, want = layer.oracle()
+        used = layer.slots
+        chunks += relative(layer.run(True)[1][used], want[used])
+        tokens += relative(layer.run(False)[1][used], want[used])
+    assert chunks <= tokens
