@@ -63,6 +63,7 @@ struct Unit {
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
+__device__ __forceinline__ bool finite(float x) { return fabsf(x) <= 3.402823466e38f; }
 
 __device__ __forceinline__ void cp_async_16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -75,6 +76,7 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // Two 32-bit numbers as three pairs of bfloat16 numbers: the nearest one, the nearest one to the rest, and what then remains, which is one.
+// A NaN stays one; an infinity leaves NaN as its rest, so that it becomes NaN in every sum.
 __device__ __forceinline__ uint32_t bf16_pair(float x, float y) {
     uint32_t d;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(y), "f"(x));
@@ -508,6 +510,24 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
                         rest[nt][e] = src[t * ld_src + c + 8 * (e >> 1)] * pre[e >> 1] * sm.beta[t] - s[nt].at(e);
                     }
             }
+            // what is no number from a token on (a zero above the block's diagonal times it would be none for the tokens in front)
+            int from[2] = {SUB, SUB};
+            bool numbers = true;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) numbers = numbers && finite(rest[i >> 2][i & 3]);
+            const bool broken = __any_sync(0xffffffffu, !numbers);
+            if (broken) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                    for (int i = 3; i >= 0; --i) {
+                        float& x_t = rest[i >> 1][2 * h + (i & 1)];
+                        if (!finite(x_t)) from[h] = (i >> 1) * 8 + 2 * c2 + (i & 1), x_t = 0.f;
+                    }
+                    from[h] = min(from[h], __shfl_xor_sync(0xffffffffu, from[h], 1));
+                    from[h] = min(from[h], __shfl_xor_sync(0xffffffffu, from[h], 2));
+                }
+            }
             Sum s[2];
             const Left a = turned(rest[0], rest[1]);
 #pragma unroll
@@ -516,6 +536,12 @@ __global__ void __launch_bounds__(THREADS, 2) channel_inner_kernel(Inputs in, fl
 #pragma unroll
                 for (int e = 0; e < 4; ++e) x[2 * I + nt][e] = rest[nt][e] + s[nt].at(e);
             }
+            if (broken)
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (nt * 8 + 2 * c2 + (e & 1) >= from[e >> 1]) x[2 * I + nt][e] = NAN;
             if (part == 0) {
                 pre[0] *= sm.total[I][c];
                 pre[1] *= sm.total[I][c + 8];
@@ -719,7 +745,9 @@ __global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, con
     Sum s[8];
     cp_async_wait<0>();
     __syncthreads();
-    auto product = [&](const float4* left, int steps, const float(*right)[LD]) {
+    // last: the sixteen tokens on the diagonal, where a zero times what is no number would be none for the tokens in front of it
+    bool numbers = true;
+    auto product = [&](const float4* left, int steps, const float(*right)[LD], bool last) {
         float4 ahead[4];  // from L2, four steps ahead
 #pragma unroll
         for (int i = 0; i < 4; ++i) ahead[i] = i < steps ? left[i * 32 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -734,11 +762,33 @@ __global__ void __launch_bounds__(THREADS, 2) channel_read_kernel(Inputs in, con
                 const float *b0 = &right[ks * 8 + 2 * c2][v0 + r], *b1 = b0 + LD;
 #pragma unroll
                 for (int nt = 0; nt < 8; ++nt)
-                    if (nt < tiles) s[nt].add(a, Right(b0[nt * 8], b1[nt * 8], b0[nt * 8 + 8 * LD], b1[nt * 8 + 8 * LD]));
+                    if (nt < tiles) {
+                        float x[4] = {b0[nt * 8], b1[nt * 8], b0[nt * 8 + 8 * LD], b1[nt * 8 + 8 * LD]};
+                        if (last)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                const bool number = finite(x[e]);
+                                numbers = numbers && number;
+                                x[e] = number ? x[e] : 0.f;
+                            }
+                        s[nt].add(a, Right(x[0], x[1], x[2], x[3]));
+                    }
             }
     };
-    product(reinterpret_cast<const float4*>(mine + Unit<D>::Q) + mt * (D / 8) * 32, D / 8, sm.state);
-    product(reinterpret_cast<const float4*>(mine + Unit<D>::P) + mt * 8 * 32, 2 * (mt + 1), sm.u);
+    product(reinterpret_cast<const float4*>(mine + Unit<D>::Q) + mt * (D / 8) * 32, D / 8, sm.state, false);
+    const float4* within = reinterpret_cast<const float4*>(mine + Unit<D>::P) + mt * 8 * 32;
+    product(within, 2 * mt, sm.u, false);
+    product(within + 2 * mt * 32, 2, sm.u + mt * SUB, true);
+    if (__any_sync(0xffffffffu, !numbers)) {
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (nt < tiles)
+#pragma unroll 1
+                    for (int j = 0; j <= r + 8 * (e >> 1); ++j)
+                        if (!finite(sm.u[mt * SUB + j][v0 + nt * 8 + 2 * c2 + (e & 1)])) s[nt].acc[e] = NAN;
+    }
     float ss[2] = {0.f, 0.f};
 #pragma unroll
     for (int nt = 0; nt < 8; ++nt)

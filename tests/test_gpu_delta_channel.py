@@ -146,3 +146,37 @@ def test_states_are_no_further_from_64_bits_than_token_by_token(lens, decay):
         chunks += relative(layer.run(True)[1][used], want[used])
         tokens += relative(layer.run(False)[1][used], want[used])
     assert chunks <= tokens
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf")])
+@pytest.mark.parametrize("where", ["q", "k", "v", "beta", "decay", "gate", "state", "conv"])
+def test_what_is_no_number_comes_out_where_it_does_token_by_token(where, value):
+    """Of one token (in the middle of a block of 16, behind other tokens of its chunk) or of the state: the tokens in front, the other heads and
+    the other sequence stay numbers, and nothing that is no number is lost."""
+    H, G, d, dv = 2, 2, 128, 128
+    for at in (0, 87, 127):
+        layer = Layer([150, 40], H, G, d, dv, 4, -1.0, seed=11)
+        column = {"q": d + 3, "k": G * d + d + 3, "v": 2 * G * d + dv + 5, "beta": layer.C + 1}
+        if where in column:
+            layer.proj[at, column[where]] = value
+        elif where in ("decay", "gate"):
+            layer.low[at, d + 7 if where == "decay" else H * d + dv + 7] = value
+        elif where == "state":
+            layer.state[layer.slots[0], 1, 9, 5] = value
+        else:
+            layer.conv[layer.slots[0], 2, 2 * G * d + dv + 5] = value
+        y, state, conv = layer.run(True)
+        y0, state0, conv0 = layer.run(False)
+        assert torch.equal(conv.isnan(), conv0.isnan()) and torch.equal(conv[~conv.isnan()], conv0[~conv0.isnan()])
+        # a head's row at a token; for infinities 0 * infinity decides which of a row's entries are none, so rows and states' columns as a whole
+        lost = lambda t, t0: (~t0.isfinite()).any(-1) & t.isfinite().all(-1)
+        made = lambda t, t0: (~t.isfinite()).any(-1) & t0.isfinite().all(-1)
+        rows, rows0 = y.view(190, H, dv), y0.view(190, H, dv)
+        turned, turned0 = state.transpose(-1, -2), state0.transpose(-1, -2)
+        assert not lost(rows, rows0).any() and not lost(turned, turned0).any()
+        assert not made(rows, rows0).any() and not made(turned, turned0).any()
+        if value != value:
+            assert torch.equal(y.isnan(), y0.isnan()) and torch.equal(state.isnan(), state0.isnan())
+        # what stays a number is what it was
+        fine, fine0 = y.isfinite() & y0.isfinite(), state.isfinite() & state0.isfinite()
+        assert ((y - y0).abs()[fine] <= 2.0**-7 * y0.abs()[fine] + 1e-4).all() and ((state - state0).abs()[fine0] <= 1e-5).all()
