@@ -1391,9 +1391,34 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, g: torch.Tenso
     return out
 
 
-# The longest run of a step from which on the chunks are the faster way: their three kernels take 57 us for one chunk and some 2.5 more
-# a chunk, the kernels that go token by token 0.27 us a token behind 14 (8 heads of 128, one prompt: 33 tokens: 57 / 23 us, 2,048: 146 / 620).
+# The longest run of a step below which the chunks are not tried: a chain of their three kernels takes some 55 us however short, what the kernels
+# that go token by token need for 150 tokens (8 heads of 128, one prompt of 128: 69 / 49 us).
 DELTA_CHANNEL_MIN_TOKENS = 192
+
+
+def delta_channel_plan(n_seqs: int, max_q_len: int, n_heads: int, unit: int) -> tuple[int, int]:
+    """How many sequences, and how many chunks of each, :func:`delta_channel` has in flight at a time, so that what they leave (``unit`` 32-bit
+    numbers a chunk and head) stays within ``DELTA_WORKSPACE_BYTES``."""
+    room = max(1, DELTA_WORKSPACE_BYTES // (4 * unit * n_heads))
+    group = max(1, min(n_seqs, room))
+    return group, max(1, min(-(-max_q_len // DELTA_CHUNK), room // group))
+
+
+def delta_channel_wins(n_tokens: int, n_seqs: int, max_q_len: int, n_heads: int, d: int) -> bool:
+    """Whether the chunks are the faster way for a step, from estimates of both (us).  Chunks: every turn (sequences and chunks in flight) is a
+    chain of three kernels, which looks at all its sequences; a chunk's length in the walk; what there is to do in all.  Token by token:
+    the longest run, slower where more columns share the device, and what there is to do in all.  Fitted to 180 steps of 8 to 32
+    heads of 128 (one run of 128 to 2,048 beside up to 63 single tokens, 2 to 32 runs of 40 to 512), mean error 7 and 6%: the way it takes is at most 4%
+    slower than the other (token by token / chunks: 8 heads, 1,024 + 15 x 1: 462 / 319, 1,024 + 63 x 1: 474 / 1,392; 256 + 63 x 1: 137 / 490;
+    16 heads, 256 + 1: 125 / 85; 32 heads, 16 x 300: 1,973 / 1,438)."""
+    if max_q_len < DELTA_CHANNEL_MIN_TOKENS:
+        return False
+    group, wave = delta_channel_plan(n_seqs, max_q_len, n_heads, library().gk_delta_channel_work(d))
+    chunks = -(-max_q_len // DELTA_CHUNK)
+    turns = -(-n_seqs // group) * -(-chunks // wave)
+    by_chunks = turns * (52 + 0.036 * group * n_heads) + 1.37 * -(-n_seqs // group) * chunks + 0.29 * n_heads * (n_tokens / DELTA_CHUNK + n_seqs)
+    by_tokens = 12 + max_q_len * (0.17 + 0.0013 * min(n_seqs * n_heads, 128)) + 0.0116 * n_tokens * n_heads
+    return by_chunks < by_tokens
 
 
 def delta_channel_ok(proj: torch.Tensor, low: torch.Tensor, dt_bias: torch.Tensor, norm_w: torch.Tensor, conv_state: torch.Tensor | None,
@@ -1434,13 +1459,13 @@ def delta_channel(proj: torch.Tensor, low: torch.Tensor, conv_w: torch.Tensor, c
         _check(t, name, torch.int32, 1)
     dev = proj.device
     unit = library().gk_delta_channel_work(d)
-    chunks = max(1, -(-int(max_q_len) // DELTA_CHUNK))
-    wave = max(1, min(chunks, DELTA_WORKSPACE_BYTES // max(1, 4 * unit * n_seqs * n_heads)))
-    work = torch.empty((max(1, n_seqs) * wave * n_heads * unit,), dtype=torch.float32, device=dev)
+    group, wave = delta_channel_plan(int(n_seqs), int(max_q_len), n_heads, unit)
+    work = torch.empty((group * wave * n_heads * unit,), dtype=torch.float32, device=dev)
     out = torch.empty((T, n_heads * dv), dtype=torch.bfloat16, device=dev)
-    call("gk_delta_channel", ptr(proj), proj.shape[1], ptr(low), low.shape[1], ptr(conv_w), ptr(conv_state) if taps > 1 else None, ptr(a_log),
-         ptr(dt_bias), ptr(norm_w), float(eps), ptr(state), ptr(work), ptr(out), ptr(cu_q), ptr(slots), int(n_seqs), n_heads, n_kv, d, dv,
-         taps, int(max_q_len), wave, stream_ptr())
+    for first in range(0, int(n_seqs), group):  # a sequence's tokens, state and outputs are where cu_q and slots say
+        call("gk_delta_channel", ptr(proj), proj.shape[1], ptr(low), low.shape[1], ptr(conv_w), ptr(conv_state) if taps > 1 else None, ptr(a_log),
+             ptr(dt_bias), ptr(norm_w), float(eps), ptr(state), ptr(work), ptr(out), ptr(cu_q) + 4 * first, ptr(slots) + 4 * first,
+             min(group, int(n_seqs) - first), n_heads, n_kv, d, dv, taps, int(max_q_len), wave, stream_ptr())
     return out
 
 

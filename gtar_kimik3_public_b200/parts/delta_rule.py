@@ -20,7 +20,8 @@ A step's kernels: the packed projection q | k | v | b; the packed first halves o
 for their second halves (a block-diagonal matrix); one kernel for convolutions, activations, unit lengths, decays and
 beta; one that moves the convolution state on; the recurrence; norm and gate; the output projection.  Prompts,
 portions of prompts and single tokens take the same path in 32-bit runs; bfloat16 steps with a run of 192 tokens and more
-(heads of 64 or 128) do everything between the projections in chunks of 64 tokens on the tensor cores, with 32-bit operands.
+(heads of 64 or 128) do everything between the projections in chunks of 64 tokens on the tensor cores, with 32-bit operands,
+where that is the faster way for all of their sequences together.
 
 The second, ``head_delta``, has one decay number per head, ``g_t = exp(-exp(A_h) * softplus(W_a x + dt_bias_h))``, and its gate is
 ``silu(W_g x)``; everything else is as above.  All of its input projections are one packed product q | k | v | b | a | gate.  A
@@ -121,7 +122,7 @@ class ChannelDeltaRule(Mixer):
         conv_state = cache[1] if self.taps > 1 else None
         proj = linear(x, self.w_in)
         low = linear(linear(x, self.w_low1), self.w_low2, torch.float32)
-        if (ctx.dtype == torch.bfloat16 and not ctx.all_single and ctx.max_q_len >= F.DELTA_CHANNEL_MIN_TOKENS
+        if (ctx.dtype == torch.bfloat16 and not ctx.all_single and F.delta_channel_wins(ctx.n_tokens, ctx.n_seqs, ctx.max_q_len, self.n_heads, self.d)
                 and F.delta_channel_ok(proj, low, self.dt_bias, self.norm_w, conv_state, state, self.d, self.dv, self.taps)):
             y = F.delta_channel(proj, low, self.conv_w, conv_state, self.a_log, self.dt_bias, self.norm_w, self.norm_eps, state, ctx.cu_q,
                                 ctx.slots, ctx.n_seqs, ctx.max_q_len, self.n_heads, self.n_kv, self.d, self.dv, self.taps)

@@ -180,3 +180,37 @@ def test_what_is_no_number_comes_out_where_it_does_token_by_token(where, value):
         # what stays a number is what it was
         fine, fine0 = y.isfinite() & y0.isfinite(), state.isfinite() & state0.isfinite()
         assert ((y - y0).abs()[fine] <= 2.0**-7 * y0.abs()[fine] + 1e-4).all() and ((state - state0).abs()[fine0] <= 1e-5).all()
+
+
+def test_many_sequences_stay_within_the_workspace_and_go_in_groups(monkeypatch):
+    """One run beside many single tokens: the workspace is bounded whatever the number of sequences, and a sequence's result does not depend on it."""
+    layer = Layer([200] + [1] * 40 + [70], 8, 8, 128, 128, 4, -1.0, seed=5)
+    whole = layer.run(True)
+    f = F()
+    monkeypatch.setattr(f, "DELTA_WORKSPACE_BYTES", 5 * 8 * 4 * f.library().gk_delta_channel_work(128))
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    sizes, empty = [], torch.empty
+    monkeypatch.setattr(torch, "empty", lambda shape, **kw: sizes.append(4 * shape[0]) or empty(shape, **kw) if len(shape) == 1 else empty(shape, **kw))
+    grouped = layer.run(True)
+    assert sizes and max(sizes) <= f.DELTA_WORKSPACE_BYTES
+    assert all(torch.equal(a, b) for a, b in zip(whole, grouped))
+
+
+def test_a_long_run_beside_many_single_tokens_goes_token_by_token(monkeypatch):
+    from gtar_kimik3_public_b200.engine.step import SequenceStep, plan_step
+    from gtar_kimik3_public_b200.parts.base import build_part
+
+    part = build_part("mixer", "channel_delta", hidden_size=256, n_heads=2, n_kv_heads=2, key_dim=128, value_dim=128, conv_taps=4, norm_eps=EPS)
+    b = lambda *shape: rand(*shape, seed=sum(shape), scale=0.05).to(torch.bfloat16).to(DEV)
+    wide = 256
+    part.load({"q": b(wide, 256), "k": b(wide, 256), "v": b(wide, 256), "q.conv": b(wide, 4), "k.conv": b(wide, 4), "v.conv": b(wide, 4), "b": b(2, 256),
+               "A_log": b(2), "norm": b(128), "a1": b(64, 256), "a2": b(wide, 64), "dt_bias": b(wide), "g1": b(64, 256), "g2": b(wide, 64), "o": b(256, wide)})
+    taken, chunks = [], F().delta_channel
+    monkeypatch.setattr(F(), "delta_channel", lambda *a: taken.append(1) or chunks(*a))
+    for counts, want in (([512], 1), ([512] + [1] * 127, 0), ([100, 100], 0)):
+        taken.clear()
+        cache = tuple(torch.zeros((len(counts), *r.shape), dtype=r.dtype, device=DEV) for r in part.cache_request())
+        ctx = plan_step([SequenceStep(i, 0, [0] * c, []) for i, c in enumerate(counts)], torch.bfloat16, torch.device(DEV), 1)
+        part.forward(b(sum(counts), 256), ctx, cache)
+        assert len(taken) == want, counts

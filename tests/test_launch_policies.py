@@ -1,6 +1,6 @@
 """Host-side choices of launch shapes: pure functions of the step's sizes, checked without a GPU."""
 
-from gtar_kimik3_public_b200.ops.functional import SCRATCH_SPLITS_FROM, decode_splits, split_k_for
+from gtar_kimik3_public_b200.ops.functional import DELTA_WORKSPACE_BYTES, SCRATCH_SPLITS_FROM, decode_splits, delta_channel_plan, delta_channel_wins, split_k_for
 
 
 def test_decode_splits_stay_within_what_the_kernels_take():
@@ -171,3 +171,23 @@ def test_split_k_of_more_than_sixteen_tokens_leaves_every_block_an_sm():
         for n in range(128, 2700, 128):
             splits = split_k_for(m, n, 9728)
             assert splits < 8 or -(-n // 128) * splits <= 148
+
+
+def test_delta_chunks_in_flight_stay_within_the_workspace():
+    for d, unit in ((64, 24640), (128, 53376)):
+        for heads in (1, 8, 16, 32, 64, 128):
+            for n_seqs in (1, 2, 16, 64, 79, 256, 1000):
+                for longest in (1, 64, 200, 2048, 32768):
+                    group, wave = delta_channel_plan(n_seqs, longest, heads, unit)
+                    assert 1 <= group <= n_seqs and 1 <= wave <= -(-longest // 64)
+                    assert 4 * unit * heads * group * wave <= DELTA_WORKSPACE_BYTES
+
+
+def test_delta_chunks_where_they_measured_faster():
+    """(tokens, sequences, longest run, heads of 128): us token by token and in chunks."""
+    measured = {(128, 1, 128, 8): (49, 69), (192, 1, 192, 8): (67, 77), (255, 64, 192, 8): (109, 416), (256, 1, 256, 8): (88, 79), (319, 64, 256, 8): (137, 490),
+                (543, 32, 512, 8): (241, 351), (1024, 1, 1024, 8): (314, 99), (1039, 16, 1024, 8): (462, 319), (1087, 64, 1024, 8): (474, 1392),
+                (2048, 1, 2048, 8): (622, 147), (223, 32, 192, 16): (116, 417), (257, 2, 256, 16): (125, 85), (1031, 8, 1024, 16): (502, 352),
+                (1055, 32, 1024, 16): (513, 1416), (192, 1, 192, 32): (118, 90), (271, 16, 256, 32): (209, 504), (4800, 16, 300, 32): (1973, 1438)}
+    for (tokens, n_seqs, longest, heads), (by_tokens, by_chunks) in measured.items():
+        assert delta_channel_wins(tokens, n_seqs, longest, heads, 128) == (by_chunks < by_tokens), (tokens, n_seqs, longest, heads)
