@@ -42,11 +42,12 @@ GK_EXPORT int gk_set_pdl(int on) {
 
 thread_local int t_gk_chain = 0;
 
-// on = 1: the calls of this thread up to the one with 0 launch the kernels of one layer, which read nothing before pdl_wait() that one of
-// them writes; all but the first may start early.  Returns the state before (0: outside a layer).
-GK_EXPORT int gk_chain(int on) {
+// 1: the calls of this thread up to the one with 0 launch the kernels of one layer, which read nothing before pdl_wait() that one of
+// them writes; all but the first may start early.  Returns the state before (0: outside a layer, 2: behind its first kernel), which may be
+// put back.
+GK_EXPORT int gk_chain(int state) {
     const int before = t_gk_chain;
-    t_gk_chain = on ? 1 : 0;
+    t_gk_chain = state;
     return before;
 }
 

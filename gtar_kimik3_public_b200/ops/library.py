@@ -206,10 +206,13 @@ def one_layer(forward):
     @functools.wraps(forward)
     def marked(*args, **kwargs):
         chain = library().gk_chain
-        chain(1)
+        before = chain(1)
+        if before:  # a layer within a layer: the outer one's mark stays what it is, and ends with the outer one
+            chain(before)
         try:
             return forward(*args, **kwargs)
         finally:
-            chain(0)
+            if not before:
+                chain(0)
 
     return marked

@@ -35,3 +35,21 @@ def test_the_mark_is_the_threads_own():
     thread.start()
     thread.join()
     assert other == [0] and chain(0) == 1
+
+
+def test_a_layer_within_a_layer_leaves_the_mark_as_it_is():
+    """2: the outer layer's first kernel has been launched."""
+    chain, seen = library().gk_chain, []
+
+    @one_layer
+    def inner():
+        seen.append(chain(2))
+
+    @one_layer
+    def outer():
+        chain(2)
+        inner()
+        seen.append(chain(2))
+
+    outer()
+    assert seen == [2, 2] and chain(0) == 0
