@@ -36,10 +36,13 @@ int gk_fail(int status, const char* fmt, ...);
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-extern int g_gk_pdl;  // set through gk_set_pdl(): launch kernels with programmatic stream serialization
+// gk_set_pdl(): 1: every kernel may start early (programmatic stream serialization), 0: none may, -1 (as the library is loaded): those behind
+// the first of a layer or of a call.
+extern int g_gk_pdl;
 // gk_chain(): this thread is launching the kernels of one layer.  1: none of them yet (the first waits for all that is in front of
-// it, as ever), 2: the later ones, which may start early like those of a captured step.
+// it, as ever), 2: the later ones, which may start early like those of a captured step.  -1: none of this thread's kernels starts early.
 extern thread_local int t_gk_chain;
+inline bool gk_early(bool behind) { return t_gk_chain >= 0 && g_gk_pdl != 0 && (g_gk_pdl > 0 || behind); }
 void gk_prepare_kernel(const void* kernel);  // once per kernel: its preferred L1 / shared-memory split
 
 // Launches `kernel` on `stream` as thread-block clusters of `cluster` blocks (where that is more than one), with the
@@ -71,11 +74,12 @@ inline cudaError_t gk_launch_with(bool early, void (*kernel)(KArgs...), dim3 gri
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// The attribute where it is switched on: what the kernel reads before pdl_wait() no kernel of such a step may write.
+// The attribute where it is switched on or the kernel is behind the first of a layer: what it reads before pdl_wait() no kernel of such a
+// step may write.
 template <typename... KArgs, typename... Args>
 inline cudaError_t gk_launch_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                      dim3 cluster, Args... args) {
-    const bool early = g_gk_pdl != 0 || t_gk_chain == 2;
+    const bool early = gk_early(t_gk_chain == 2);
     if (t_gk_chain == 1) t_gk_chain = 2;
     return gk_launch_with(early, kernel, grid, block, smem, stream, cluster, args...);
 }
@@ -87,12 +91,12 @@ inline cudaError_t gk_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 
 // For the second and later kernels of one call of this library: the kernel in front is the call's own, which waits for what is in
-// front of it, and this one touches no memory before pdl_wait(); so it may take its place on the SMs early whatever the switch says.
+// front of it, and this one touches no memory before pdl_wait(); so it may take its place on the SMs early unless that is switched off.
 // (What it saves where kernels are launched one by one: two products of a feed-forward, which start early in the same way, take 33.2 us
 // instead of 36.9.)
 template <typename... KArgs, typename... Args>
 inline cudaError_t gk_launch_behind(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
-    return gk_launch_with(true, kernel, grid, block, smem, stream, dim3(1, 1, 1), args...);
+    return gk_launch_with(gk_early(true), kernel, grid, block, smem, stream, dim3(1, 1, 1), args...);
 }
 
 __device__ __forceinline__ float to_float(float x) { return x; }

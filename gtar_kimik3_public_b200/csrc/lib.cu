@@ -18,7 +18,7 @@ int gk_fail(int status, const char* fmt, ...) {
     return status;
 }
 
-int g_gk_pdl = 0;
+int g_gk_pdl = -1;
 
 // Every kernel asks for the largest shared-memory share of the SM's L1/shared-memory array.  An SM changes
 // that split only when it is idle, so kernels that prefer different splits cannot be resident side by side,
@@ -36,15 +36,15 @@ void gk_prepare_kernel(const void* kernel) {
 // library; returns the previous setting.
 GK_EXPORT int gk_set_pdl(int on) {
     const int before = g_gk_pdl;
-    g_gk_pdl = on ? 1 : 0;
+    g_gk_pdl = on < 0 ? -1 : on ? 1 : 0;
     return before;
 }
 
 thread_local int t_gk_chain = 0;
 
 // 1: the calls of this thread up to the one with 0 launch the kernels of one layer, which read nothing before pdl_wait() that one of
-// them writes; all but the first may start early.  Returns the state before (0: outside a layer, 2: behind its first kernel), which may be
-// put back.
+// them writes; all but the first may start early.  -1: up to the next call of this none of the thread's kernels starts early, whatever the
+// switch says.  Returns the state before (0: neither, 2: behind the first of a layer), which may be put back.
 GK_EXPORT int gk_chain(int state) {
     const int before = t_gk_chain;
     t_gk_chain = state;

@@ -18,6 +18,7 @@ import torch
 
 from ..cache import Cache, CacheFull
 from ..models.model import Model
+from ..ops.library import in_order
 from .step import SequenceStep, pack_step, plan_step
 
 
@@ -50,11 +51,12 @@ class Engine:
         self.slot_of: dict[object, int] = {}
         self.steps_run = 0
         self.graphs = None
+        if use_pdl is None:
+            use_pdl = os.environ.get("GTAR_B200_PDL", "1") != "0"
+        self.use_pdl = use_pdl
         if use_graphs and model.device.type == "cuda" and model.graph_safe():
             from .graphs import StepGraphs
 
-            if use_pdl is None:
-                use_pdl = os.environ.get("GTAR_B200_PDL", "1") != "0"
             self.graphs = StepGraphs(model, self.cache, use_pdl)
 
     # ------------------------------------------------------------------ requests
@@ -152,7 +154,11 @@ class Engine:
                 logits = self.graphs.run(packed, key=key)
                 return logits.clone() if keep_output else logits
         ctx = plan_step(sequences, self.model.dtype, self.model.device, vocab)
-        return self.model.step(ctx, self.cache)
+        return self._launch(ctx)
+
+    def _launch(self, ctx) -> torch.Tensor:
+        step = self.model.step if self.use_pdl or self.model.device.type != "cuda" else in_order(self.model.step)
+        return step(ctx, self.cache)
 
     def decode_on_device(self, request_ids: list, tokens: torch.Tensor) -> torch.Tensor:
         """One token for each of the listed live requests, the token ids being on the device already
@@ -173,4 +179,4 @@ class Engine:
         if self.graphs is not None:
             return self.graphs.run(pack_step(sequences, self.model.vocab_size, check_tokens=False), device_tokens=tokens)
         ctx = plan_step(sequences, self.model.dtype, self.model.device, self.model.vocab_size, device_tokens=tokens)
-        return self.model.step(ctx, self.cache)
+        return self._launch(ctx)

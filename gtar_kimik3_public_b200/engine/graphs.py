@@ -148,7 +148,8 @@ class StepGraphs:
         # launch shapes inside a graph must not depend on the lengths of the day: a bound stands in
         bound, typical = self.length_bounds(packed)
         ctx = context_from_views(packed, self.views(packed), self.model.dtype, max_kv_len=bound, typical_kv_len=typical)
-        result = self.model.step(ctx, self.cache)  # one-time set-up happens here, outside the capture
+        step = self.model.step if self.use_pdl else library.in_order(self.model.step)
+        result = step(ctx, self.cache)  # one-time set-up happens here, outside the capture
         torch.cuda.synchronize()
         while len(self.graphs) >= self.MAX_PREFILL_GRAPHS + 3 * self.s_max:
             self.graphs.popitem(last=False)
@@ -163,7 +164,7 @@ class StepGraphs:
         gc.disable()
         try:
             with torch.cuda.graph(graph, pool=self.pool):
-                logits = self.model.step(ctx, self.cache)
+                logits = step(ctx, self.cache)
         finally:
             set_pdl(before)
             if collecting:

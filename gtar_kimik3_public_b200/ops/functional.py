@@ -399,11 +399,13 @@ def copy_to_device(device_ints: torch.Tensor, pinned_ints: torch.Tensor, begin: 
         raise KernelError(library().gk_last_error().decode(errors="replace"))  # (no kernel: not among the launches that `call` counts)
 
 
-def set_pdl(on: bool) -> bool:
-    """Switches programmatic dependent launch for all later kernel launches; returns the old setting."""
+def set_pdl(on: bool | None) -> bool | None:
+    """Switches programmatic dependent launch for all later kernel launches: for all of them, for none, or (None, as the library is loaded)
+    for those behind the first of a layer or of a call.  Returns the old setting."""
     from .library import library
 
-    return bool(library().gk_set_pdl(int(on)))
+    before = library().gk_set_pdl(-1 if on is None else int(on))
+    return None if before < 0 else bool(before)
 
 
 GEMV_MAX_TOKENS = 16

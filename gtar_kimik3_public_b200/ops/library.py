@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import os
 import threading
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_ulonglong, c_void_p
 
@@ -143,6 +144,8 @@ def library() -> ctypes.CDLL:
             fn.argtypes = argtypes
             fn.restype = c_int
         lib.gk_device_capability.restype = c_int
+        if os.environ.get("GTAR_B200_PDL", "1") == "0":
+            lib.gk_set_pdl(0)
         _lib = lib
         return lib
 
@@ -207,7 +210,7 @@ def one_layer(forward):
     def marked(*args, **kwargs):
         chain = library().gk_chain
         before = chain(1)
-        if before:  # a layer within a layer: the outer one's mark stays what it is, and ends with the outer one
+        if before:  # a layer within a layer, or a thread whose kernels wait for one another: stays what it is
             chain(before)
         try:
             return forward(*args, **kwargs)
@@ -216,3 +219,18 @@ def one_layer(forward):
                 chain(0)
 
     return marked
+
+
+def in_order(function):
+    """``function`` with every kernel that it launches waiting for the one in front, whatever is switched on (the calling thread's own)."""
+
+    @functools.wraps(function)
+    def waiting(*args, **kwargs):
+        chain = library().gk_chain
+        before = chain(-1)
+        try:
+            return function(*args, **kwargs)
+        finally:
+            chain(before)
+
+    return waiting
