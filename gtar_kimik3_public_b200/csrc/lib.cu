@@ -32,8 +32,8 @@ void gk_prepare_kernel(const void* kernel) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }
 
-// Switches programmatic dependent launch on (1) or off (0) for every later kernel launch of the
-// library; returns the previous setting.
+// Switches programmatic dependent launch on (1) or off (0) for every later kernel launch of the library, or leaves it to those behind the
+// first of a layer or of a call (-1); returns the previous setting.
 GK_EXPORT int gk_set_pdl(int on) {
     const int before = g_gk_pdl;
     g_gk_pdl = on < 0 ? -1 : on ? 1 : 0;

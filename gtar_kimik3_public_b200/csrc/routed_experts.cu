@@ -1297,7 +1297,7 @@ int launch_ring(const MmaStep& p, int at_once, size_t staged, int blocks, cudaSt
     const long long most = std::min(p.pairs, (long long)MMA_LIST) * (p.n_rows / 16);
     cudaFuncSetAttribute(experts_mma_kernel<UP, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - MMA_STATIC_SMEM));
     // the down product stands behind the up product of the same call
-    gk_launch_with(gk_early(!UP), experts_mma_kernel<UP, DEPTH>,
+    gk_launch_with(gk_early(!UP || t_gk_chain == 2), experts_mma_kernel<UP, DEPTH>,
                    dim3((unsigned)std::min(most, (long long)blocks * sm_count()), 1, (unsigned)((p.pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32),
                    staged + ring_bytes(UP, DEPTH), s, dim3(1, 1, 1), map, (const __nv_bfloat16*)p.source, p.ids, (__nv_bfloat16*)p.act, p.parts, (int)p.pairs,
                    p.k, p.n_rows, p.divide, p.n_experts, at_once, (int)staged, box_k, p.error_flag);
