@@ -742,7 +742,7 @@ struct BoxRing {
     int asked = 0, taken = 0, put = 0, take = 0;
     uint32_t phase = 0;
     bool ok = true;
-    // one lane asks; the whole warp has read what stood in the place before
+    // one lane asks; the whole warp has read what stood in the place before.  Behind a wait that was given up nothing more is asked for.
     __device__ __forceinline__ void ask(const CUtensorMap* map, int k, int row, int rows_apart, int box_k, bool elected) {
         if (elected) {
             const uint32_t bar = smem_address(full + put);
@@ -757,17 +757,21 @@ struct BoxRing {
         ++asked;
         put = put + 1 == DEPTH ? 0 : put + 1;
     }
+    // Every lane waits for itself; one that gave up stays at the box that it gave up, so that drain() waits for it again.
     __device__ __forceinline__ const unsigned char* next() {
         if (ok) ok = box_wait(full + take, phase);
         return slots + take * SLOT;
     }
-    __device__ __forceinline__ void done() {
+    __device__ __forceinline__ void pass() {
         ++taken;
         take = take + 1 == DEPTH ? 0 : take + 1;
         if (take == 0) phase ^= 1;
     }
+    __device__ __forceinline__ void done() {
+        if (ok) pass();
+    }
     __device__ __forceinline__ void drain() {  // nothing may land in shared memory after the block is gone
-        for (; taken < asked; done()) box_wait(full + take, phase);
+        for (; taken < asked; pass()) box_wait(full + take, phase);
     }
 };
 
@@ -884,7 +888,7 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) experts_mma_kernel(
         if (ahead < unit_end) row = runs[ahead / tiles].expert * NM * n_rows + (ahead % tiles) * 16;
     };
     const auto ask = [&]() {
-        if (ahead >= unit_end) return;
+        if (ahead >= unit_end || !ring.ok) return;
         ring.ask(&map, piece * 32, row, n_rows, box_k, lane == 0);
         piece += per;
         if (piece >= end) {
@@ -961,7 +965,7 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) experts_mma_kernel(
         }
         // the next unit's first barrier stands before `part` is written again
     }
-    if (!ring.ok && lane == 0) atomicExch(error_flag, 41);
+    if (!__all_sync(0xffffffffu, ring.ok) && lane == 0) atomicExch(error_flag, 71);
     ring.drain();
 }
 

@@ -173,6 +173,15 @@ def test_split_k_of_more_than_sixteen_tokens_leaves_every_block_an_sm():
             assert splits < 8 or -(-n // 128) * splits <= 148
 
 
+def test_every_code_of_a_given_up_wait_is_one_kernels_own():
+    import re
+
+    from gtar_kimik3_public_b200.csrc import build
+
+    codes = [(int(code), path.name) for path in build.sources() for code in re.findall(r"atomicExch\([\w.]*error_flag, (\d+)\)", path.read_text())]
+    assert len(codes) > 15 and len({code for code, _ in codes}) == len(codes), sorted(codes)
+
+
 def test_delta_chunks_in_flight_stay_within_the_workspace():
     for d, unit in ((64, 24640), (128, 53376)):
         for heads in (1, 8, 16, 32, 64, 128):
