@@ -683,14 +683,14 @@ __global__ void __launch_bounds__(UP_WARPS * 32) token_down_kernel(const T* __re
 // and take equal runs of (expert, sixteen rows) units: the experts that were chosen are listed by every block for itself.  (One block a pair
 // and chunk of rows, most of which found that another had their expert, spent their time in the chain ids - list - weights - tokens.)
 //
-// The weights come by TMA, boxes of sixteen rows x 64 entries into a ring of every warp's own that runs on across the ends of units, 48 KB
-// of them a block and two blocks an SM.  (Loads into registers had four pieces in flight that ended with every unit, and went through
+// The weights come by TMA, boxes of sixteen rows x 64 entries into a ring of every warp's own that runs on across the ends of units, in two to
+// four blocks an SM.  (Loads into registers had four pieces in flight that ended with every unit, and went through
 // the load unit 64 bytes of a row at a time: 400 cycles a piece and warp, which also held for copies of 16 bytes into a ring.)
 // (Tensor-memory products would want 128 rows a tile, for a step that does next to no arithmetic.)
-// Measured (us, cold; up, down and join; loads into registers / here): 6 of 64 experts of 2,048 x 1,024: 4 tokens 91 / 65, 8: 95 / 77,
-// 16: 114 / 81, 42: 175 / 142; 4 of 32 of 1,024 x 768: 8 tokens 46 / 34, 63: 69 / 65; 2 of 8 of 6,144 x 512: 16 tokens 108 / 81.
-// Every pair by itself on the FP32 pipes: 8 tokens 170 and 43, 42 and 63 tokens 763 and 265.  Bound by the weights (4.6 TB/s of them in
-// the up product of 8 tokens) with 6 us of launch and list before the first of them.
+// Measured (us, cold; up, down and join; loads into registers / here): 6 of 64 experts of 2,048 x 1,024: 8 tokens 140 / 93, 42: 237 / 167; 4 of
+// 32 of 1,024 x 768: 16 tokens 56 / 42, 63: 68 / 55; 2 of 16 of 4,096 x 1,536: 16 tokens 177 / 118, 120: 344 / 262; of 1,024 x 4,096, 120: 194 / 182.
+// Every pair by itself on the FP32 pipes: 8 tokens 170 and 43, 42 and 63 tokens 763 and 265.  Bound by the weights (4.7 TB/s of them in the
+// whole call of 8 tokens) with 6 us of launch and list before the first of them, by the tokens' products where an expert has sixteen and more.
 constexpr int MMA_WARPS = 4, MMA_TOKENS = 16, MMA_LIST = 512;
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -1280,7 +1280,10 @@ bool mma_suits(int k, int n_rows, int n_experts) {
 }
 
 constexpr size_t ring_bytes(bool up, int depth) { return (size_t)MMA_WARPS * depth * (up ? 2 : 1) * 16 * 128; }
-constexpr size_t MMA_STATIC_SMEM = MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + MMA_WARPS * 2 * (MMA_TOKENS / 8 * 4) * 32 * sizeof(float) + 1024;
+// at most the shared memory of a block beside its rings and its tokens' rows: whole pieces of 128 bytes, and what the device keeps for itself
+constexpr size_t mma_static_bytes(bool up, int depth) {
+    return MMA_LIST * (sizeof(int) + sizeof(MmaRun)) + MMA_WARPS * ((up ? 2 : 1) * (MMA_TOKENS / 8 * 4) * 32 * sizeof(float) + depth * sizeof(uint64_t)) + 128 + 1024;
+}
 
 struct MmaStep {
     const void *source, *weights;
@@ -1299,7 +1302,7 @@ int launch_ring(const MmaStep& p, int at_once, size_t staged, int blocks, cudaSt
     const int status = gk_matrix_map(&map, p.weights, (long long)p.n_experts * (UP ? 2 : 1) * p.n_rows, p.k, p.k, box_k, 16, false);
     if (status) return status;
     const long long most = std::min(p.pairs, (long long)MMA_LIST) * (p.n_rows / 16);
-    cudaFuncSetAttribute(experts_mma_kernel<UP, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(227 * 1024 - MMA_STATIC_SMEM));
+    cudaFuncSetAttribute(experts_mma_kernel<UP, DEPTH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(228 * 1024 - mma_static_bytes(UP, DEPTH)));
     // the down product stands behind the up product of the same call
     gk_launch_with(gk_early(!UP || t_gk_chain == 2), experts_mma_kernel<UP, DEPTH>,
                    dim3((unsigned)std::min(most, (long long)blocks * sm_count()), 1, (unsigned)((p.pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32),
@@ -1310,13 +1313,21 @@ int launch_ring(const MmaStep& p, int at_once, size_t staged, int blocks, cudaSt
 
 template <bool UP>
 int launch_mma(const MmaStep& p, cudaStream_t s) {
-    // 48 KB of rings and two blocks an SM; beside longer tokens' rows one block with 128 KB, or 32 KB where the rows leave no more
-    constexpr int TWO = UP ? 3 : 6, DEEP = UP ? 8 : 16, FLAT = UP ? 2 : 4;
     const int at_once = p.n_tokens > 8 && MMA_TOKENS * (size_t)mma_stride(p.k) <= 48 * 1024 ? MMA_TOKENS : 8;
     const size_t rows = (size_t)at_once * mma_stride(p.k), counts = (2 * (size_t)p.n_experts + MMA_LIST) * 4, staged = ((rows > counts ? rows : counts) + 127) / 128 * 128;
-    if (staged + ring_bytes(UP, TWO) + MMA_STATIC_SMEM <= 112 * 1024) return launch_ring<UP, TWO>(p, at_once, staged, 2, s);
-    if (staged + ring_bytes(UP, DEEP) + MMA_STATIC_SMEM <= 227 * 1024) return launch_ring<UP, DEEP>(p, at_once, staged, 1, s);
-    return launch_ring<UP, FLAT>(p, at_once, staged, 1, s);
+    // As many blocks an SM as find room beside the tokens' rows, up to three (up) and four (down), with rings as deep as that leaves; one block
+    // with 128 KB of rings only where two do not fit.  What a block has to do for a box (a warp a scheduler) weighs more than the boxes in
+    // flight.  Measured (us, whole call; two blocks with rings of 48 KB, or one with 128 KB where rows are 4,096 / here): 2 of 16 experts of 4,096
+    // x 1,536: 16 tokens 158 / 118, 63: 245 / 169; of 1,024 x 4,096: 120 tokens 226 / 182; 2 of 64 of 4,096 x 512: 63 tokens 221 / 149; 4 of 64 of
+    // 2,048 x 1,024: 16 tokens 130 / 117; 4 of 16 of 512 x 2,048: 63 tokens 73 / 60.
+    const auto fits = [&](int blocks, int depth) { return blocks * (staged + ring_bytes(UP, depth) + mma_static_bytes(UP, depth)) <= 228 * 1024; };
+    for (int blocks = UP ? 3 : 4; blocks >= 2; --blocks) {
+        if (!fits(blocks, 2)) continue;
+        if constexpr (UP) return fits(blocks, 3) ? launch_ring<UP, 3>(p, at_once, staged, blocks, s) : launch_ring<UP, 2>(p, at_once, staged, blocks, s);
+        else return fits(blocks, 4) ? launch_ring<UP, 4>(p, at_once, staged, blocks, s) : launch_ring<UP, 2>(p, at_once, staged, blocks, s);
+    }
+    constexpr int DEEP = UP ? 8 : 16, FLAT = UP ? 2 : 4;
+    return fits(1, DEEP) ? launch_ring<UP, DEEP>(p, at_once, staged, 1, s) : launch_ring<UP, FLAT>(p, at_once, staged, 1, s);
 }
 
 // Megabytes of weights that the pairs of a step fetch and that they would not if every expert came once (a token's experts are all

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("tokens,width,ff,experts,top", [
     (700, 64, 32, 8, 6), (512, 96, 160, 8, 4), (300, 224, 96, 5, 5), (40, 2048, 64, 16, 4), (24, 4096, 128, 3, 2), (9, 6144, 160, 4, 3), (8, 9216, 64, 4, 4),
-    (16, 96, 9216, 3, 2)])
+    (16, 96, 9216, 3, 2), (63, 512, 2048, 16, 4), (63, 1024, 768, 32, 4), (30, 2048, 1024, 8, 3)])
 def test_rows_of_every_length(tokens, width, ff, experts, top):
     gen = torch.Generator(device=DEV).manual_seed(width + ff)
     draw = lambda *shape, scale=1.0: torch.randn(shape, generator=gen, device=DEV) * scale
