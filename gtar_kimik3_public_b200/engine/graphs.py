@@ -62,6 +62,12 @@ class StepGraphs:
         self.pool = None
         self.launches: dict[tuple, int] = {}
 
+    def __del__(self):
+        # The allocator of pinned memory does not know of copy_to_device's copies: it would hand the buffers on while one is still to run.
+        for event in getattr(self, "events", ()):
+            if event is not None:
+                event.synchronize()
+
     # ------------------------------------------------------------------ step inputs
     @staticmethod
     def offsets(packed: PackedStep) -> list[int]:
