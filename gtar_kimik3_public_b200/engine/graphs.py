@@ -29,7 +29,7 @@ where it first needs them.
 from __future__ import annotations
 
 import gc
-from collections import OrderedDict
+from collections import OrderedDict, deque
 
 import numpy as np
 import torch
@@ -39,6 +39,21 @@ from ..ops.functional import copy_to_device, set_pdl
 from .step import PackedStep, context_from_views
 
 
+# Pinned buffers of engines that are gone, with the events behind the copies out of them: given back when the next engine is made, those whose
+# copies have run by then.
+_retired: deque = deque()
+
+
+def _give_back_retired() -> None:
+    for _ in range(len(_retired)):
+        try:
+            entry = _retired.popleft()
+        except IndexError:  # another thread was faster
+            return
+        if not all(event.query() for event in entry[1]):
+            _retired.append(entry)
+
+
 class StepGraphs:
     RING = 8
     MAX_PREFILL_GRAPHS = 12
@@ -46,6 +61,7 @@ class StepGraphs:
 
     def __init__(self, model, cache, use_pdl: bool = True):
         self.model, self.cache, self.use_pdl = model, cache, use_pdl
+        _give_back_retired()
         device = model.device
         self.t_max = cache.n_pages * cache.page_size  # no step can bring more tokens than the cache holds
         self.s_max = cache.max_seqs
@@ -64,9 +80,10 @@ class StepGraphs:
 
     def __del__(self):
         # The allocator of pinned memory does not know of copy_to_device's copies: it would hand the buffers on while one is still to run.
-        for event in getattr(self, "events", ()):
-            if event is not None:
-                event.synchronize()
+        # (Waiting for them here would make whoever drops an engine wait for its last step.)
+        events = [event for event in getattr(self, "events", ()) if event is not None]
+        if events:
+            _retired.append((self.host, events))
 
     # ------------------------------------------------------------------ step inputs
     @staticmethod
