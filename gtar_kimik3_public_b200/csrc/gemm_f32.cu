@@ -165,22 +165,22 @@ __device__ __forceinline__ unsigned long long twice(float a) {
     return d;
 }
 
-// Four entries of row `row` from k0 on, zeros outside the matrix.
+// Four entries of row `row` from k0 on, zeros where the row is not there and behind its end.
 template <bool VEC, typename T>
-__device__ __forceinline__ void fetch4(const T* __restrict__ src, long long ld, int row, int n_rows, int k0, int K, float (&v)[4]) {
-    if (VEC && row < n_rows && k0 + 4 <= K) {
+__device__ __forceinline__ void fetch4(const T* __restrict__ src, long long ld, int row, bool there, int k0, int K, float (&v)[4]) {
+    if (VEC && there && k0 + 4 <= K) {
         read4(src + (size_t)row * ld + k0, v);
         return;
     }
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = row < n_rows && k0 + e < K ? to_float(src[(size_t)row * ld + k0 + e]) : 0.f;
+    for (int e = 0; e < 4; ++e) v[e] = there && k0 + e < K ? to_float(src[(size_t)row * ld + k0 + e]) : 0.f;
 }
 
 constexpr int WIDE_BK = 16;
 
 // A thread has TM rows of A and TN of W, as TM x TN / 2 pairs of chains.  Operands go through registers into shared memory, turned (a step
 // of k is a row there), so that a 16-byte read brings four rows' entries of one step: what shared memory delivers, 128 bytes a clock
-// whether lanes ask for the same ones or not, is TM + TN numbers a thread for TM TN chain steps.
+// whether lanes ask for the same ones or not, is TM + TN numbers a thread for TM TN chain steps.  N is a multiple of BN (the launch's rule).
 template <typename TA, typename TC, int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_f32_wide_kernel(const Product p) {
     constexpr int RN = BN / TN, THREADS = (BM / TM) * RN, BK = WIDE_BK, LDA = BM + 4, LDW = BN + 4;
@@ -198,11 +198,14 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_f32_wide_kernel(co
     float va[NA][4], vw[NW][4];
     const auto fetch_w = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < NW; ++i) fetch4<VEC>(W, p.ldw, n0 + row + i * (THREADS / 4), p.N, k0 + piece, p.K, vw[i]);
+        for (int i = 0; i < NW; ++i) fetch4<VEC>(W, p.ldw, n0 + row + i * (THREADS / 4), true, k0 + piece, p.K, vw[i]);
     };
     const auto fetch_a = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < NA; ++i) fetch4<VEC>(A, p.lda, m0 + row + i * (THREADS / 4), p.M, k0 + piece, p.K, va[i]);
+        for (int i = 0; i < NA; ++i) {
+            const int m = m0 + row + i * (THREADS / 4);
+            fetch4<VEC>(A, p.lda, m, m < p.M, k0 + piece, p.K, va[i]);
+        }
     };
     const auto put = [&](int half) {
 #pragma unroll
@@ -260,13 +263,12 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_f32_wide_kernel(co
 #pragma unroll
             for (int e = 0; e < 4; ++e) v[e] = __uint_as_float((uint32_t)(acc[i][2 * j + (e >> 1)] >> (32 * (e & 1))));
             TC* to = C + (size_t)m * p.ldc + n;
-            if (sizeof(TC) == 4 && n + 4 <= p.N && ((uintptr_t)to & 15) == 0) {
+            if (sizeof(TC) == 4 && ((uintptr_t)to & 15) == 0) {
                 *reinterpret_cast<float4*>(to) = make_float4(v[0], v[1], v[2], v[3]);
                 continue;
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (n + e < p.N) to[e] = from_float<TC>(v[e]);
+            for (int e = 0; e < 4; ++e) to[e] = from_float<TC>(v[e]);
         }
     }
 }

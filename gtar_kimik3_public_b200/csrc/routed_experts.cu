@@ -861,7 +861,7 @@ __device__ __forceinline__ int mma_list(const int* __restrict__ ids, int first, 
 template <bool UP, int DEPTH>
 __global__ void __launch_bounds__(MMA_WARPS * 32) experts_mma_kernel(
     const __grid_constant__ CUtensorMap map, const __nv_bfloat16* __restrict__ source, const int* __restrict__ ids, __nv_bfloat16* __restrict__ act,
-    float* __restrict__ parts, int n_pairs, int k, int n_rows, int divide, int n_experts, int at_once, int staged_bytes, int box_k, int* error_flag) {
+    float* __restrict__ parts, int n_pairs, int k, int n_rows, int divide, int n_experts, int at_once, int box_k, int* error_flag) {
     constexpr int NM = UP ? 2 : 1, ENTRIES = NM * MMA_TOKENS / 8 * 4;
     extern __shared__ __align__(128) unsigned char ring_smem[];  // the rings [MMA_WARPS][DEPTH]; the tokens' rows [at_once][stride], before that counts
     __shared__ int list[MMA_LIST], n_runs;
@@ -1307,7 +1307,7 @@ int launch_ring(const MmaStep& p, int at_once, size_t staged, int blocks, cudaSt
     gk_launch_with(gk_early(!UP || t_gk_chain == 2), experts_mma_kernel<UP, DEPTH>,
                    dim3((unsigned)std::min(most, (long long)blocks * sm_count()), 1, (unsigned)((p.pairs + MMA_LIST - 1) / MMA_LIST)), dim3(MMA_WARPS * 32),
                    staged + ring_bytes(UP, DEPTH), s, dim3(1, 1, 1), map, (const __nv_bfloat16*)p.source, p.ids, (__nv_bfloat16*)p.act, p.parts, (int)p.pairs,
-                   p.k, p.n_rows, p.divide, p.n_experts, at_once, (int)staged, box_k, p.error_flag);
+                   p.k, p.n_rows, p.divide, p.n_experts, at_once, box_k, p.error_flag);
     return GK_OK;
 }
 
