@@ -687,8 +687,8 @@ __global__ void __launch_bounds__(UP_WARPS * 32) token_down_kernel(const T* __re
 // four blocks an SM.  (Loads into registers had four pieces in flight that ended with every unit, and went through
 // the load unit 64 bytes of a row at a time: 400 cycles a piece and warp, which also held for copies of 16 bytes into a ring.)
 // (Tensor-memory products would want 128 rows a tile, for a step that does next to no arithmetic.)
-// Measured (us, cold; up, down and join; loads into registers / here): 6 of 64 experts of 2,048 x 1,024: 8 tokens 140 / 93, 42: 237 / 167; 4 of
-// 32 of 1,024 x 768: 16 tokens 56 / 42, 63: 68 / 55; 2 of 16 of 4,096 x 1,536: 16 tokens 177 / 118, 120: 344 / 262; of 1,024 x 4,096, 120: 194 / 182.
+// Measured (us, cold; up, down and join; loads into registers / here): 6 of 64 experts of 2,048 x 1,024: 8 tokens 125 / 95, 42: 232 / 172; 4 of
+// 32 of 1,024 x 768: 16 tokens 54 / 42, 63: 68 / 55; 2 of 16 of 4,096 x 1,536: 16 tokens 178 / 120, 120: 346 / 228; of 1,024 x 4,096, 120: 191 / 177.
 // Every pair by itself on the FP32 pipes: 8 tokens 170 and 43, 42 and 63 tokens 763 and 265.  Bound by the weights (4.7 TB/s of them in the
 // whole call of 8 tokens) with 6 us of launch and list before the first of them, by the tokens' products where an expert has sixteen and more.
 constexpr int MMA_WARPS = 4, MMA_TOKENS = 16, MMA_LIST = 512;
