@@ -82,7 +82,7 @@ class StepGraphs:
         # The allocator of pinned memory does not know of copy_to_device's copies: it would hand the buffers on while one is still to run.
         # (Waiting for them here would make whoever drops an engine wait for its last step.)
         events = [event for event in getattr(self, "events", ()) if event is not None]
-        if events:
+        if events and _retired is not None:  # (None: the interpreter is going down)
             _retired.append((self.host, events))
 
     # ------------------------------------------------------------------ step inputs
